@@ -29,13 +29,12 @@
 #include <cuda_runtime.h>
 
 #include "gdp_device.cuh"
+#include "gdp_exact.cuh"
 #include "gdp_internal.h"
 
 namespace gdp {
 namespace {
 
-
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kQueueCap = 128;  // >= 31 pending + 64 pushed per step
 
 // Phase timers, compiled only into a library built with -DGDP_PHASE_TIMERS
@@ -339,12 +338,12 @@ __device__ __forceinline__ void record_row_infeasible(const DevProblem &P, int p
 // elements [0, e) of a row stored contiguously at (col, val), with the
 // leading 0.0 at index -1; NaN terms never count. All 32 lanes call it and
 // every lane returns the result (a butterfly of an associative selection).
-__device__ __forceinline__ void row_first_max(const DevProblem &P, const int *col, const double *val, int e,
+__device__ __forceinline__ void row_first_max(const double2 *bnd, const int *col, const double *val, int e,
                                               int lane, long long &km, int &p) {
     Acc s;
     acc_init(s);
     for (int k = lane; k < e; k += 32) {
-        const double2 b = load_bnd(P, __ldg(col + k));
+        const double2 b = bnd[__ldg(col + k)];
         acc_add_delta(s, dmul(fabs(__ldg(val + k)), dsub(b.y, b.x)), k);
     }
 #pragma unroll
@@ -365,7 +364,7 @@ __device__ __forceinline__ void row_first_max(const DevProblem &P, const int *co
 // maximum is the leading 0.0. The prefix maxima are warp passes; their values
 // wait in a stack of one level per lane. A chain deeper than 32 levels (values
 // each within EPS of the next) ends with a serial scan. All 32 lanes call it.
-__device__ __noinline__ double seq_eps_max(const DevProblem &P, const int *col, const double *val, int len,
+__device__ __noinline__ double seq_eps_max(const double2 *bnd, const int *col, const double *val, int len,
                                            long long km, int p, int lane) {
     double stack = 0.0;
     int depth = 0, E = len;
@@ -380,7 +379,7 @@ __device__ __noinline__ double seq_eps_max(const DevProblem &P, const int *col, 
             double m = 0.0;
             if (lane == 0)
                 for (int k = 0; k < E; k++) {
-                    const double2 b = load_bnd(P, __ldg(col + k));
+                    const double2 b = bnd[__ldg(col + k)];
                     const double d = dmul(fabs(__ldg(val + k)), dsub(b.y, b.x));
                     if (eps_gt(d, m)) m = d;
                 }
@@ -391,7 +390,7 @@ __device__ __noinline__ double seq_eps_max(const DevProblem &P, const int *col, 
         depth++;
         long long km2;
         int p2;
-        row_first_max(P, col, val, p, lane, km2, p2);
+        row_first_max(bnd, col, val, p, lane, km2, p2);
         if (p2 >= 0 && eps_gt(M, __longlong_as_double(km2))) {
             depth--;  // m(E) = M
             x = M;
@@ -606,7 +605,7 @@ __device__ __forceinline__ void sell_rows_exact(const DevProblem &P, const ElemV
             const int ap = __shfl_sync(kFull, s.p, src);
             const double amn = __shfl_sync(kFull, mn, src);
             const long long xb = __ldg(P.xptr + apos);
-            const double m = seq_eps_max(P, P.xcol + xb, P.xval + xb, alen, akm, ap, lane);
+            const double m = seq_eps_max(P.bnd, P.xcol + xb, P.xval + xb, alen, akm, ap, lane);
             if (lane == src) dec = eps_le(m, amn) ? 0 : 1;
         }
     }
@@ -976,7 +975,7 @@ __device__ __forceinline__ void split_row_candidates(const DevProblem &P, int ro
     go = __shfl_sync(kFull, go, 0);
     if (go == 2) {  // every tile of the row reaches the same m
         const int re = __ldg(P.tile_end + __ldg(P.lrow_tile0 + row + 1) - 1);
-        const double m = seq_eps_max(P, P.lcol + rb, P.lval + rb, re - rb, __shfl_sync(kFull, s0.km, 0),
+        const double m = seq_eps_max(P.bnd, P.lcol + rb, P.lval + rb, re - rb, __shfl_sync(kFull, s0.km, 0),
                                      __shfl_sync(kFull, s0.p, 0), lane);
         if (lane == 0) {
             go = eps_le(m, mn) ? 0 : 1;

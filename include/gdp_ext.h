@@ -322,19 +322,19 @@ void gdp_mps_free(gdp_mps_problem *p);
  * reference.
  *   - Every array argument is DEVICE memory (CSR with the reference's meaning,
  *     bounds in/out); nothing is copied to or from the host except the round
- *     flags.
+ *     state, once, at the end.
  *   - Working memory is one fixed device array inside the library, sized for
  *     GDP_NOALLOC_MAX_VARS variables (about 16 MiB); every GPU that loads the
  *     library holds it until the process exits. n_vars above the limit returns
  *     GDP_ERROR.
  *   - The first call on a device looks up that array's device address (once per
  *     device).
- *   - The host reads the round flags after every round: the call synchronizes
- *     its stream once per round.
+ *   - Every round runs in one cooperative launch; the call synchronizes its
+ *     stream once, at its end.
  *   - Calls share the array: calls that overlap on the GPU race and must be
  *     serialized by the caller. Each call re-initializes it.
- *   - Rows are summed left to right by one thread each: results equal the
- *     context path's for rows up to its thread_row_max non-zeros.
+ *   - Rows are summed left to right: results equal the context path's for rows
+ *     up to its thread_row_max non-zeros.
  * stream: CUDA stream (NULL = legacy default stream); the call returns when the
  * propagation has finished. stats may be NULL (device_ms is not measured). */
 #define GDP_NOALLOC_MAX_VARS (1 << 20)
