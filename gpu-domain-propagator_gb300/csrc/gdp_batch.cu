@@ -97,6 +97,14 @@ __device__ __forceinline__ void mark_var_rows_learned(const BatchDev &B, const D
     }
 }
 
+// The warp turns to unit u (-1: none): statistics gathered for another unit go
+// to its flags.
+__device__ __forceinline__ void stats_unit(const BatchDev &B, WarpSmem &ws, int &unit, int u, int lane) {
+    if (unit == u) return;
+    if (unit >= 0) stats_flush(B.units[unit], ws, lane);
+    unit = u;
+}
+
 // Marks the rows of variable j of unit u for round `stamp` and queues them.
 __device__ __forceinline__ void mark_var_rows(const BatchDev &B, const DevProblem &Pu, int u, int j, int stamp) {
     for (int k = __ldg(Pu.var_ptr + j); k < __ldg(Pu.var_ptr + j + 1); k++) {
@@ -210,14 +218,17 @@ namespace {
 // loop took 2,093 / 912 / 866 / 844 / 1,269 ms at 2 / 3 / 4 / 5 / 6 CTAs per
 // SM, the plain one 590 / 567 / 561 / 566 ms at 3 / 4 / 5 / 6.
 template <bool kLearned>
-__global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
-    __shared__ WarpSmem ws[kWarpsPerCta];
+__global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
+    WarpSmem *ws = warp_smem();
     __shared__ LearnSmem ls[kLearned ? kWarpsPerCta : 1];
     const int lane = threadIdx.x & 31;
     WarpSmem &mine = ws[threadIdx.x >> 5];
     LearnSmem &L = ls[kLearned ? (threadIdx.x >> 5) : 0];
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
     int last = 0;
+    unsigned target = 0;  // grid barrier
+    int stat_unit = -1;   // unit that the warp's statistics belong to
+    stats_zero(mine, lane);
     for (int r = 1; r <= B.max_rounds; r++) {
         const int par = r & 1;
         unsigned *ctr = B.ctr + 4 * par;
@@ -232,10 +243,12 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
             const int fs_items = *((volatile int *)(B.fs_prefix + nfs));
             const int n_entries = (int)min(*((volatile unsigned *)(B.tail + par)), B.cap_entries);
             const unsigned long long *ent = B.entries + (size_t)par * B.cap_entries;
-            stats_zero(mine, lane);
+            const int n_work = fs_items + n_entries;
+            WarpCursor<false> cur;
+            cur.start(ctr + 0, 1, grid_warps(), n_work);
             for (;;) {
-                const int i = warp_next(ctr + 0, lane);
-                if (i >= fs_items + n_entries) break;
+                const int i = cur.next(lane);
+                if (i >= n_work) break;
                 int u, it;
                 bool marked;
                 if (i < fs_items) {
@@ -249,6 +262,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
                     it = (int)(unsigned)e;
                     marked = true;
                 }
+                stats_unit(B, mine, stat_unit, u, lane);
                 const DevProblem &Pu = B.units[u];
                 if (*((volatile int *)&Pu.flags[0].infeasible)) continue;
                 int *change = &Pu.flags[1 + par].change;
@@ -273,10 +287,9 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
                 } else if (split_partial<0>(Pu, -it - 1, lane, r, marked, change, tight, mine) && lane == 0) {
                     push_tile(B.cq, B.tail + 2, B.cap_tiles, B.error, u, -it - 1);
                 }
-                stats_flush(Pu, mine, lane);  // statistics belong to the item's unit
             }
         }
-        if (!grid_barrier(B.barrier, B.error, B.spin_limit)) return;
+        if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
         // ---- B (plus the resets for round r + 1: its slots were last used in r - 1)
         if (gtid == 0) {
             unsigned *nctr = B.ctr + 4 * (par ^ 1);
@@ -290,30 +303,34 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
         }
         const int n_cq = (int)min(*((volatile unsigned *)(B.tail + 2)), B.cap_tiles);
         if (n_cq) {
+            WarpCursor<false> cur;
+            cur.start(ctr + 1, 1, grid_warps(), n_cq);
             for (;;) {
-                const int i = warp_next(ctr + 1, lane);
+                const int i = cur.next(lane);
                 if (i >= n_cq) break;
                 const unsigned long long e = B.cq[i];
                 const int u = (int)(e >> 32), t = (int)(unsigned)e;
+                stats_unit(B, mine, stat_unit, u, lane);
                 const DevProblem &Pu = B.units[u];
                 if (split_cand<0>(Pu, t, lane, r, false, &Pu.flags[1 + par].exact, mine) && lane == 0)
                     push_tile(B.xq, B.tail + 3, B.cap_tiles, B.error, u, t);
-                stats_flush(Pu, mine, lane);
             }
-            if (!grid_barrier(B.barrier, B.error, B.spin_limit)) return;
+            if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
             // ---- C
             const int n_xq = (int)min(*((volatile unsigned *)(B.tail + 3)), B.cap_tiles);
             if (n_xq) {
+                WarpCursor<false> curx;
+                curx.start(ctr + 2, 1, grid_warps(), n_xq);
                 for (;;) {
-                    const int i = warp_next(ctr + 2, lane);
+                    const int i = curx.next(lane);
                     if (i >= n_xq) break;
                     const unsigned long long e = B.xq[i];
                     const int u = (int)(e >> 32), t = (int)(unsigned)e;
+                    stats_unit(B, mine, stat_unit, u, lane);
                     const DevProblem &Pu = B.units[u];
                     split_exact<0>(Pu, t, lane, r, &Pu.flags[1 + par].change, &Pu.flags[1 + par].tight, mine);
-                    stats_flush(Pu, mine, lane);
                 }
-                if (!grid_barrier(B.barrier, B.error, B.spin_limit)) return;
+                if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
             }
         }
         // ---- F (a row recorded infeasible in round r turns into the unit's
@@ -379,7 +396,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
                 }
             }
         }
-        if (!grid_barrier(B.barrier, B.error, B.spin_limit)) return;
+        if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
         last = r;
         const int nfs = *((volatile int *)B.n_fs);
         const int next = *((volatile int *)(B.fs_prefix + nfs)) +
@@ -387,6 +404,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_batch_loop(BatchDev B) {
         const int pending = kLearned ? *((volatile int *)B.n_pending) : 0;
         if (!more || (next == 0 && pending == 0)) break;
     }
+    stats_unit(B, mine, stat_unit, -1, lane);
     for (int u = gtid; u < B.n_units; u += gthreads) close_round(B, u, last);
     if (gtid == 0) B.rounds_out[0] = last;
 }
@@ -467,8 +485,10 @@ __global__ void __launch_bounds__(256) k_batch_fini(BatchDev B, double *lb, doub
 
 // ---- launchers --------------------------------------------------------------
 int batch_occupancy(int *blocks_per_sm, bool learned) {
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            blocks_per_sm, learned ? k_batch_loop<true> : k_batch_loop<false>, kCtaThreads, 0);
+    const void *k = learned ? (const void *)k_batch_loop<true> : (const void *)k_batch_loop<false>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaSmem);
+    if (e != cudaSuccess) return (int)e;
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kCtaThreads, kCtaSmem);
 }
 
 int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub, double *lb_out,
@@ -487,7 +507,7 @@ int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub
     BatchDev Bc = B;
     void *args[] = {&Bc};
     e = cudaLaunchCooperativeKernel(learned ? (const void *)k_batch_loop<true> : (const void *)k_batch_loop<false>,
-                                    dim3(grid), dim3(kCtaThreads), args, 0, s);
+                                    dim3(grid), dim3(kCtaThreads), args, kCtaSmem, s);
     if (e != cudaSuccess) return (int)e;
     k_batch_fini<<<vgrid, 256, 0, s>>>(B, lb_out, ub_out, var_base);
     return (int)cudaGetLastError();

@@ -24,7 +24,7 @@ struct BatchDev {
     int *fs_unit;         // units swept in full in the coming round
     int *fs_prefix;       // n_fs + 1: prefix of their work-item counts
     int *n_fs;
-    unsigned *barrier;    // {count, generation}
+    unsigned *barrier;    // arrivals
     int *error;
     int *rounds_out;
     int *n_pending;       // learned units that need the next round (learned batches)

@@ -66,10 +66,7 @@ GDP_RETCODE Batch::init_instances(int n_inst, const int *n_cons, const int *n_va
     nodes = false;
     max_rounds = inst_[0]->opts.max_rounds;
     units_h_.resize(n_units);
-    for (int u = 0; u < n_units; u++) {
-        units_h_[u] = inst_[u]->P;
-        units_h_[u].defer_exact = 0;  // the batch loop runs exact passes in place
-    }
+    for (int u = 0; u < n_units; u++) units_h_[u] = inst_[u]->P;
     // per-unit batch state: slice stamps
     for (int u = 0; u < n_units; u++) {
         DevProblem &Q = units_h_[u];
@@ -95,7 +92,6 @@ GDP_RETCODE Batch::init_nodes(Context *ctx, int n_nodes) {
     const DevProblem &S = ctx->P;
     const int n = std::max(S.n, 1), npos = std::max(S.n_srows + S.n_lrows, 1);
     units_h_.assign(n_units, S);
-    for (int u = 0; u < n_units; u++) units_h_[u].defer_exact = 0;  // exact passes run in place
     for (int u = 0; u < n_units; u++) {
         DevProblem &Q = units_h_[u];
         Q.bnd = (double2 *)arena_.alloc_bytes(sizeof(double2) * (size_t)n);

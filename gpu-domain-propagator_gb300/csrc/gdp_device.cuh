@@ -33,103 +33,6 @@ __device__ __forceinline__ bool is_neginf(double x) { return x <= -kInf; }
 __device__ __forceinline__ double eps_floor(double x) { return floor(dadd(x, kEps)); }
 __device__ __forceinline__ double eps_ceil(double x) { return ceil(dsub(x, kEps)); }
 
-// Row statistics (reference ActivitiesTuple, src/propagation_methods.cuh:10-17).
-struct RowActs {
-    double minact, maxact, maxactdelta;
-    int minact_inf, maxact_inf;
-};
-
-// One term of computeActivities (src/propagation_methods.cuh:188-214), added
-// to the running left-to-right state.
-__device__ __forceinline__ void acts_add(RowActs &a, double coeff, double lb, double ub) {
-    const double delta = dmul(fabs(coeff), dsub(ub, lb));
-    if (eps_gt(delta, a.maxactdelta)) a.maxactdelta = delta;
-    const bool pos = coeff > kEps;  // EPSGT(coeff, 0): coeff - 0 is exact
-    const bool min_inf = pos ? is_neginf(lb) : is_posinf(ub);
-    const bool max_inf = pos ? is_posinf(ub) : is_neginf(lb);
-    a.minact_inf += min_inf;
-    a.maxact_inf += max_inf;
-    const bool gt0 = coeff > 0.0;
-    if (!min_inf) a.minact = dadd(a.minact, dmul(coeff, gt0 ? lb : ub));
-    if (!max_inf) a.maxact = dadd(a.maxact, dmul(coeff, gt0 ? ub : lb));
-}
-
-__device__ __forceinline__ void acts_init(RowActs &a) {
-    a.minact = 0.0; a.maxact = 0.0; a.maxactdelta = 0.0; a.minact_inf = 0; a.maxact_inf = 0;
-}
-
-// reference canConsBeTightened, src/propagation_methods.cuh:136-154
-__device__ __forceinline__ bool can_cons_be_tightened(const RowActs &a, double lhs, double rhs) {
-    if (a.minact_inf > 1 && a.maxact_inf > 1) return false;
-    if (a.maxactdelta < kInf) {  // EPSLT(maxactdelta, GDP_INF)
-        const double s = dsub(rhs, a.minact), t = dsub(a.maxact, lhs);
-        return !eps_le(a.maxactdelta, (t < s) ? t : s);  // std::min(s, t)
-    }
-    return true;
-}
-
-// Per-row constants of tightenVariable (src/propagation_methods.cuh:223-276).
-struct RowCand {
-    double slack, surplus, neg_surplus;  // rhs - minact, lhs - maxact, maxact - lhs
-    int minact_inf, maxact_inf;
-    bool rhs_side_ok;  // !ISPOSINF(rhs) && !ISNEGINF(minact)
-    bool lhs_side_ok;  // !ISNEGINF(lhs) && !ISPOSINF(maxact)
-};
-
-__device__ __forceinline__ RowCand row_cand(const RowActs &a, double lhs, double rhs) {
-    RowCand c;
-    c.slack = dsub(rhs, a.minact);
-    c.surplus = dsub(lhs, a.maxact);
-    c.neg_surplus = dsub(a.maxact, lhs);
-    c.minact_inf = a.minact_inf;
-    c.maxact_inf = a.maxact_inf;
-    c.rhs_side_ok = !is_posinf(rhs) && !is_neginf(a.minact);
-    c.lhs_side_ok = !is_neginf(lhs) && !is_posinf(a.maxact);
-    return c;
-}
-
-// tightenVarUpperBound, src/propagation_methods.cuh:78-106
-__device__ __forceinline__ bool tighten_upper(double coeff, const RowCand &c, int num_inf, double lb,
-                                              double ub, bool is_cont, double &newb) {
-    if (!(num_inf == 0 || (num_inf == 1 && is_neginf(lb)))) return false;
-    double nb = ddiv(coeff > 0 ? c.slack : c.surplus, coeff);
-    if (num_inf == 0) nb = dadd(nb, lb);
-    if (!is_cont) nb = eps_floor(nb);
-    if (eps_lt(nb, ub)) { newb = nb; return true; }
-    return false;
-}
-
-// tightenVarLowerBound, src/propagation_methods.cuh:108-134
-__device__ __forceinline__ bool tighten_lower(double coeff, const RowCand &c, int num_inf, double lb,
-                                              double ub, bool is_cont, double &newb) {
-    if (!(num_inf == 0 || (num_inf == 1 && is_posinf(ub)))) return false;
-    double nb = ddiv(coeff > 0 ? c.surplus : c.slack, coeff);
-    if (num_inf == 0) nb = dadd(nb, ub);
-    if (!is_cont) nb = eps_ceil(nb);
-    if (eps_gt(nb, lb)) { newb = nb; return true; }
-    return false;
-}
-
-// tightenVariable, src/propagation_methods.cuh:223-276. coeff*(ub-lb) for
-// coeff > 0 and coeff*(lb-ub) otherwise both equal |coeff|*(ub-lb) bit for bit
-// (round-to-nearest is sign-symmetric), so one product serves both branches.
-__device__ __forceinline__ void tighten_variable(double coeff, const RowCand &c, bool is_cont, double lb,
-                                                 double ub, bool &lb_t, double &newlb, bool &ub_t,
-                                                 double &newub) {
-    lb_t = false;
-    ub_t = false;
-    const double d = dmul(fabs(coeff), dsub(ub, lb));
-    const bool rhs_side = c.rhs_side_ok && eps_gt(d, c.slack);
-    const bool lhs_side = c.lhs_side_ok && eps_gt(d, c.neg_surplus);
-    if (coeff > 0.0) {
-        if (rhs_side) ub_t = tighten_upper(coeff, c, c.minact_inf, lb, ub, is_cont, newub);
-        if (lhs_side) lb_t = tighten_lower(coeff, c, c.maxact_inf, lb, ub, is_cont, newlb);
-    } else {
-        if (rhs_side) lb_t = tighten_lower(coeff, c, c.minact_inf, lb, ub, is_cont, newlb);
-        if (lhs_side) ub_t = tighten_upper(coeff, c, c.maxact_inf, lb, ub, is_cont, newub);
-    }
-}
-
 // FP64 max / min as one integer atomic each: for sign bit 0 the bit pattern
 // orders like a signed integer; for sign bit 1 it orders in reverse as an
 // unsigned integer. No CAS loop, no return value (RED.MAX / RED.MIN).
@@ -182,36 +85,16 @@ __device__ __forceinline__ float f32_mag(unsigned long long mag, bool up) {
     if (up && (man & 0x1FFFFFFFULL)) fb += 1u;
     return __uint_as_float(fb);
 }
-__device__ __forceinline__ float f32_up(long long b) {
-    const unsigned long long mag = (unsigned long long)b & 0x7FFFFFFFFFFFFFFFULL;
-    return b < 0 ? -f32_mag(mag, false) : f32_mag(mag, true);
-}
 __device__ __forceinline__ float f32_dn(long long b) {
     const unsigned long long mag = (unsigned long long)b & 0x7FFFFFFFFFFFFFFFULL;
     return b < 0 ? -f32_mag(mag, true) : f32_mag(mag, false);
 }
 constexpr float kUMargin = 1.00000095367431640625f;  // 1 + 2^-20
 
-// Sign-aware FP32 enclosure lo <= |a| (ub - lb) <= hi of one element, each end
-// widened by a relative 2^-20 (covers the round-to-nearest float operations).
-// NaN (e.g. inf - inf) makes every comparison inconclusive, which sends the
-// element to the exact FP64 path.
+// FP32 enclosure lo <= |a| (ub - lb) <= hi of one element (delta_box32).
 struct DeltaBox {
     float lo, hi;
 };
-__device__ __forceinline__ float widen_up(float x) { return __fadd_rn(x, fabsf(x) * 9.5367431640625e-7f); }
-__device__ __forceinline__ float widen_dn(float x) { return __fsub_rn(x, fabsf(x) * 9.5367431640625e-7f); }
-__device__ __forceinline__ DeltaBox delta_box(long long ab, long long lbb, long long ubb) {
-    const unsigned long long am = (unsigned long long)ab & 0x7FFFFFFFFFFFFFFFULL;
-    const float a_up = f32_mag(am, true), a_dn = f32_mag(am, false);
-    const float dh = __fsub_rn(f32_up(ubb), f32_dn(lbb));  // >= ub - lb (up to rounding)
-    const float dl = __fsub_rn(f32_dn(ubb), f32_up(lbb));  // <= ub - lb (up to rounding)
-    DeltaBox b;
-    b.hi = widen_up(__fmul_rn(dh >= 0.0f ? a_up : a_dn, dh));
-    b.lo = widen_dn(__fmul_rn(dl >= 0.0f ? a_dn : a_up, dl));
-    return b;
-}
-
 // Activity accumulator: the reference's computeActivities terms with integer
 // classification (no FP64 compares), plus the first maximum of the FP64
 // |a| (ub - lb) over the elements seen: km is its order key (order_key of its
@@ -247,7 +130,6 @@ __device__ __forceinline__ void acc_take_max(Acc &s, long long km, int p) {
         s.p = p;
     }
 }
-__device__ __forceinline__ double acc_max(const Acc &s) { return __longlong_as_double(s.km); }
 // The activity terms and infinity counts of one element.
 __device__ __forceinline__ void acc_add_terms(Acc &s, double a, double lb, double ub) {
     const long long ab = dbits(a), lbb = dbits(lb), ubb = dbits(ub);
@@ -267,18 +149,6 @@ __device__ __forceinline__ void acc_combine(Acc &a, const Acc &b) {
     a.minf += b.minf;
     a.maxf += b.maxf;
     acc_take_max(a, b.km, b.p);
-}
-
-// min(rhs - minact, maxact - lhs) as std::min(s, t) in canConsBeTightened.
-__device__ __forceinline__ double row_min_slack(double minact, double maxact, double lhs, double rhs) {
-    const double s = dsub(rhs, minact), t = dsub(maxact, lhs);
-    return (t < s) ? t : s;
-}
-// The reference's decision from its sequential maxactdelta (canConsBeTightened).
-__device__ __forceinline__ bool reference_row_go(int minf, int maxf, double maxactdelta, double mn) {
-    if (minf > 1 && maxf > 1) return false;
-    if (maxactdelta < kInf) return !eps_le(maxactdelta, mn);
-    return true;
 }
 
 // The reference's row test (canConsBeTightened, src/propagation_methods.cuh:

@@ -1,32 +1,23 @@
 // gdp_exact.cuh -- the exact FP64 pass of the rows that the FP32 screen cannot
 // skip: activities, the reference's row test, candidates and their divisions,
-// for a few rows per warp.
+// for a few rows per warp (an item).
 //
 // What bounds it: the FP64 pipe. A dependent FP64 add takes 71 cycles, and a
 // warp's next FP64 instruction starts 68 to 76 cycles after its last one even
 // when it does not depend on it (measured: one FP64 unit per SM quarter, 0.44
 // lanes per clock), so an FP64 instruction costs the same with one active lane
 // as with 32, and the number of FP64 instructions in a row's path is its
-// latency. One lane walking a row of 32 elements executes 8 of them per
-// element (two products, two sums, |a| (ub - lb), the EPS-max): 256
-// instructions, 9.4 us, whether the warp's other lanes have rows or not.
-//
-// Here the rows of a warp are one flat list of elements. 32 lanes form the
-// products of 32 consecutive elements, whichever rows they belong to, and
-// stage them in shared memory (5 FP64 instructions per 32 elements); then one
-// lane per row, lane of the row's summation order and side (minimum and
-// maximum activity in different lanes) adds them up in that order: one FP64
-// add per step for both sides of 16 / g rows. The additions and their order
-// are those of one lane (g = 1) or g lanes per row, so every bit is the same.
-// The first maximum of |a| (ub - lb) is found by integer compares beside the
-// adds. 16 rows of L elements take 3.5 L FP64 instructions instead of 8 L (and
-// 32 rows 7 L instead of 8 L).
-//
-// Elements whose |a| (ub - lb) exceeds the screen's lower bound of both slacks
-// -- the only ones that can yield a candidate -- are collected while they are
-// staged, so the candidate tests run on full warps over a few elements per row
-// instead of visiting the rows again; divisions wait in a queue that carries
-// their numerators and outlives the rows, and run 32 at a time.
+// latency. So
+//   * per element 4 products and 2 additions are FP64 (no conversion, no
+//     compare, no subtraction for the EPS-max: the first maximum of
+//     |a| (ub - lb) is found by integer compares and decides the row test
+//     (row_go_from_max) unless it lies in a band of 1e-9);
+//   * elements whose |a| (ub - lb) exceeds the screen's lower bound of both
+//     slacks -- the only ones that can yield a candidate -- are collected on
+//     the way, and the candidate tests run on full warps over those alone
+//     instead of visiting the rows again;
+//   * divisions wait in a queue that carries their numerators and outlives the
+//     rows, and run 32 at a time.
 #pragma once
 
 #include "gdp_device.cuh"
@@ -35,10 +26,9 @@ namespace gdp {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kStage = 128;     // elements staged at a time
-constexpr int kItemRows = 16;   // most rows of a warp's item (g = 1; 16 / g rows of g lanes)
+constexpr int kItemRows = 32;   // most rows of an item
 constexpr int kCandCap = 96;    // collected elements; rows that yield more are read again
-constexpr int kDivCap = 96;     // >= 31 pending + 64 pushed per step
+constexpr int kDivCap = 64;     // >= 31 pending + 32 pushed per side
 
 // A queued division: numerator, element, and code: bit 0 the side (0 upper
 // bound, 1 lower), bit 1 whether the variable's other bound is added, bits 2..
@@ -50,16 +40,12 @@ struct DivEntry {
 };
 
 struct ExactSmem {
-    double t[2][kStage];  // minimum / maximum activity terms
-    double d[kStage];     // |a| (ub - lb)
     DivEntry div[kDivCap];
-    double cand_d[kCandCap];
-    int cand_k[kCandCap];
-    unsigned char cand_s[kCandCap];  // row slot, bit 7: a > 0
     double slack[kItemRows], nsur[kItemRows];  // rhs - minact, maxact - lhs
-    long long cut[kItemRows];  // order key that |a| (ub - lb) must exceed
-    int src[kItemRows];        // element index of the row's flat index 0
-    unsigned info[kItemRows];  // bits 0, 1: usable sides; 2, 3: minf; 4, 5: maxf; 6: candidates wanted
+    int cand_k[kCandCap];
+    int src[kItemRows];                 // element index of the row's flat index 0
+    unsigned char cand_s[kCandCap];     // row slot
+    unsigned char info[kItemRows];      // bits 0, 1: usable sides; 2, 3: minf; 4, 5: maxf; 6: candidates wanted
 };
 
 // The rows of an item: lane r < n holds row r (in is set for those lanes).
@@ -93,16 +79,16 @@ __device__ __forceinline__ FlatRows flat_rows(const ExactRow &R, int lane) {
     F.len = R.in ? R.len : 0;
     int inc = F.len;
 #pragma unroll
-    for (int off = 1; off < kItemRows; off <<= 1) {
+    for (int off = 1; off < 32; off <<= 1) {
         const int v = __shfl_up_sync(kFull, inc, off);
         if (lane >= off) inc += v;
     }
-    F.total = __shfl_sync(kFull, inc, kItemRows - 1);
+    F.total = __shfl_sync(kFull, inc, 31);
     F.pre = inc - F.len;
     return F;
 }
 // The slot of the row that owns flat element f0 + lane (rows of the list are
-// not empty, so their first elements are distinct).
+// not empty, so their first elements are distinct; slots are lanes 0, 1, ...).
 __device__ __forceinline__ int flat_slot(const FlatRows &F, int f0, int lane) {
     const int s = F.pre - f0;
     const unsigned starts = __reduce_or_sync(kFull, (F.len && s >= 0 && s < 32) ? 1u << s : 0u);
@@ -148,30 +134,26 @@ __device__ __forceinline__ void exact_drain(const T &t, ExactSmem &xs, ExactQueu
             }
         }
         __syncwarp();
-        const int rest = Q.cnt - take;
-        DivEntry mv[2];
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-            if (lane + 32 * i < rest) mv[i] = xs.div[take + lane + 32 * i];
+        Q.cnt -= take;  // at most 31 are left: they do not overlap the ones that ran
+        if (lane < Q.cnt) xs.div[lane] = xs.div[take + lane];
         __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-            if (lane + 32 * i < rest) xs.div[lane + 32 * i] = mv[i];
-        __syncwarp();
-        Q.cnt = rest;
     }
 }
 
 // Queues the divisions of one element per lane (tightenVariable, src/
 // propagation_methods.cuh:223-276): element k with |a| (ub - lb) = d of the row
-// in slot `slot`; pos: a > 0. Lanes without an element pass on = false.
+// in slot `slot`. Lanes without an element pass on = false.
 template <class T>
 __device__ __forceinline__ void exact_push(const T &t, ExactSmem &xs, ExactQueue &Q, bool on, int k, int slot,
-                                           bool pos, double d, int lane, int *row_tight) {
-    int sides = 0;
+                                           int lane, int *row_tight) {
+    bool uo = false, lo = false, pos = false;
     unsigned info = 0;
     double s = 0.0, u = 0.0;
     if (on) {
+        const double a = __ldg(t.val + k);
+        const double2 b = t.bnd[__ldg(t.col + k)];
+        const double d = dmul(fabs(a), dsub(b.y, b.x));
+        pos = gt0_bits(dbits(a));
         info = xs.info[slot];
         s = xs.slack[slot];
         u = xs.nsur[slot];
@@ -179,118 +161,216 @@ __device__ __forceinline__ void exact_push(const T &t, ExactSmem &xs, ExactQueue
         const bool ls = (info & 2u) && eps_gt_fast(d, u);
         const int minf = (info >> 2) & 3, maxf = (info >> 4) & 3;
         const int nu = pos ? minf : maxf, nl = pos ? maxf : minf;
-        bool uo = (pos ? rs : ls) && nu <= 1, lo = (pos ? ls : rs) && nl <= 1;
-        if ((uo && nu == 1) || (lo && nl == 1)) {  // the only infinite contribution must be this variable's
-            const double2 b = t.bnd[__ldg(t.col + k)];
-            uo = uo && (nu == 0 || neginf_bits(dbits(b.x)));
-            lo = lo && (nl == 0 || posinf_bits(dbits(b.y)));
-        }
-        sides = (uo ? 1 : 0) | (lo ? 2 : 0);
+        // a side with one infinite contribution is usable if it is this variable's
+        uo = (pos ? rs : ls) && (nu == 0 || (nu == 1 && neginf_bits(dbits(b.x))));
+        lo = (pos ? ls : rs) && (nl == 0 || (nl == 1 && posinf_bits(dbits(b.y))));
     }
-    const unsigned bu = __ballot_sync(kFull, sides & 1), bl = __ballot_sync(kFull, sides & 2);
-    if (!(bu | bl)) return;
+    const unsigned bu = __ballot_sync(kFull, uo), bl = __ballot_sync(kFull, lo);
     const unsigned lt = (1u << lane) - 1u;
     // lhs - maxact is -(maxact - lhs) (round-to-nearest is symmetric), +0.0 when they are equal
     const double surplus = __longlong_as_double((dbits(u) << 1) ? dbits(u) ^ (1LL << 63) : 0LL);
-    if (sides & 1)
-        xs.div[Q.cnt + __popc(bu & lt)] =
-                DivEntry{pos ? s : surplus, k, (unsigned)slot << 2 | ((pos ? info >> 2 : info >> 4) & 3u ? 0u : 2u)};
-    if (sides & 2)
-        xs.div[Q.cnt + __popc(bu) + __popc(bl & lt)] = DivEntry{
-                pos ? surplus : s, k, (unsigned)slot << 2 | ((pos ? info >> 4 : info >> 2) & 3u ? 0u : 2u) | 1u};
-    __syncwarp();
-    Q.cnt += __popc(bu) + __popc(bl);
-    Q.pushed += __popc(bu) + __popc(bl);
-    exact_drain(t, xs, Q, false, lane, row_tight);
+    if (bu) {
+        if (uo)
+            xs.div[Q.cnt + __popc(bu & lt)] =
+                    DivEntry{pos ? s : surplus, k, (unsigned)slot << 2 | ((info >> (pos ? 2 : 4)) & 3u ? 0u : 2u)};
+        __syncwarp();
+        Q.cnt += __popc(bu);
+        Q.pushed += __popc(bu);
+        exact_drain(t, xs, Q, false, lane, row_tight);
+    }
+    if (bl) {
+        if (lo)
+            xs.div[Q.cnt + __popc(bl & lt)] = DivEntry{
+                    pos ? surplus : s, k, (unsigned)slot << 2 | ((info >> (pos ? 4 : 2)) & 3u ? 0u : 2u) | 1u};
+        __syncwarp();
+        Q.cnt += __popc(bl);
+        Q.pushed += __popc(bl);
+        exact_drain(t, xs, Q, false, lane, row_tight);
+    }
 }
 
-// Activities and first maximum of the item's rows, g = 2^lg lanes per row in
-// the summation order (16 / g rows; one row for g = 32). Collects the elements
-// above the rows' cuts; cand receives their number (more than kCandCap: the
-// list is not complete).
-template <class T>
-__device__ __forceinline__ ExactSums exact_sums(const T &t, ExactSmem &xs, const ExactRow &R, const FlatRows &F,
-                                                int lg, int lane, int &cand) {
-    const int g = 1 << lg;
-    __syncwarp();
-    if (R.in) {
-        xs.src[lane] = R.base - F.pre;
-        xs.cut[lane] = order_key(dbits(R.slack_lo == R.slack_lo ? (double)R.slack_lo : -1e308));
+// The order key that |a| (ub - lb) must exceed to be collected.
+__device__ __forceinline__ long long candidate_cut(float slack_lo) {
+    return order_key(dbits(slack_lo == slack_lo ? (double)slack_lo : -1e308));
+}
+// Collects the lanes' elements with keep set: element k of the row in `slot`.
+// cand counts them all; the list holds the first kCandCap.
+__device__ __forceinline__ void collect(ExactSmem &xs, int &cand, bool keep, int k, int slot, int lane) {
+    const unsigned bal = __ballot_sync(kFull, keep);
+    const int at = cand + __popc(bal & ((1u << lane) - 1u));
+    if (keep && at < kCandCap) {
+        xs.cand_k[at] = k;
+        xs.cand_s[at] = (unsigned char)slot;
     }
-    __syncwarp();
-    // this lane's part of the adds: side, row slot and lane of the row
-    const int side = lg < 5 ? lane >> 4 : 0;
-    const int slot = lg < 5 ? (lane & 15) >> lg : 0;
-    const int sub = lane & (g - 1);
-    const int rpre = __shfl_sync(kFull, F.pre, slot), rlen = __shfl_sync(kFull, F.len, slot);
-    double acc = 0.0, acc2 = 0.0;  // acc2: maximum activity of a 32-lane row
+    cand += __popc(bal);
+}
+
+// First maximum by integer compares: the larger key, of equal ones the earlier
+// element.
+__device__ __forceinline__ void take_first_max(long long &km, int &p, long long ok, int op) {
+    if (ok > km || (ok == km && op < p)) {
+        km = ok;
+        p = op;
+    }
+}
+
+// Activities and first maximum of the item's rows. A chain is one of the
+// g = 2^lg lanes in the row's summation order; H = 2^lh lanes work on a chain,
+// so an item has 32 / H chains (32 / H / g rows). The additions and their order
+// are those of the contract whatever H is (an element beyond the row's end adds
+// +0.0, which changes no sum that starts at +0.0).
+//
+// H = 1: a lane forms its chain's terms and adds up both sides: 6 FP64
+// instructions per step of the chains. For rounds with many rows.
+// T::kAligned: rows start on 16-byte boundaries and are padded to them, so
+// four columns and four coefficients of a one-lane row are three loads.
+template <class T>
+__device__ __forceinline__ ExactSums exact_sums(const T &t, ExactSmem &xs, const ExactRow &R, int lg, int lane,
+                                                int &cand) {
+    constexpr int kU = 4;
+    const int g = 1 << lg;
+    const int slot = lane >> lg, sub = lane & (g - 1);
+    const int base = __shfl_sync(kFull, R.base, slot) + sub;
+    const int len = __shfl_sync(kFull, R.in ? R.len : 0, slot);
+    const long long cut = candidate_cut(__shfl_sync(kFull, R.slack_lo, slot));
+    const int steps = len > sub ? (len - sub + g - 1) >> lg : 0;
+    const int most = __reduce_max_sync(kFull, steps);
+    double acc = 0.0, acc2 = 0.0;
     long long km = 0;
-    int p = -1, e = sub;
+    int p = -1;
     cand = 0;
-    for (int w0 = 0; w0 < F.total; w0 += kStage) {
-        constexpr int kSteps = kStage / 32;
-        int k[kSteps], slots[kSteps], j[kSteps];
-        double a[kSteps];
-        double2 b[kSteps];
-#pragma unroll
-        for (int i = 0; i < kSteps; i++) {
-            slots[i] = flat_slot(F, w0 + 32 * i, lane);
-            const int f = w0 + 32 * i + lane;
-            k[i] = f < F.total ? xs.src[slots[i]] + f : -1;
-            j[i] = k[i] >= 0 ? __ldg(t.col + k[i]) : 0;
-            a[i] = k[i] >= 0 ? __ldg(t.val + k[i]) : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < kSteps; i++) b[i] = k[i] >= 0 ? t.bnd[j[i]] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int i = 0; i < kSteps; i++) {
-            if (w0 + 32 * i >= F.total) break;  // warp-uniform
-            double d;
-            exact_terms(a[i], b[i], xs.t[0][32 * i + lane], xs.t[1][32 * i + lane], d);
-            xs.d[32 * i + lane] = d;
-            const long long db = dbits(d);
-            const bool keep = k[i] >= 0 && (order_key(db) > xs.cut[slots[i]] ||
-                                            (db & 0x7FF0000000000000LL) == 0x7FF0000000000000LL);
-            const unsigned bal = __ballot_sync(kFull, keep);
-            const int at = cand + __popc(bal & ((1u << lane) - 1u));
-            if (keep && at < kCandCap) {
-                xs.cand_d[at] = d;
-                xs.cand_k[at] = k[i];
-                xs.cand_s[at] = (unsigned char)(slots[i] | (gt0_bits(dbits(a[i])) ? 128 : 0));
+    __syncwarp();  // the list is free
+    for (int s0 = 0; s0 < most; s0 += kU) {
+        int j[kU];
+        double a[kU];
+        double2 b[kU];
+        if (T::kAligned && lg == 0) {
+            if (s0 < steps) {
+                const int4 c4 = __ldg(reinterpret_cast<const int4 *>(t.col + base + s0));
+                const double2 v0 = __ldg(reinterpret_cast<const double2 *>(t.val + base + s0));
+                const double2 v1 = __ldg(reinterpret_cast<const double2 *>(t.val + base + s0 + 2));
+                j[0] = c4.x; j[1] = c4.y; j[2] = c4.z; j[3] = c4.w;
+                a[0] = v0.x; a[1] = v0.y; a[2] = v1.x; a[3] = v1.y;
             }
-            cand += __popc(bal);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kU; i++)
+                if (s0 + i < steps) {
+                    j[i] = __ldg(t.col + base + ((s0 + i) << lg));
+                    a[i] = __ldg(t.val + base + ((s0 + i) << lg));
+                }
         }
-        __syncwarp();
-        const int end = min(rlen, w0 + kStage - rpre);  // elements of my row staged so far
-        const int at = rpre - w0;  // staged index of my row's element 0
-#pragma unroll 4
-        for (; e < end; e += g) {
-            acc = dadd(acc, xs.t[side][at + e]);
-            if (lg == 5) acc2 = dadd(acc2, xs.t[1][at + e]);
-            const long long kd = order_key(dbits(xs.d[at + e]));
-            if (kd > km && kd <= kKeyPosInf) {
-                km = kd;
-                p = e;
+#pragma unroll
+        for (int i = 0; i < kU; i++)
+            if (s0 + i < steps) b[i] = t.bnd[j[i]];
+        unsigned keep = 0u;
+#pragma unroll
+        for (int i = 0; i < kU; i++)
+            if (s0 + i < steps) {
+                double tmin, tmax, d;
+                exact_terms(a[i], b[i], tmin, tmax, d);
+                acc = dadd(acc, tmin);
+                acc2 = dadd(acc2, tmax);
+                const long long db = dbits(d), kd = order_key(db);
+                if (kd > km && kd <= kKeyPosInf) {
+                    km = kd;
+                    p = sub + ((s0 + i) << lg);
+                }
+                if (kd > cut || (db & 0x7FF0000000000000LL) == 0x7FF0000000000000LL) keep |= 1u << i;
             }
+        if (__any_sync(kFull, keep)) {
+#pragma unroll
+            for (int i = 0; i < kU; i++) collect(xs, cand, (keep >> i) & 1u, base + ((s0 + i) << lg), slot, lane);
         }
-        __syncwarp();
     }
     for (int off = g >> 1; off > 0; off >>= 1) {
         acc = dadd(acc, __shfl_down_sync(kFull, acc, off));
-        if (lg == 5) acc2 = dadd(acc2, __shfl_down_sync(kFull, acc2, off));
+        acc2 = dadd(acc2, __shfl_down_sync(kFull, acc2, off));
         const long long ok = __shfl_down_sync(kFull, km, off);
-        const int op = __shfl_down_sync(kFull, p, off);
-        if (ok > km || (ok == km && op < p)) {
-            km = ok;
-            p = op;
-        }
+        take_first_max(km, p, ok, __shfl_down_sync(kFull, p, off));
     }
     // back to the lanes that hold the rows
     const int lead = R.in ? lane << lg : 0;
     ExactSums s;
     s.minact = __shfl_sync(kFull, acc, lead);
-    const double hi = __shfl_sync(kFull, acc, (lead + 16) & 31), hi32 = __shfl_sync(kFull, acc2, 0);
-    s.maxact = lg < 5 ? hi : hi32;
+    s.maxact = __shfl_sync(kFull, acc2, lead);
+    s.km = __shfl_sync(kFull, km, lead);
+    s.p = __shfl_sync(kFull, p, lead);
+    return s;
+}
+
+// H = 2^lh >= 2 lanes per chain: they form the terms of H consecutive steps
+// together (4 FP64 instructions), then the even lanes add up the minimum and
+// the odd lanes the maximum activity (H adds, terms by shuffles): 4 / H + 1 per
+// step. The same rate as H = 1 at H = 2 and a shorter path: a 32-element row
+// takes 96 FP64 instructions at H = 2, 48 at H = 8, 192 at H = 1. For rounds
+// with few rows.
+template <class T>
+__device__ __forceinline__ ExactSums exact_sums_spread(const T &t, ExactSmem &xs, const ExactRow &R, int lg, int lh,
+                                                       int lane, int &cand) {
+    constexpr int kU = 4;
+    const int g = 1 << lg, H = 1 << lh;
+    const int chain = lane >> lh, h = lane & (H - 1), first = lane - h;
+    const int slot = chain >> lg, sub = chain & (g - 1);
+    const int base = __shfl_sync(kFull, R.base, slot) + sub;
+    const int len = __shfl_sync(kFull, R.in ? R.len : 0, slot);
+    const long long cut = candidate_cut(__shfl_sync(kFull, R.slack_lo, slot));
+    const int steps = len > sub ? (len - sub + g - 1) >> lg : 0;
+    const int most = __reduce_max_sync(kFull, steps);
+    double acc = 0.0;
+    long long km = 0;
+    int p = -1;
+    cand = 0;
+    __syncwarp();  // the list is free
+    for (int s0 = 0; s0 < most; s0 += kU * H) {
+        int j[kU];
+        double a[kU];
+        double2 b[kU];
+#pragma unroll
+        for (int i = 0; i < kU; i++) {
+            const int q = s0 + i * H + h;
+            j[i] = q < steps ? __ldg(t.col + base + (q << lg)) : -1;
+            a[i] = q < steps ? __ldg(t.val + base + (q << lg)) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < kU; i++) b[i] = j[i] >= 0 ? t.bnd[j[i]] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < kU; i++) {
+            const int q0 = s0 + i * H;
+            if (q0 >= most) break;  // warp-uniform
+            double tmin = 0.0, tmax = 0.0;
+            bool keep = false;
+            if (j[i] >= 0) {
+                double d;
+                exact_terms(a[i], b[i], tmin, tmax, d);
+                const long long db = dbits(d), kd = order_key(db);
+                if (kd > km && kd <= kKeyPosInf) {
+                    km = kd;
+                    p = sub + ((q0 + h) << lg);
+                }
+                keep = kd > cut || (db & 0x7FF0000000000000LL) == 0x7FF0000000000000LL;
+            }
+            const int adds = min(H, most - q0);
+            for (int q = 0; q < adds; q++) {
+                const double lo = __shfl_sync(kFull, tmin, first + q), hi = __shfl_sync(kFull, tmax, first + q);
+                acc = dadd(acc, (h & 1) ? hi : lo);
+            }
+            if (__any_sync(kFull, keep)) collect(xs, cand, keep, base + ((q0 + h) << lg), slot, lane);
+        }
+    }
+    for (int off = 1; off < H; off <<= 1) {
+        const long long ok = __shfl_xor_sync(kFull, km, off);
+        take_first_max(km, p, ok, __shfl_xor_sync(kFull, p, off));
+    }
+    for (int off = g >> 1; off > 0; off >>= 1) {
+        acc = dadd(acc, __shfl_down_sync(kFull, acc, off << lh));
+        const long long ok = __shfl_down_sync(kFull, km, off << lh);
+        take_first_max(km, p, ok, __shfl_down_sync(kFull, p, off << lh));
+    }
+    const int lead = R.in ? lane << (lg + lh) : 0;
+    ExactSums s;
+    s.minact = __shfl_sync(kFull, acc, lead);
+    s.maxact = __shfl_sync(kFull, acc, lead + 1);
     s.km = __shfl_sync(kFull, km, lead);
     s.p = __shfl_sync(kFull, p, lead);
     return s;
@@ -310,44 +390,36 @@ __device__ __forceinline__ int exact_decide(const ExactRow &R, const ExactSums &
 }
 
 // Candidates of the rows with go set (lanes that hold rows), from their
-// slacks s and t; cand: the collected elements.
+// slacks s and u; cand: the collected elements.
 template <class T>
 __device__ __forceinline__ void exact_candidates(const T &t, ExactSmem &xs, ExactQueue &Q, const ExactRow &R,
-                                                 const FlatRows &F, const ExactSums &S, bool go, double s, double u,
-                                                 int cand, int lane, int *row_tight = nullptr) {
+                                                 const ExactSums &S, bool go, double s, double u, int cand, int lane,
+                                                 int *row_tight = nullptr) {
     if (!__any_sync(kFull, go)) return;
     if (R.in) {
         const bool rhs_ok = !posinf_bits(dbits(R.rhs)) && !neginf_bits(dbits(S.minact));
         const bool lhs_ok = !neginf_bits(dbits(R.lhs)) && !posinf_bits(dbits(S.maxact));
         xs.slack[lane] = s;
         xs.nsur[lane] = u;
-        xs.info[lane] = (rhs_ok ? 1u : 0u) | (lhs_ok ? 2u : 0u) | (unsigned)min(R.minf, 3) << 2 |
-                        (unsigned)min(R.maxf, 3) << 4 | (go ? 64u : 0u);
+        xs.info[lane] = (unsigned char)((rhs_ok ? 1 : 0) | (lhs_ok ? 2 : 0) | min(R.minf, 3) << 2 |
+                                        min(R.maxf, 3) << 4 | (go ? 64 : 0));
     }
     __syncwarp();
     if (cand <= kCandCap) {
         for (int i0 = 0; i0 < cand; i0 += 32) {
             const int i = i0 + lane;
-            const bool on = i < cand && (xs.info[xs.cand_s[i] & 127] & 64u);
-            const int c = on ? xs.cand_s[i] : 0;
-            exact_push(t, xs, Q, on, on ? xs.cand_k[i] : 0, c & 127, c & 128, on ? xs.cand_d[i] : 0.0, lane,
-                       row_tight);
+            const int slot = i < cand ? xs.cand_s[i] : 0;
+            const bool on = i < cand && (xs.info[slot] & 64);
+            exact_push(t, xs, Q, on, on ? xs.cand_k[i] : 0, slot, lane, row_tight);
         }
     } else {  // more than the list holds: every element of the rows again
+        const FlatRows F = flat_rows(R, lane);
+        if (R.in) xs.src[lane] = R.base - F.pre;
+        __syncwarp();
         for (int f0 = 0; f0 < F.total; f0 += 32) {
-            const int slot = flat_slot(F, f0, lane), f = f0 + lane;
-            const bool on = f < F.total && (xs.info[slot] & 64u);
-            int k = 0;
-            bool pos = false;
-            double d = 0.0;
-            if (on) {
-                k = xs.src[slot] + f;
-                const double a = __ldg(t.val + k);
-                const double2 b = t.bnd[__ldg(t.col + k)];
-                pos = gt0_bits(dbits(a));
-                d = dmul(fabs(a), dsub(b.y, b.x));
-            }
-            exact_push(t, xs, Q, on, k, slot, pos, d, lane, row_tight);
+            const int slot = max(flat_slot(F, f0, lane), 0), f = f0 + lane;
+            const bool on = f < F.total && (xs.info[slot] & 64);
+            exact_push(t, xs, Q, on, on ? xs.src[slot] + f : 0, slot, lane, row_tight);
         }
     }
 }

@@ -50,7 +50,7 @@ struct XRow {
     long long base;
     int pos, len;
     float slack_lo;  // the screen's lower bound of min(rhs - minact, maxact - lhs)
-    int pad;
+    int inf;         // infinite contributions, up to 3 each: minact in bits 0, 1, maxact in bits 2, 3
 };
 
 // FP32 screen partial of a split-row tile (see Scr in gdp_device.cuh).
@@ -163,13 +163,12 @@ struct DevProblem {
     unsigned mark_threshold;
     // deferred exact pass (single-problem kernels): rows the FP32 screen
     // cannot skip are queued per lanes-per-row class (log2 g = 0..5) and run in
-    // the next phase 32/g rows per warp, so the FP64 pipe sees full warps.
+    // the next phase, so the FP64 pipe sees full warps.
     // Class lg's queue is xrow[cls_begin[lg] .. cls_end[lg]) (its row positions
     // are exactly that range, slices being sorted by g).
-    int defer_exact;
     int cls_begin[6], cls_end[6];
     XRow *xrow;            // n_srows
-    unsigned *xctr;        // [parity * 16 + lg]: queue tails, [parity * 16 + 8 + lg]: pull counters
+    unsigned *xctr;        // [parity * 16 + lg]: queue tails, [parity * 16 + 8]: claimed items
     // learned marking (SELL rows; null when no model is attached). learned:
     // 1 = rounds process the marked rows the model selects, 2 = trace (every
     // marked row is processed and logged with its label).
@@ -208,7 +207,7 @@ struct DevProblem {
     unsigned *chg;         // changed-variable bitmap, n_chg_words words
     int n_chg_words;
     RoundFlags *flags;
-    unsigned *barrier;     // megakernel grid barrier {count, generation}
+    unsigned *barrier;     // megakernel grid barrier: arrivals
     unsigned *queue;       // work counters: [parity * 4 + phase]
     int max_rounds;
     long long spin_limit;  // clock64 cycles one grid-barrier wait may last (gdp_options.barrier_wait_kcycles)

@@ -37,11 +37,10 @@ namespace {
 __device__ __forceinline__ void learned_activity_phase(const DevProblem &P, int round, int kind, unsigned *ctr,
                                                        int *change, unsigned *tight_ctr, WarpSmem &ws,
                                                        LearnSmem &L, int lane, unsigned long long *marked_ctr) {
-    stats_zero(ws, lane);
     if (lane == 0) L.marked = 0;
     __syncwarp();
-    WarpCursor cur;
-    cur.start(ctr, 1u, lane);
+    WarpCursor<true> cur;
+    cur.start(ctr, 1, grid_warps(), P.n_items);
     for (;;) {
         const int i = cur.next(lane);
         if (i >= P.n_items) break;
@@ -49,7 +48,6 @@ __device__ __forceinline__ void learned_activity_phase(const DevProblem &P, int 
         if (it >= 0) sell_slice_learned<1>(P, it, lane, round, kind, change, tight_ctr, ws, L);
         else split_partial<1>(P, -it - 1, lane, round, kind != kRoundFull, change, tight_ctr, ws);
     }
-    stats_flush(P, ws, lane);
     if (lane == 0 && L.marked) atomicAdd(marked_ctr, L.marked);
 }
 
@@ -83,14 +81,16 @@ __device__ __forceinline__ void learned_finalize(const DevProblem &P, int round,
     flush_changed(P, changed);
 }
 
-__global__ void __launch_bounds__(kCtaThreads, 3) k_megakernel_learned(DevProblem P) {
-    __shared__ WarpSmem ws[kWarpsPerCta];
+__global__ void __launch_bounds__(kCtaThreads, 3) k_megakernel_learned(const __grid_constant__ DevProblem P) {
+    WarpSmem *ws = warp_smem();
     __shared__ LearnSmem ls[kWarpsPerCta];
     const int lane = threadIdx.x & 31;
     WarpSmem &mine = ws[threadIdx.x >> 5];
     LearnSmem &L = ls[threadIdx.x >> 5];
     int *err = &P.flags[0].error;
     int last_change = 0;
+    unsigned target = 0;  // grid barrier
+    stats_zero(mine, lane);
     int kind = kRoundFull;  // round 1 processes every row
     if (*((volatile int *)&P.flags[0].infeasible) == 0) {
         for (int round = 1; round <= P.max_rounds; round++) {
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_megakernel_learned(DevProble
             const bool full = kind == kRoundFull;
             learned_activity_phase(P, round, kind, q + 0, change, tight, mine, L, lane,
                                    &P.flags[1 + par].rows_deferred);
-            if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+            if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 P.flags[1 + (par ^ 1)].change = 0;
                 P.flags[1 + (par ^ 1)].tight = 0u;
@@ -114,11 +114,11 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_megakernel_learned(DevProble
                 if (full) P.flags[0].full_rounds += 1;
             }
             if (P.n_mtiles) {
-                candidate_phase(P, round, !full, q + 1, exact, mine, lane);
-                if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+                candidate_phase(P, round, !full, exact, mine, lane);
+                if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
                 if (*((volatile int *)exact)) {
-                    exact_phase(P, round, q + 2, change, tight, mine, lane);
-                    if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+                    exact_phase(P, round, change, tight, mine, lane);
+                    if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
                 }
             }
             const unsigned t = *((volatile unsigned *)tight);
@@ -129,13 +129,14 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_megakernel_learned(DevProble
             learned_finalize(P, round, !certified && next != kRoundFull && round < P.max_rounds,
                              blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
             if (blockIdx.x == 0 && threadIdx.x == 0) P.flags[0].rounds = round;
-            if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+            if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             last_change = *((volatile int *)change);
             const int infeasible = *((volatile int *)&P.flags[0].infeasible);
             if (certified || infeasible) break;
             kind = next;
         }
     }
+    stats_flush(P, mine, lane);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         P.flags[0].change = last_change;
         P.flags[0].done = 1;
@@ -162,11 +163,15 @@ int launch_learned(const DevProblem &P, int grid, int vec_blocks, cudaStream_t s
     DevProblem Pc = P;
     void *args[] = {&Pc};
     return (int)cudaLaunchCooperativeKernel((const void *)k_megakernel_learned, dim3(grid), dim3(kCtaThreads), args,
-                                            0, s);
+                                            kCtaSmem, s);
 }
 
 int learned_occupancy(int *blocks_per_sm) {
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_megakernel_learned, kCtaThreads, 0);
+    const cudaError_t e = cudaFuncSetAttribute(k_megakernel_learned, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kCtaSmem);
+    if (e != cudaSuccess) return (int)e;
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_megakernel_learned, kCtaThreads,
+                                                              kCtaSmem);
 }
 
 }  // namespace gdp

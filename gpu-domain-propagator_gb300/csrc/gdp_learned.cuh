@@ -89,7 +89,7 @@ __device__ __forceinline__ bool sell_slice_learned(const DevProblem &P, int slic
     // a row the model can ever score: its state (features of later rounds) is kept
     const bool scored_row = P.learned == 2 || len >= P.learn_min_len;
     const bool decide = select && leader0 && scored_row && round - P.dirty[r] < kMaxDeferRounds;
-    __nv_bfloat16 (*feat)[16] = reinterpret_cast<__nv_bfloat16 (*)[16]>(ws.q);
+    __nv_bfloat16 (*feat)[16] = reinterpret_cast<__nv_bfloat16 (*)[16]>(ws.xs.div);
     unsigned trace_idx = 0xffffffffu;
     const bool any_decide = __any_sync(kFull, decide);  // every lane, outside any condition
     if (logged || (select && any_decide)) {
@@ -176,17 +176,11 @@ __device__ __forceinline__ bool sell_slice_learned(const DevProblem &P, int slic
         }
     }
     count_work(ws, lane, leader ? 1 : 0, leader ? len : 0, (leader && exact) ? len : 0);
-    exact = __shfl_sync(kFull, exact, rl << lg) && act;
     __syncwarp();
-    if (__any_sync(kFull, exact)) {
-        ws.base[lane] = base;
-        __syncwarp();
-        sell_rows_exact<kRec>(P, sell_view(P), lg, lane, exact, len, cnt, lhs, rhs, r, slack_lo, change, tight_ctr, ws,
-                        L.tight, L.go);
-    }
+    exact_slice(P, ws, lg, exact, r, len, slack_lo, c.minf, c.maxf, lhs, rhs, lane, change, tight_ctr, L.tight, L.go);
     __syncwarp();
     if (leader) {
-        const bool tightened = L.tight[rl] > 0;
+        const bool tightened = L.tight[rl] != 0;
         if (logged && trace_idx < P.trace_cap) P.trace_y[trace_idx] = tightened ? 1.f : 0.f;
         if (scored_row) {  // rows the model never scores need no feature state
             const unsigned old = P.rinfo[r];

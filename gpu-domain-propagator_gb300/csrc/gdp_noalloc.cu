@@ -212,14 +212,20 @@ __device__ __forceinline__ bool bit_of(const unsigned *map, int j) { return (map
 
 // ---- shared memory of a warp ------------------------------------------------------
 // The chunk's screen stages its copies where the exact pass stages its terms.
+constexpr int kStage = 64;   // elements the exact pass stages at a time
+constexpr int kNaRows = 16;  // rows of an item of the exact pass
 struct NaWarp {
     ExactSmem xs;
+    double t[2][kStage];  // minimum / maximum activity terms
+    double d[kStage];     // |a| (ub - lb)
     int src[32];
     unsigned char own[32];  // lanes of the rows that take the exact pass
 };
-__device__ __forceinline__ float *stage_a(NaWarp &ws) { return reinterpret_cast<float *>(ws.xs.t[0]); }
-__device__ __forceinline__ float2 *stage_b(NaWarp &ws) { return reinterpret_cast<float2 *>(ws.xs.t[1]); }
-static_assert(sizeof(float2) * kStage <= sizeof(double) * kStage, "the copies fit the staging area");
+constexpr int kScreenStage = 128;  // elements the screen stages at a time
+__device__ __forceinline__ float2 *stage_b(NaWarp &ws) { return reinterpret_cast<float2 *>(ws.t[0]); }
+__device__ __forceinline__ float *stage_a(NaWarp &ws) { return reinterpret_cast<float *>(ws.d); }
+static_assert(sizeof(float2) * kScreenStage <= sizeof(NaWarp::t) && sizeof(float) * kScreenStage <= sizeof(NaWarp::d),
+              "the copies fit the staging area");
 
 // A flat list over the chunk's rows: the lanes with `in` set hold rows of `len`
 // elements whose first is at CSR index b and at flat index pre; ws.src[rank]
@@ -279,8 +285,80 @@ struct NaTarget {
     }
 };
 
+// Left-to-right activities and first maximum of an item of up to kNaRows rows.
+// The rows are one flat list of elements, kStage staged at a time: 32 lanes
+// form the products of 32 consecutive elements, whichever rows they belong
+// to, then lane 2 r adds up row r's minimum activity and lane 2 r + 1 its
+// maximum activity, so a long row costs one FP64 add per element.
+__device__ __forceinline__ ExactSums flat_sums(const NaTarget &t, NaWarp &ws, const ExactRow &R, int lane, int &cand) {
+    ExactSmem &xs = ws.xs;
+    const FlatRows F = flat_rows(R, lane);
+    __syncwarp();
+    if (R.in) xs.src[lane] = R.base - F.pre;
+    __syncwarp();
+    const int side = lane & 1, mine = lane >> 1;
+    const int rpre = __shfl_sync(kFull, F.pre, mine), rlen = __shfl_sync(kFull, F.len, mine);
+    const long long my_cut = candidate_cut(R.slack_lo);
+    double acc = 0.0;
+    long long km = 0;
+    int p = -1, e = 0;
+    cand = 0;
+    constexpr int kSteps = kStage / 32;
+    int k[kSteps], slots[kSteps], j[kSteps];
+    double a[kSteps];
+    auto load = [&](int w0) {  // element indices, columns and coefficients of a window
+#pragma unroll
+        for (int i = 0; i < kSteps; i++) {
+            slots[i] = flat_slot(F, w0 + 32 * i, lane);
+            const int f = w0 + 32 * i + lane;
+            k[i] = f < F.total ? xs.src[slots[i]] + f : -1;
+            j[i] = k[i] >= 0 ? __ldg(t.col + k[i]) : 0;
+            a[i] = k[i] >= 0 ? __ldg(t.val + k[i]) : 0.0;
+        }
+    };
+    load(0);
+    for (int w0 = 0; w0 < F.total; w0 += kStage) {
+        double2 b[kSteps];
+#pragma unroll
+        for (int i = 0; i < kSteps; i++) b[i] = k[i] >= 0 ? t.bnd[j[i]] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < kSteps; i++) {
+            if (w0 + 32 * i >= F.total) break;  // warp-uniform
+            double d;
+            exact_terms(a[i], b[i], ws.t[0][32 * i + lane], ws.t[1][32 * i + lane], d);
+            ws.d[32 * i + lane] = d;
+            const long long db = dbits(d);
+            const long long cut = __shfl_sync(kFull, my_cut, max(slots[i], 0));
+            const bool keep = k[i] >= 0 && (order_key(db) > cut ||
+                                            (db & 0x7FF0000000000000LL) == 0x7FF0000000000000LL);
+            collect(xs, cand, keep, k[i], slots[i], lane);
+        }
+        if (w0 + kStage < F.total) load(w0 + kStage);  // in flight while this window is added up
+        __syncwarp();
+        const int end = min(rlen, w0 + kStage - rpre);  // elements of my row staged so far
+        const int at = rpre - w0;  // staged index of my row's element 0
+#pragma unroll 4
+        for (; e < end; e++) {
+            acc = dadd(acc, ws.t[side][at + e]);
+            const long long kd = order_key(dbits(ws.d[at + e]));
+            if (kd > km && kd <= kKeyPosInf) {
+                km = kd;
+                p = e;
+            }
+        }
+        __syncwarp();
+    }
+    ExactSums s;
+    const int lead = R.in ? 2 * lane : 0;
+    s.minact = __shfl_sync(kFull, acc, lead);
+    s.maxact = __shfl_sync(kFull, acc, lead + 1);
+    s.km = __shfl_sync(kFull, km, lead);
+    s.p = __shfl_sync(kFull, p, lead);
+    return s;
+}
+
 // The exact pass of the rows of `rows` (lanes; each holds its row's CSR start
-// b, length and the screen's results), kItemRows at a time.
+// b, length and the screen's results), kNaRows at a time.
 __device__ __forceinline__ void exact_rows(const Csr &A, const NoallocView &S, const NaTarget &T, NaWarp &ws,
                                            ExactQueue &Q, unsigned rows, int row0, int b, int len, float slack_lo,
                                            int minf, int maxf, int lane) {
@@ -288,9 +366,9 @@ __device__ __forceinline__ void exact_rows(const Csr &A, const NoallocView &S, c
     __syncwarp();
     if ((rows >> lane) & 1u) ws.own[__popc(rows & ((1u << lane) - 1u))] = (unsigned char)lane;
     __syncwarp();
-    for (int i0 = 0; i0 < n; i0 += kItemRows) {
+    for (int i0 = 0; i0 < n; i0 += kNaRows) {
         ExactRow R;
-        R.in = lane < kItemRows && i0 + lane < n;
+        R.in = lane < kNaRows && i0 + lane < n;
         const int own = R.in ? ws.own[i0 + lane] : 0;
         R.base = __shfl_sync(kFull, b, own);
         R.len = __shfl_sync(kFull, len, own);
@@ -299,9 +377,8 @@ __device__ __forceinline__ void exact_rows(const Csr &A, const NoallocView &S, c
         R.maxf = __shfl_sync(kFull, maxf, own);
         R.lhs = R.in ? __ldg(A.lhs + row0 + own) : 0.0;
         R.rhs = R.in ? __ldg(A.rhs + row0 + own) : 0.0;
-        const FlatRows F = flat_rows(R, lane);
         int cand;
-        const ExactSums X = exact_sums(T, ws.xs, R, F, 0, lane, cand);
+        const ExactSums X = flat_sums(T, ws, R, lane, cand);
         double s = 0.0, t = 0.0, mn = 0.0;
         int dec = 0;
         if (R.in) {
@@ -316,7 +393,7 @@ __device__ __forceinline__ void exact_rows(const Csr &A, const NoallocView &S, c
                                          __shfl_sync(kFull, X.p, q), lane);
             if (lane == q) dec = eps_le(m, mn) ? 0 : 1;
         }
-        exact_candidates(T, ws.xs, Q, R, F, X, R.in && dec == 1, s, t, cand, lane);
+        exact_candidates(T, ws.xs, Q, R, X, R.in && dec == 1, s, t, cand, lane);
     }
 }
 
@@ -380,13 +457,13 @@ __device__ __forceinline__ void na_chunk(const Csr &A, const NoallocView &S, con
     scr_init(c);
     unsigned hits = 0u;
     const Flat F = flat_of(ws, small, b, len, lane);
-    for (int w0 = 0; w0 < F.total; w0 += kStage) {
-        int j[kStage / 32];
-        double a[kStage / 32];
-        double2 bb[kStage / 32];
-        bool ok[kStage / 32], hit[kStage / 32];
+    for (int w0 = 0; w0 < F.total; w0 += kScreenStage) {
+        int j[kScreenStage / 32];
+        double a[kScreenStage / 32];
+        double2 bb[kScreenStage / 32];
+        bool ok[kScreenStage / 32], hit[kScreenStage / 32];
 #pragma unroll
-        for (int i = 0; i < kStage / 32; i++) {
+        for (int i = 0; i < kScreenStage / 32; i++) {
             const int f0 = w0 + 32 * i;
             const int rank = flat_rank(F, f0, lane);
             ok[i] = f0 + lane < F.total;
@@ -395,18 +472,18 @@ __device__ __forceinline__ void na_chunk(const Csr &A, const NoallocView &S, con
             a[i] = ok[i] ? __ldg(A.val + k) : 0.0;
         }
 #pragma unroll
-        for (int i = 0; i < kStage / 32; i++) {
+        for (int i = 0; i < kScreenStage / 32; i++) {
             bb[i] = ok[i] ? S.cur[j[i]] : make_double2(0.0, 0.0);
             hit[i] = ok[i] && bit_of(prev, j[i]);
         }
 #pragma unroll
-        for (int i = 0; i < kStage / 32; i++) {
+        for (int i = 0; i < kScreenStage / 32; i++) {
             hits |= __ballot_sync(kFull, hit[i]) & flat_range(F, w0 + 32 * i);
             stage_a(ws)[32 * i + lane] = coef_screen_bits(a[i]);
             stage_b(ws)[32 * i + lane] = bnd_screen_bits(bb[i]);
         }
         __syncwarp();
-        const int lo = max(F.pre - w0, 0), hi = F.in ? min(F.pre + F.len - w0, kStage) : 0;
+        const int lo = max(F.pre - w0, 0), hi = F.in ? min(F.pre + F.len - w0, kScreenStage) : 0;
         for (int i = lo; i < hi; i++) scr_add(c, stage_a(ws)[i], stage_b(ws)[i]);
         __syncwarp();
     }
@@ -522,7 +599,7 @@ __device__ __forceinline__ void na_long_row(const Csr &A, const NoallocView &S, 
         for (int i = 0; i < kStage / 32; i++)
             if (j[i] >= 0) {
                 double d;
-                exact_terms(a[i], bb[i], wss[wid].xs.t[0][32 * i + lane], wss[wid].xs.t[1][32 * i + lane], d);
+                exact_terms(a[i], bb[i], wss[wid].t[0][32 * i + lane], wss[wid].t[1][32 * i + lane], d);
                 const long long kd = order_key(dbits(d));
                 if (kd > km && kd <= kKeyPosInf) {
                     km = kd;
@@ -534,7 +611,7 @@ __device__ __forceinline__ void na_long_row(const Csr &A, const NoallocView &S, 
             for (int w = 0; w < kNaWarps && w0 + w * kStage < len; w++) {
                 const int n = (int)min(len - w0 - w * kStage, (unsigned)kStage);
 #pragma unroll 8
-                for (int i = 0; i < n; i++) acc = dadd(acc, wss[w].xs.t[lane][i]);
+                for (int i = 0; i < n; i++) acc = dadd(acc, wss[w].t[lane][i]);
             }
         __syncthreads();
     }
@@ -581,21 +658,10 @@ __device__ __forceinline__ void na_long_row(const Csr &A, const NoallocView &S, 
         // the row in slot 0 of every warp; each warp tests its share of the elements
         ExactSmem &xs = wss[wid].xs;
         R.in = lane == 0;
-        FlatRows F;
-        F.pre = 0;
-        F.len = F.total = 0;
-        exact_candidates(T, xs, Q, R, F, bs.sums, lane == 0, bs.s, bs.t, 0, lane);  // the row's constants alone
+        exact_candidates(T, xs, Q, R, bs.sums, lane == 0, bs.s, bs.t, 0, lane);  // the row's constants alone
         for (unsigned o0 = 32 * wid; o0 < len; o0 += kNaThreads) {
             const unsigned o = o0 + lane;
-            bool pos = false;
-            double d = 0.0;
-            if (o < len) {
-                const double a = __ldg(A.val + b + o);
-                const double2 bb = T.bnd[__ldg(A.col + b + o)];
-                pos = gt0_bits(dbits(a));
-                d = dmul(fabs(a), dsub(bb.y, bb.x));
-            }
-            exact_push(T, xs, Q, o < len, (int)(b + o), 0, pos, d, lane, nullptr);
+            exact_push(T, xs, Q, o < len, o < len ? (int)(b + o) : 0, 0, lane, nullptr);
         }
     }
     __syncthreads();  // bs and the staging areas are free for the next row
@@ -622,6 +688,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
     const int n_long = st->n_long <= kLongCap ? (int)st->n_long : 0;
     const int long_len = n_long == (int)st->n_long ? kLongRow : INT_MAX;
     int last_tight = 0;
+    unsigned target = 0;  // grid barrier
     for (int round = 1; round <= max_rounds; round++) {
         const int par = round & 1;
         const unsigned *prev = S.chg[par ^ 1];
@@ -640,7 +707,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
         }
         exact_drain(T, ws.xs, Q, true, lane);
         if (__any_sync(kFull, Q.tight) && lane == 0) st->tight[par] = 1;
-        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit)) return;
+        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit, target)) return;
         // commit: the caller's arrays hold the round's result
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             st->claim[par ^ 1] = 0u;
@@ -669,7 +736,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
             atomicAdd(&st->changed[par], (unsigned)changed);
             atomicAdd(&st->flags.changed_vars, (unsigned long long)changed);
         }
-        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit)) return;
+        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit, target)) return;
         last_tight = *((volatile int *)&st->tight[par]);
         if (!last_tight || *((volatile int *)&st->flags.infeasible)) break;
     }

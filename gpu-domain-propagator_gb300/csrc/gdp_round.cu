@@ -10,34 +10,42 @@ namespace gdp {
 
 namespace {
 
+// Shared memory of 24 warps (and 1 KB the system keeps per CTA) as a share of
+// the 228 KB per SM, in percent.
+constexpr int kCarveout = (int)((24 * sizeof(WarpSmem) + 6 * 1024) * 100 / (228 * 1024) + 1);
+
 // ---- phase kernels (CPU_LOOP / GPU_LOOP) -----------------------------------
-__global__ void __launch_bounds__(kCtaThreads, 4) k_activity(DevProblem P) {
-    __shared__ WarpSmem ws[kWarpsPerCta];
+__global__ void __launch_bounds__(kCtaThreads, 4) k_activity(const __grid_constant__ DevProblem P) {
+    WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible) return;
+    stats_zero(ws[threadIdx.x >> 5], threadIdx.x & 31);
     activity_phase(P, round, P.flags[0].mark_cur != 0, P.queue + 0, &P.flags[0].change, &P.flags[0].tight,
                    ws[threadIdx.x >> 5], threadIdx.x & 31);
+    stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
-__global__ void __launch_bounds__(kCtaThreads, 4) k_candidates(DevProblem P) {
-    __shared__ WarpSmem ws[kWarpsPerCta];
+__global__ void __launch_bounds__(kCtaThreads, 4) k_candidates(const __grid_constant__ DevProblem P) {
+    WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible) return;
     // the multi-tile rows' tiles (1,024 non-zeros each) first, the deferred
     // exact rows (at most split_tile non-zeros, mostly short) after them: the
     // heavy items do not end up as the phase's tail
-    candidate_phase(P, round, P.flags[0].mark_cur != 0, P.queue + 1, &P.flags[0].exact, ws[threadIdx.x >> 5],
-                    threadIdx.x & 31);
+    stats_zero(ws[threadIdx.x >> 5], threadIdx.x & 31);
+    candidate_phase(P, round, P.flags[0].mark_cur != 0, &P.flags[0].exact, ws[threadIdx.x >> 5], threadIdx.x & 31);
     if (exact_rows_queued(P, 0))
         exact_rows_phase(P, 0, &P.flags[0].change, &P.flags[0].tight, ws[threadIdx.x >> 5], threadIdx.x & 31);
+    stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
-__global__ void __launch_bounds__(kCtaThreads, 4) k_exact(DevProblem P) {
-    __shared__ WarpSmem ws[kWarpsPerCta];
+__global__ void __launch_bounds__(kCtaThreads, 4) k_exact(const __grid_constant__ DevProblem P) {
+    WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible || P.flags[0].exact == 0) return;
-    exact_phase(P, round, P.queue + 2, &P.flags[0].change, &P.flags[0].tight, ws[threadIdx.x >> 5],
-                threadIdx.x & 31);
+    stats_zero(ws[threadIdx.x >> 5], threadIdx.x & 31);
+    exact_phase(P, round, &P.flags[0].change, &P.flags[0].tight, ws[threadIdx.x >> 5], threadIdx.x & 31);
+    stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
 // Every thread derives the same next-round mode from the final tightening count.
@@ -137,7 +145,9 @@ __device__ __forceinline__ void timer_stamp(const DevProblem &P, int round, int 
 // adds the warp's time in phase k of round r since t0 (0: A, 1: B multi-tile
 // rows, 2: B deferred exact rows, 3: C, 4: F), and keeps the longest single
 // warp's time of the phase group in slot 5 (A), 6 (B) or 7 (C and F)
-__device__ __forceinline__ void timer_busy(int lane, int round, int k, unsigned long long t0) {
+__device__ __forceinline__ void timer_busy(const DevProblem &P, WarpSmem &ws, int lane, int round, int k,
+                                           unsigned long long t0) {
+    stats_flush(P, ws, lane);  // the stamps read the work counters round by round
     if (lane == 0 && round < kTimerRounds) {
         const unsigned long long dt = timer_now() - t0;
         atomicAdd(&g_timer_busy[round * kTimerSlots + k], dt);
@@ -146,7 +156,7 @@ __device__ __forceinline__ void timer_busy(int lane, int round, int k, unsigned 
 }
 #else
 __device__ __forceinline__ void timer_stamp(const DevProblem &, int, int) {}
-__device__ __forceinline__ void timer_busy(int, int, int, unsigned long long) {}
+__device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, int, int, unsigned long long) {}
 #endif
 
 // Round loop on the device. flags[0] holds the sticky state; flags[1 + (round
@@ -158,12 +168,14 @@ __device__ __forceinline__ void timer_busy(int, int, int, unsigned long long) {}
 // W warps per CTA; with 24 / W resident CTAs per SM every instance holds about
 // 24 warps per SM under the same register budget.
 template <int W>
-__global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(DevProblem P) {
-    __shared__ WarpSmem ws[W];
+__global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_constant__ DevProblem P) {
+    WarpSmem *ws = warp_smem();
     const int lane = threadIdx.x & 31;
     WarpSmem &mine = ws[threadIdx.x >> 5];
     int *err = &P.flags[0].error;
     int last_change = 0;
+    unsigned target = 0;  // grid barrier
+    stats_zero(mine, lane);
     bool marked = false;  // round 1 processes every row
     if (*((volatile int *)&P.flags[0].infeasible) == 0) {
         for (int round = 1; round <= P.max_rounds; round++) {
@@ -175,8 +187,8 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(DevProblem P) {
             timer_stamp(P, round, 0);
             unsigned long long t0 = timer_now();
             activity_phase(P, round, marked, q + 0, change, tight, mine, lane, par);
-            timer_busy(lane, round, 0, t0);
-            if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+            timer_busy(P, mine, lane, round, 0, t0);
+            if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             timer_stamp(P, round, 1);
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 P.flags[1 + (par ^ 1)].change = 0;
@@ -191,33 +203,34 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(DevProblem P) {
             const bool xrows = exact_rows_queued(P, par);
             if (xrows || P.n_mtiles) {
                 t0 = timer_now();
-                if (P.n_mtiles) candidate_phase(P, round, marked, q + 1, exact, mine, lane);  // heavy items first
-                timer_busy(lane, round, 1, t0);
+                if (P.n_mtiles) candidate_phase(P, round, marked, exact, mine, lane);  // heavy items first
+                timer_busy(P, mine, lane, round, 1, t0);
                 t0 = timer_now();
                 if (xrows) exact_rows_phase(P, par, change, tight, mine, lane);
-                timer_busy(lane, round, 2, t0);
-                if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+                timer_busy(P, mine, lane, round, 2, t0);
+                if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
                 timer_stamp(P, round, 2);
                 if (P.n_mtiles && *((volatile int *)exact)) {
                     t0 = timer_now();
-                    exact_phase(P, round, q + 2, change, tight, mine, lane);
-                    timer_busy(lane, round, 3, t0);
-                    if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+                    exact_phase(P, round, change, tight, mine, lane);
+                    timer_busy(P, mine, lane, round, 3, t0);
+                    if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
                     timer_stamp(P, round, 3);
                 }
             }
             marked = next_round_marked(P, *((volatile unsigned *)tight));
             t0 = timer_now();
             finalize_words(P, round, marked, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-            timer_busy(lane, round, 4, t0);
+            timer_busy(P, mine, lane, round, 4, t0);
             if (blockIdx.x == 0 && threadIdx.x == 0) P.flags[0].rounds = round;
-            if (!grid_barrier(P.barrier, err, P.spin_limit)) return;
+            if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             timer_stamp(P, round, 4);
             last_change = *((volatile int *)change);
             const int infeasible = *((volatile int *)&P.flags[0].infeasible);
             if (!last_change || infeasible) break;
         }
     }
+    stats_flush(P, mine, lane);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         P.flags[0].change = last_change;
         P.flags[0].done = 1;
@@ -291,19 +304,18 @@ int launch_round_begin(const DevProblem &P, cudaStream_t s) {
 
 int launch_activity_phase(const DevProblem &P, int blocks, cudaStream_t s) {
     if (P.n_items == 0) return 0;
-    k_activity<<<blocks, kCtaThreads, 0, s>>>(P);
+    k_activity<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
     return (int)cudaGetLastError();
 }
 
 int launch_candidate_phase(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (P.n_mtiles == 0 && !P.defer_exact) return 0;
-    k_candidates<<<blocks, kCtaThreads, 0, s>>>(P);
+    k_candidates<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
     return (int)cudaGetLastError();
 }
 
 int launch_exact_phase(const DevProblem &P, int blocks, cudaStream_t s) {
     if (P.n_mtiles == 0) return 0;
-    k_exact<<<blocks, kCtaThreads, 0, s>>>(P);
+    k_exact<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
     return (int)cudaGetLastError();
 }
 
@@ -329,24 +341,27 @@ const void *megakernel_of(int cta_warps) {
 }  // namespace
 
 int phase_occupancy(int *act, int *cand, int *mega, int cta_warps) {
-    // the megakernel's shared memory (warp queues and row constants, ~3.6 KB
-    // per warp, ~24 warps per SM) is small: prefer a carveout that just holds
-    // it, the rest of the 256 KB per SM serving as L1 for the element streams
     const void *mk = megakernel_of(cta_warps);
-    cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
+    const size_t mega_smem = sizeof(WarpSmem) * (size_t)cta_warps;
+    cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mega_smem);
+    for (const void *k : {(const void *)k_activity, (const void *)k_candidates, (const void *)k_exact})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaSmem);
+    // a carveout that just holds 24 warps' shared memory, the rest of the
+    // 256 KB per SM serving as L1 for the element streams
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mk, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     if (e != cudaSuccess) return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(act, k_activity, kCtaThreads, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(act, k_activity, kCtaThreads, kCtaSmem);
     if (e != cudaSuccess) return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(cand, k_exact, kCtaThreads, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(cand, k_exact, kCtaThreads, kCtaSmem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(mega, mk, 32 * cta_warps, 0);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(mega, mk, 32 * cta_warps, mega_smem);
 }
 
 int launch_megakernel(const DevProblem &P, int grid, int cta_warps, cudaStream_t s) {
     DevProblem Pc = P;
     void *args[] = {&Pc};
-    return (int)cudaLaunchCooperativeKernel(megakernel_of(cta_warps), dim3(grid), dim3(32 * cta_warps), args, 0,
-                                            s);
+    return (int)cudaLaunchCooperativeKernel(megakernel_of(cta_warps), dim3(grid), dim3(32 * cta_warps), args,
+                                            sizeof(WarpSmem) * (size_t)cta_warps, s);
 }
 
 }  // namespace gdp
