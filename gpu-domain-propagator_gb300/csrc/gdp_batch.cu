@@ -66,51 +66,82 @@ __device__ __forceinline__ void push_tile(unsigned long long *q, unsigned *tail,
     q[idx] = ((unsigned long long)(unsigned)u << 32) | (unsigned)t;
 }
 
-// Queues row position p of unit u for round `stamp` (its mark is already set):
-// the slice holding it once per round, or every tile of a split row.
-__device__ __forceinline__ void queue_position(const BatchDev &B, const DevProblem &Pu, int u, int p, int stamp) {
+// The rows of the changed variables of a warp (lane l's variable if `on`, its
+// index entries [k0, k1)) of unit u are marked and queued for round `stamp`:
+// variable by variable, 32 entries at a time (a thread that walks its
+// variables' rows alone makes up to four dependent trips to L2 for each). A
+// slice is queued once per round, a split row with all its tiles; the queue
+// slots of a step's slices are reserved together. Learned units: SELL rows
+// turn dirty instead of marked (learned_mark_position).
+template <bool kLearned>
+__device__ __forceinline__ void push_rows(const BatchDev &B, const DevProblem &Pu, int u, bool on, int k0, int k1,
+                                          int stamp, int lane) {
     const int par = stamp & 1;
-    if (p < Pu.n_srows) {
-        const int s = __ldg(Pu.pos_slice + p);
-        if (atomicExch(Pu.slice_stamp + s, stamp) != stamp) push_entry(B, par, u, s);
-    } else {
-        const int row = p - Pu.n_srows;
-        for (int t = __ldg(Pu.lrow_tile0 + row); t < __ldg(Pu.lrow_tile0 + row + 1); t++) push_entry(B, par, u, -t - 1);
-    }
-}
-
-// Learned units: variable j of unit u changed; its SELL rows turn dirty and
-// their slices are queued for round `stamp`, its split rows are marked and
-// their tiles queued (as in learned_mark_position).
-__device__ __forceinline__ void mark_var_rows_learned(const BatchDev &B, const DevProblem &Pu, int u, int j,
-                                                      int stamp) {
-    for (int k = __ldg(Pu.var_ptr + j); k < __ldg(Pu.var_ptr + j + 1); k++) {
-        const int p = __ldg(&Pu.var_ent[k].pos);
-        if (p < Pu.n_srows) {
-            atomicAdd(Pu.dcount + p, 1);
-            if (Pu.dirty[p] == 0) atomicCAS(Pu.dirty + p, 0, stamp);
-            const int s = __ldg(Pu.pos_slice + p);
-            if (atomicExch(Pu.slice_stamp + s, stamp) != stamp) push_entry(B, stamp & 1, u, s);
-        } else if (atomicExch(Pu.mark + p, stamp) != stamp) {
-            queue_position(B, Pu, u, p, stamp);
+    unsigned long long *ent = B.entries + (size_t)par * B.cap_entries;
+    const unsigned long long unit = (unsigned long long)(unsigned)u << 32;
+    const bool lrn = kLearned && Pu.learned == 1;
+    for (unsigned vars = __ballot_sync(kFull, on && k0 < k1); vars; vars &= vars - 1) {
+        const int src = __ffs(vars) - 1;
+        const int e0 = __shfl_sync(kFull, k0, src), e1 = __shfl_sync(kFull, k1, src);
+        for (int e = e0; e < e1; e += 32) {
+            bool fresh = false;
+            int slice = 0;
+            if (e + lane < e1) {
+                const int p = __ldg(&Pu.var_ent[e + lane].pos);
+                if (p < Pu.n_srows) {
+                    slice = __ldg(Pu.pos_slice + p);
+                    if (lrn) {
+                        atomicAdd(Pu.dcount + p, 1);
+                        if (Pu.dirty[p] == 0) atomicCAS(Pu.dirty + p, 0, stamp);
+                    } else {
+                        Pu.mark[p] = stamp;
+                    }
+                    fresh = __ldcg(Pu.slice_stamp + slice) != stamp &&
+                            atomicExch(Pu.slice_stamp + slice, stamp) != stamp;
+                } else if (atomicExch(Pu.mark + p, stamp) != stamp) {
+                    const int row = p - Pu.n_srows;
+                    const int t0 = __ldg(Pu.lrow_tile0 + row), nt = __ldg(Pu.lrow_tile0 + row + 1) - t0;
+                    const unsigned at = atomicAdd(B.tail + par, (unsigned)nt);
+                    if ((unsigned long long)at + nt > B.cap_entries) atomicExch(B.error, (int)kErrQueueOverflow);
+                    else
+                        for (int t = 0; t < nt; t++) ent[at + t] = unit | (unsigned)(-(t0 + t) - 1);
+                }
+            }
+            const unsigned bal = __ballot_sync(kFull, fresh);
+            if (!bal) continue;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(B.tail + par, (unsigned)__popc(bal));
+            at = __shfl_sync(kFull, at, 0);
+            if ((unsigned long long)at + __popc(bal) > B.cap_entries) {
+                if (lane == 0) atomicExch(B.error, (int)kErrQueueOverflow);
+            } else if (fresh) {
+                ent[at + __popc(bal & ((1u << lane) - 1u))] = unit | (unsigned)slice;
+            }
         }
     }
 }
 
-// The warp turns to unit u (-1: none): statistics gathered for another unit go
-// to its flags.
-__device__ __forceinline__ void stats_unit(const BatchDev &B, WarpSmem &ws, int &unit, int u, int lane) {
-    if (unit == u) return;
-    if (unit >= 0) stats_flush(B.units[unit], ws, lane);
-    unit = u;
-}
-
-// Marks the rows of variable j of unit u for round `stamp` and queues them.
-__device__ __forceinline__ void mark_var_rows(const BatchDev &B, const DevProblem &Pu, int u, int j, int stamp) {
-    for (int k = __ldg(Pu.var_ptr + j); k < __ldg(Pu.var_ptr + j + 1); k++) {
-        const int p = __ldg(&Pu.var_ent[k].pos);
-        if (atomicExch(Pu.mark + p, stamp) != stamp) queue_position(B, Pu, u, p, stamp);
+// A warp's copy of the unit it works on, in shared memory: the fields are
+// pointers and sizes that do not change during the launch, and every access
+// through a unit in global memory is one more dependent load (from L2 after
+// each barrier). Turning to unit u, statistics gathered for another one go to
+// its flags.
+struct UnitCache {
+    alignas(16) unsigned char raw[sizeof(DevProblem)];
+};
+__device__ __forceinline__ const DevProblem &unit_of(const BatchDev &B, UnitCache &c, WarpSmem &ws, int &unit, int u,
+                                                     int lane) {
+    static_assert(sizeof(DevProblem) % 8 == 0 && alignof(DevProblem) <= 16, "copied by 8-byte words");
+    if (unit != u) {
+        if (unit >= 0) stats_flush(*reinterpret_cast<const DevProblem *>(c.raw), ws, lane);
+        __syncwarp();
+        const unsigned long long *src = reinterpret_cast<const unsigned long long *>(B.units + u);
+        unsigned long long *dst = reinterpret_cast<unsigned long long *>(c.raw);
+        for (int i = lane; i < (int)(sizeof(DevProblem) / 8); i += 32) dst[i] = __ldg(src + i);
+        __syncwarp();
+        unit = u;
     }
+    return *reinterpret_cast<const DevProblem *>(c.raw);
 }
 
 // One block builds the list of units swept in full in the next round, in
@@ -223,11 +254,13 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
     __shared__ LearnSmem ls[kLearned ? kWarpsPerCta : 1];
     const int lane = threadIdx.x & 31;
     WarpSmem &mine = ws[threadIdx.x >> 5];
+    __shared__ UnitCache units[kWarpsPerCta];
+    UnitCache &cache = units[threadIdx.x >> 5];
     LearnSmem &L = ls[kLearned ? (threadIdx.x >> 5) : 0];
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
     int last = 0;
     unsigned target = 0;  // grid barrier
-    int stat_unit = -1;   // unit that the warp's statistics belong to
+    int unit = -1;        // unit in the warp's cache, which its statistics belong to
     stats_zero(mine, lane);
     for (int r = 1; r <= B.max_rounds; r++) {
         const int par = r & 1;
@@ -262,8 +295,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
                     it = (int)(unsigned)e;
                     marked = true;
                 }
-                stats_unit(B, mine, stat_unit, u, lane);
-                const DevProblem &Pu = B.units[u];
+                const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
                 if (*((volatile int *)&Pu.flags[0].infeasible)) continue;
                 int *change = &Pu.flags[1 + par].change;
                 unsigned *tight = &Pu.flags[1 + par].tight;
@@ -293,7 +325,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
         // ---- B (plus the resets for round r + 1: its slots were last used in r - 1)
         if (gtid == 0) {
             unsigned *nctr = B.ctr + 4 * (par ^ 1);
-            nctr[0] = 0u; nctr[1] = 0u; nctr[2] = 0u;
+            nctr[0] = 0u; nctr[1] = 0u; nctr[2] = 0u; nctr[3] = 0u;
             B.tail[par] = 0u;  // round r's entry queue is consumed; it fills again in round r + 1
         }
         for (int u = gtid; u < B.n_units; u += gthreads) {
@@ -310,8 +342,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
                 if (i >= n_cq) break;
                 const unsigned long long e = B.cq[i];
                 const int u = (int)(e >> 32), t = (int)(unsigned)e;
-                stats_unit(B, mine, stat_unit, u, lane);
-                const DevProblem &Pu = B.units[u];
+                const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
                 if (split_cand<0>(Pu, t, lane, r, false, &Pu.flags[1 + par].exact, mine) && lane == 0)
                     push_tile(B.xq, B.tail + 3, B.cap_tiles, B.error, u, t);
             }
@@ -326,8 +357,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
                     if (i >= n_xq) break;
                     const unsigned long long e = B.xq[i];
                     const int u = (int)(e >> 32), t = (int)(unsigned)e;
-                    stats_unit(B, mine, stat_unit, u, lane);
-                    const DevProblem &Pu = B.units[u];
+                    const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
                     split_exact<0>(Pu, t, lane, r, &Pu.flags[1 + par].change, &Pu.flags[1 + par].tight, mine);
                 }
                 if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
@@ -369,30 +399,51 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
         if (kLearned)
             for (int u = gtid; u < B.n_units; u += gthreads)
                 if (B.units[u].learned == 1) B.units[u].flags[1 + (par ^ 1)].kind = unit_next_kind(B.units[u], r);
-        for (int w = gtid; w < B.total_words; w += gthreads) {
-            const int u = find_unit(B.wbase, B.n_units, w);
-            const DevProblem &Pu = B.units[u];
-            const int wl = w - __ldg(B.wbase + u);
-            unsigned bits = Pu.chg[wl];
-            if (!bits) continue;
-            Pu.chg[wl] = 0u;
-            atomicAdd(&Pu.flags[0].changed_vars, (unsigned long long)__popc(bits));  // per word, per unit
-            const bool lrn = kLearned && Pu.learned == 1;
-            const bool push = more && (lrn ? (!unit_certified(Pu, r) && unit_next_kind(Pu, r) != kRoundFull)
-                                           : unit_next_marked(Pu, r));
-            while (bits) {
-                const int j = wl * 32 + __ffs(bits) - 1;
-                bits &= bits - 1;
-                const double2 b = Pu.bnd_nxt[j];
-                Pu.bnd[j] = b;
-                store_bnd32<0>(Pu, j, b, r);
-                if (var_infeasible(b.x, b.y)) {
-                    Pu.flags[0].infeasible = 1;
-                    atomicMin(&Pu.flags[0].infeasible_var, j);
+        // the units' bitmaps are one array of words: a warp reads a few of them
+        // at a time, commits a word's 32 variables with a lane each and pushes
+        // their rows together
+        {
+            const int nw = grid_warps();
+            int gw = 1;  // words of a claim: about one claim per warp, at most 32 words
+            while (gw < 32 && 2LL * gw * nw <= B.total_words) gw <<= 1;
+            const int groups = (B.total_words + gw - 1) / gw;
+            WarpCursor<false> cur;
+            cur.start(ctr + 3, 1, nw, groups);
+            for (;;) {
+                const int grp = cur.next(lane);
+                if (grp >= groups) break;
+                const int w0 = grp * gw;
+                unsigned my = 0u;
+                if (lane < gw && w0 + lane < B.total_words) {
+                    my = __ldcg(B.chg + w0 + lane);
+                    if (my) B.chg[w0 + lane] = 0u;
                 }
-                if (push) {
-                    if (lrn) mark_var_rows_learned(B, Pu, u, j, r + 1);
-                    else mark_var_rows(B, Pu, u, j, r + 1);
+                for (unsigned words = __ballot_sync(kFull, my != 0u); words; words &= words - 1) {
+                    const int q = __ffs(words) - 1;
+                    const unsigned bits = __shfl_sync(kFull, my, q);
+                    const int u = find_unit(B.wbase, B.n_units, w0 + q);
+                    const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
+                    if (lane == 0) atomicAdd(&Pu.flags[0].changed_vars, (unsigned long long)__popc(bits));
+                    const bool lrn = kLearned && Pu.learned == 1;
+                    const bool push = more && (lrn ? (!unit_certified(Pu, r) && unit_next_kind(Pu, r) != kRoundFull)
+                                                   : unit_next_marked(Pu, r));
+                    const bool on = (bits >> lane) & 1u;
+                    int k0 = 0, k1 = 0;
+                    if (on) {
+                        const int j = (w0 + q - __ldg(B.wbase + u)) * 32 + lane;
+                        const double2 b = Pu.bnd_nxt[j];
+                        if (push) {
+                            k0 = __ldg(Pu.var_ptr + j);
+                            k1 = __ldg(Pu.var_ptr + j + 1);
+                        }
+                        Pu.bnd[j] = b;
+                        store_bnd32<0>(Pu, j, b, r);
+                        if (var_infeasible(b.x, b.y)) {
+                            Pu.flags[0].infeasible = 1;
+                            atomicMin(&Pu.flags[0].infeasible_var, j);
+                        }
+                    }
+                    if (push) push_rows<kLearned>(B, Pu, u, on, k0, k1, r + 1, lane);
                 }
             }
         }
@@ -404,7 +455,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
         const int pending = kLearned ? *((volatile int *)B.n_pending) : 0;
         if (!more || (next == 0 && pending == 0)) break;
     }
-    stats_unit(B, mine, stat_unit, -1, lane);
+    if (unit >= 0) stats_flush(*reinterpret_cast<const DevProblem *>(cache.raw), mine, lane);
     for (int u = gtid; u < B.n_units; u += gthreads) close_round(B, u, last);
     if (gtid == 0) B.rounds_out[0] = last;
 }
@@ -451,9 +502,20 @@ __global__ void __launch_bounds__(256) k_batch_seed_marks(BatchDev B, const doub
     const int u = blockIdx.y;
     const DevProblem &Pu = B.units[u];
     if (seed_mode[u] != 1 || Pu.flags[0].infeasible) return;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < Pu.n; j += gridDim.x * blockDim.x) {
-        const double2 a = Pu.bnd[j], b = ref[j];
-        if (dbits(a.x) != dbits(b.x) || dbits(a.y) != dbits(b.y)) mark_var_rows(B, Pu, u, j, 1);
+    const int lane = threadIdx.x & 31;
+    for (int j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); j0 < Pu.n; j0 += gridDim.x * blockDim.x) {
+        const int j = j0 + lane;
+        bool on = false;
+        int k0 = 0, k1 = 0;
+        if (j < Pu.n) {
+            const double2 a = Pu.bnd[j], b = ref[j];
+            on = dbits(a.x) != dbits(b.x) || dbits(a.y) != dbits(b.y);
+            if (on) {
+                k0 = __ldg(Pu.var_ptr + j);
+                k1 = __ldg(Pu.var_ptr + j + 1);
+            }
+        }
+        push_rows<false>(B, Pu, u, on, k0, k1, 1, lane);
     }
 }
 

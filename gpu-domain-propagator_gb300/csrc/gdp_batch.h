@@ -14,12 +14,13 @@ struct BatchDev {
     int n_units;
     const int *wbase;   // n_units + 1: first change-bitmap word of each unit in the batch's word space
     int total_words;
+    unsigned *chg;      // the units' change bitmaps, one after another (units[u].chg = chg + wbase[u])
     int max_rounds;
     unsigned long long *entries;  // 2 x cap_entries: (unit << 32 | work item) queued for a round, by parity
     unsigned cap_entries;
     unsigned long long *cq, *xq;  // tiles of multi-tile rows: candidate-phase / exact-phase queues
     unsigned cap_tiles;
-    unsigned *ctr;        // work counters [parity * 4 + phase]
+    unsigned *ctr;        // work counters [parity * 4 + phase] (A, B, C, F)
     unsigned *tail;       // [0], [1]: entries by parity; [2]: cq; [3]: xq
     int *fs_unit;         // units swept in full in the coming round
     int *fs_prefix;       // n_fs + 1: prefix of their work-item counts

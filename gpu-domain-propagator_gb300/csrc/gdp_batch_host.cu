@@ -97,13 +97,12 @@ GDP_RETCODE Batch::init_nodes(Context *ctx, int n_nodes) {
         Q.bnd = (double2 *)arena_.alloc_bytes(sizeof(double2) * (size_t)n);
         Q.bnd_nxt = (double2 *)arena_.alloc_bytes(sizeof(double2) * (size_t)n);
         Q.bnd32 = (float2 *)arena_.alloc_bytes(sizeof(float2) * (size_t)n);  // 8-byte copies
-        Q.chg = (unsigned *)arena_.alloc_bytes(sizeof(unsigned) * (size_t)std::max(S.n_chg_words, 1));
         Q.mark = (int *)arena_.alloc_bytes(sizeof(int) * (size_t)npos);
         Q.slice_stamp = (int *)arena_.alloc_bytes(sizeof(int) * (size_t)std::max(S.n_slices, 1));
         Q.tile_part = (TilePart *)arena_.alloc_bytes(sizeof(TilePart) * (size_t)std::max(S.n_tiles, 1));
         Q.tile_scr = (TileScr *)arena_.alloc_bytes(sizeof(TileScr) * (size_t)std::max(S.n_tiles, 1));
         Q.row_exact = (int *)arena_.alloc_bytes(sizeof(int) * (size_t)std::max(S.n_lrows, 1));
-        if (!Q.bnd || !Q.bnd_nxt || !Q.bnd32 || !Q.chg || !Q.mark || !Q.slice_stamp || !Q.tile_part || !Q.tile_scr ||
+        if (!Q.bnd || !Q.bnd_nxt || !Q.bnd32 || !Q.mark || !Q.slice_stamp || !Q.tile_part || !Q.tile_scr ||
             !Q.row_exact) {
             set_error("device allocation failed (node state)");
             return GDP_ERROR;
@@ -163,6 +162,7 @@ GDP_RETCODE Batch::finish_init(int device, int ctas_per_sm) {
     B_.units = (DevProblem *)dev(sizeof(DevProblem) * (size_t)n_units);
     B_.wbase = (const int *)dev(sizeof(int) * (size_t)(n_units + 1));
     B_.total_words = wbase[n_units];
+    B_.chg = (unsigned *)dev(sizeof(unsigned) * (size_t)B_.total_words);
     B_.max_rounds = max_rounds;
     B_.spin_limit = units_h_[0].spin_limit;
     B_.cap_entries = (unsigned)std::max<long long>(cap_entries, 1);
@@ -185,11 +185,12 @@ GDP_RETCODE Batch::finish_init(int device, int ctas_per_sm) {
     d_ub_ = (double *)dev(sizeof(double) * (size_t)total_vars_);
     d_var_base_ = (long long *)dev(sizeof(long long) * (size_t)(n_units + 1));
     d_seed_mode_ = (int *)dev(sizeof(int) * (size_t)n_units);
-    if (!B_.units || !B_.wbase || !B_.entries || !B_.cq || !B_.xq || !B_.ctr || !B_.tail || !B_.fs_unit ||
+    if (!B_.units || !B_.wbase || !B_.chg || !B_.entries || !B_.cq || !B_.xq || !B_.ctr || !B_.tail || !B_.fs_unit ||
         !B_.fs_prefix || !B_.n_fs || !B_.barrier || !misc || !d_lb_ || !d_ub_ || !d_var_base_ || !d_seed_mode_) {
         set_error("device allocation failed (batch)");
         return GDP_ERROR;
     }
+    for (int u = 0; u < n_units; u++) units_h_[u].chg = B_.chg + wbase[u];
     GDP_BCUDA(cudaMemcpyAsync(B_.units, units_h_.data(), sizeof(DevProblem) * (size_t)n_units,
                               cudaMemcpyHostToDevice, stream_));
     GDP_BCUDA(cudaMemcpyAsync((void *)B_.wbase, wbase.data(), sizeof(int) * (size_t)(n_units + 1),
