@@ -404,8 +404,8 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
         // their rows together
         {
             const int nw = grid_warps();
-            int gw = 1;  // words of a claim: about one claim per warp, at most 32 words
-            while (gw < 32 && 2LL * gw * nw <= B.total_words) gw <<= 1;
+            int gw = 1;  // words of a claim: about four claims per warp, at most 32 words
+            while (gw < 32 && 8LL * gw * nw <= B.total_words) gw <<= 1;
             const int groups = (B.total_words + gw - 1) / gw;
             WarpCursor<false> cur;
             cur.start(ctr + 3, 1, nw, groups);
