@@ -57,7 +57,7 @@ GDP_RETCODE propagate_once_impl(int n_cons, int n_vars, int nnz, const int *col,
     Context ctx;
     GDP_RETCODE rc = ctx.init(n_cons, n_vars, nnz, col, row_ptr, val, lhs, rhs, vartypes, opts);
     if (rc != GDP_OKAY) return rc;
-    rc = ctx.propagate_host(lbs, ubs, stats);
+    rc = ctx.propagate_host(lbs, ubs, lbs, ubs, stats);
     if (stats)
         stats->total_ms =
                 std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -249,7 +249,7 @@ GDP_RETCODE gdp_propagate(gdp_context *ctx, double *lbs, double *ubs, gdp_stats 
         if (!ctx || !lbs || !ubs) { gdp::set_error("null argument"); return GDP_ERROR; }
         const auto t0 = std::chrono::steady_clock::now();
         if (stats) *stats = gdp_stats{};
-        const GDP_RETCODE rc = ctx->impl.propagate_host(lbs, ubs, stats);
+        const GDP_RETCODE rc = ctx->impl.propagate_host(lbs, ubs, lbs, ubs, stats);
         if (stats)
             stats->total_ms =
                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -266,16 +266,7 @@ GDP_RETCODE gdp_propagate_into(gdp_context *ctx, const double *lbs_in, const dou
         }
         const auto t0 = std::chrono::steady_clock::now();
         if (stats) *stats = gdp_stats{};
-        const long long n = ctx->impl.n;
-        // chunked copies on the host threads (one thread copies a few GB/s)
-        const long long chunk = 1 << 16;
-#pragma omp parallel for schedule(static)
-        for (long long c = 0; c < (n + chunk - 1) / chunk; c++) {
-            const long long b = c * chunk, len = std::min(chunk, n - b);
-            if (lbs_out != lbs_in) std::memcpy(lbs_out + b, lbs_in + b, sizeof(double) * (size_t)len);
-            if (ubs_out != ubs_in) std::memcpy(ubs_out + b, ubs_in + b, sizeof(double) * (size_t)len);
-        }
-        const GDP_RETCODE rc = ctx->impl.propagate_host(lbs_out, ubs_out, stats);
+        const GDP_RETCODE rc = ctx->impl.propagate_host(lbs_in, ubs_in, lbs_out, ubs_out, stats);
         if (stats)
             stats->total_ms =
                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -48,7 +48,10 @@ public:
     ~Context();
     GDP_RETCODE init(int m, int n, int nnz, const int *col, const int *row_ptr, const double *val,
                      const double *lhs, const double *rhs, const int *vartype, const gdp_options *o);
-    GDP_RETCODE propagate_host(double *lbs, double *ubs, gdp_stats *st);
+    // Host bounds (an output may be its input); a failed call leaves the inputs
+    // in the outputs.
+    GDP_RETCODE propagate_host(const double *lbs_in, const double *ubs_in, double *lbs_out, double *ubs_out,
+                               gdp_stats *st);
     GDP_RETCODE propagate_device(double *d_lbs, double *d_ubs, cudaStream_t s, gdp_stats *st);
     // Loop driver, resident CTAs per SM (0: as many as fit) and megakernel CTA
     // size of later propagations; the layout stays.
@@ -67,7 +70,7 @@ public:
     RoundFlags *h_flags = nullptr;  // pinned
     Arena arena;
     DevProblem P{};
-    double *d_lb = nullptr, *d_ub = nullptr;  // staging for host bounds
+    double *d_lb = nullptr, *d_ub = nullptr;  // staging for host bounds (not with host_direct)
     int n_sms = 0, vec_blocks = 1, act_blocks = 1, cand_blocks = 1, mega_grid = 1, learned_grid = 1;
     int mega_warps = 8;  // warps per CTA of the megakernel (opts.cta_threads / 32)
     int n_srows = 0, n_slices = 0, n_lrows = 0, n_tiles = 0;
@@ -84,7 +87,8 @@ private:
                     cudaStream_t s, gdp_stats *st);
     GDP_RETCODE build_graph(cudaStream_t s);
     GDP_RETCODE rounds_cpu_loop(cudaStream_t s, int *launches);
-    GDP_RETCODE rounds_gpu_loop(cudaStream_t s, int *launches);
+    GDP_RETCODE rounds_gpu_loop(cudaStream_t s);
+    void copy_bounds(const double *lbs_in, const double *ubs_in, double *lbs_out, double *ubs_out) const;
     GDP_RETCODE rounds_megakernel(cudaStream_t s, int *launches);
     GDP_RETCODE rounds_learned(cudaStream_t s, int *launches);
     GDP_RETCODE alloc_learned_state();

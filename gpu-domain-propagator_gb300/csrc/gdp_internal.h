@@ -71,9 +71,9 @@ struct __align__(16) BndScr {
     int pad;
 };
 
-// Device-written round status. [0] is read by the host (CPU_LOOP), by the
-// graph's condition kernel (GPU_LOOP) and by every CTA of the megakernel;
-// [1], [2] are the megakernel's double-buffered per-round change flags.
+// Device-written round status. [0] is read by the host at the end, by the last
+// CTA of a graph's round (GPU_LOOP) and by every CTA of the megakernel; [1],
+// [2] are the megakernel's double-buffered per-round change flags.
 struct RoundFlags {
     int change;          // a candidate tightened some bound in the (last) round
     int infeasible;      // the infeasibility rule fired
@@ -207,8 +207,8 @@ struct DevProblem {
     unsigned *chg;         // changed-variable bitmap, n_chg_words words
     int n_chg_words;
     RoundFlags *flags;
-    unsigned *barrier;     // megakernel grid barrier: arrivals
-    unsigned *queue;       // work counters: [parity * 4 + phase]
+    unsigned *barrier;     // megakernel grid barrier: {arrivals, arrivals at the end of the last launch}
+    unsigned *queue;       // work counters: [parity * 4 + phase]; GPU_LOOP: [3] finished CTAs of the finalize kernel
     int max_rounds;
     long long spin_limit;  // clock64 cycles one grid-barrier wait may last (gdp_options.barrier_wait_kcycles)
 };
@@ -217,20 +217,20 @@ constexpr int kWarpsPerCta = 8;
 constexpr int kCtaThreads = 32 * kWarpsPerCta;
 
 // Launch helpers (gdp_round.cu). All return the cudaError_t of the launch.
-int launch_check_bounds(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_interleave(const DevProblem &P, const double *lb, const double *ub, int blocks, cudaStream_t s);
-int launch_copy_out(const double *lb, const double *ub, double *lb_out, double *ub_out, int n, int blocks,
-                    cudaStream_t s);
-int launch_deinterleave(const DevProblem &P, double *lb, double *ub, int blocks, cudaStream_t s);
-int launch_mark_all(const DevProblem &P, int blocks, cudaStream_t s);
+// Round state and bounds at the start of a propagation from lb / ub (two
+// kernels, one for small problems), and the result (unless the rounds ended
+// with a device error); both take host memory that the device reaches directly.
+int launch_start(const DevProblem &P, const double *lb, const double *ub, int blocks, cudaStream_t s);
+int launch_finish(const DevProblem &P, double *lb, double *ub, int blocks, cudaStream_t s);
 int launch_round_begin(const DevProblem &P, cudaStream_t s);
 int launch_activity_phase(const DevProblem &P, int blocks, cudaStream_t s);
 int launch_candidate_phase(const DevProblem &P, int blocks, cudaStream_t s);
 int launch_exact_phase(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_finalize(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_condition(const DevProblem &P, unsigned long long handle, cudaStream_t s);
-// cta_warps: 4, 8 or 16 warps per CTA of the megakernel
-int launch_megakernel(const DevProblem &P, int grid, int cta_warps, cudaStream_t s);
+int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, cudaStream_t s);
+// Rounds first .. last; mail (may be null) is host memory that receives {round,
+// whether another one follows} at the end of the launch. cta_warps: 4, 8 or 16
+// warps per CTA.
+int launch_megakernel(const DevProblem &P, int first, int last, int *mail, int grid, int cta_warps, cudaStream_t s);
 int phase_occupancy(int *act_blocks_per_sm, int *cand_blocks_per_sm, int *mega_blocks_per_sm, int cta_warps);
 // Phase timers of the megakernel (a library built with GDP_PHASE_TIMERS):
 // 0 or a CUDA error; -1 when the library was built without them.

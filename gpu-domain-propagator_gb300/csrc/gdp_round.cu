@@ -1,8 +1,9 @@
 // gdp_round.cu -- one Jacobi propagation round on sm_103a, as phase kernels
-// (CPU_LOOP and GPU_LOOP drivers) and as a persistent cooperative megakernel
-// that runs every round in one launch (MEGAKERNEL driver). The round's device
-// functions live in gdp_round.cuh.
+// (GPU_LOOP driver) and as a persistent cooperative megakernel that runs every
+// round in one launch (MEGAKERNEL driver) or one round per launch (CPU_LOOP).
+// The round's device functions live in gdp_round.cuh.
 #include <algorithm>
+#include <cstddef>
 
 #include "gdp_round.cuh"
 
@@ -14,7 +15,7 @@ namespace {
 // the 228 KB per SM, in percent.
 constexpr int kCarveout = (int)((24 * sizeof(WarpSmem) + 6 * 1024) * 100 / (228 * 1024) + 1);
 
-// ---- phase kernels (CPU_LOOP / GPU_LOOP) -----------------------------------
+// ---- phase kernels (GPU_LOOP) -----------------------------------
 __global__ void __launch_bounds__(kCtaThreads, 4) k_activity(const __grid_constant__ DevProblem P) {
     WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
@@ -48,38 +49,44 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_exact(const __grid_constant_
     stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
-// Every thread derives the same next-round mode from the final tightening count.
-__global__ void __launch_bounds__(256) k_finalize(DevProblem P) {
-    const bool push = next_round_marked(P, P.flags[0].tight);
-    finalize_words(P, P.flags[0].rounds, push, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-
-// Starts a round: counts it, takes the mode the previous finalize chose,
-// clears the change flag, tightening count and work counters (unless the
-// propagation is already infeasible).
-__global__ void k_round_begin(DevProblem P) {
-    if (P.flags[0].infeasible) return;
+// Starts a round: counts it, takes the mode that the finished round's
+// tightenings chose, clears the change flag, tightening count and work
+// counters. One thread.
+__device__ __forceinline__ void begin_round(const DevProblem &P) {
     const int r = P.flags[0].rounds;
     P.flags[0].mark_cur = r > 0 && next_round_marked(P, P.flags[0].tight);
     P.flags[0].change = 0;
     P.flags[0].tight = 0u;
     P.flags[0].exact = 0;
     P.flags[0].rounds = r + 1;
-    P.queue[0] = 0u;
-    P.queue[1] = 0u;
-    P.queue[2] = 0u;
-    if (P.xctr)
-        for (int i = 0; i < 16; i++) P.xctr[i] = 0u;
+    for (int i = 0; i < 4; i++) P.queue[i] = 0u;
+    for (int i = 0; i < 16; i++) P.xctr[i] = 0u;
 }
 
-// GPU_LOOP: decides whether the graph's WHILE node runs another round.
-__global__ void k_condition(DevProblem P, cudaGraphConditionalHandle h) {
-    const RoundFlags &f = P.flags[0];
-    const bool more = f.change && !f.infeasible && f.rounds < P.max_rounds;
+__global__ void k_round_begin(DevProblem P) {
+    if (!P.flags[0].infeasible) begin_round(P);
+}
+
+// Every thread derives the same next-round mode from the final tightening
+// count. The last CTA to finish (queue[3] counts them) decides whether the
+// graph's WHILE node runs another round, and starts it: two single-thread
+// kernels less per round (about 3 us of a 28 us round on 2,000 rows).
+__global__ void __launch_bounds__(256) k_finalize(DevProblem P, cudaGraphConditionalHandle h) {
+    const bool push = next_round_marked(P, P.flags[0].tight);
+    finalize_words(P, P.flags[0].rounds, push, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(P.queue + 3, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    volatile RoundFlags *f = P.flags;
+    const bool more = f->change && !f->infeasible && f->rounds < P.max_rounds;
+    if (more) begin_round(P);
     cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
-__global__ void __launch_bounds__(256) k_check_bounds(DevProblem P) {
+// The initial bounds' infeasibility check.
+__device__ __forceinline__ void check_bounds(const DevProblem &P) {
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < P.n; j += gridDim.x * blockDim.x) {
         const double2 b = P.bnd[j];
         if (var_infeasible(b.x, b.y)) {
@@ -88,43 +95,53 @@ __global__ void __launch_bounds__(256) k_check_bounds(DevProblem P) {
         }
     }
 }
+__global__ void __launch_bounds__(256) k_check_bounds(DevProblem P) { check_bounds(P); }
 
-__global__ void __launch_bounds__(256) k_interleave(DevProblem P, const double *lb, const double *ub) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < P.n; j += gridDim.x * blockDim.x) {
+// Everything that a propagation starts from: round state, bounds in the three
+// forms the rounds read, cleared bitmap, marks and drift bounds. lb / ub may
+// be host memory that the device reaches directly. A single CTA checks the
+// bounds itself.
+__global__ void __launch_bounds__(1024) k_start(DevProblem P, const double *lb, const double *ub) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    int *state = reinterpret_cast<int *>(P.flags);
+    for (int i = tid; i < (int)(3 * sizeof(RoundFlags) / sizeof(int)); i += nt)
+        state[i] = i == (int)(offsetof(RoundFlags, infeasible_var) / sizeof(int)) ||
+                                   i == (int)(offsetof(RoundFlags, infeasible_row) / sizeof(int))
+                           ? INT_MAX
+                           : 0;
+    if (tid < 8) P.queue[tid] = 0u;
+    if (tid < 32) P.xctr[tid] = 0u;
+    if (tid < 2) P.barrier[tid] = 0u;
+    for (int w = tid; w < P.n_chg_words; w += nt) P.chg[w] = 0u;
+    for (int r = tid; r < P.n_lrows; r += nt) {
+        P.row_exact[r] = 0;
+        P.lrow_margin[r] = -1.0;  // no drift bound carried over from an earlier propagation
+        P.lrow_drift[r] = 0.0;
+        P.lrow_skip[r] = 0;
+    }
+    if (P.use_marking)
+        for (int p = tid; p < P.n_srows + P.n_lrows; p += nt) P.mark[p] = 0;
+    for (int j = tid; j < P.n; j += nt) {
         const double2 b = make_double2(lb[j], ub[j]);
         P.bnd[j] = b;
         P.bnd_nxt[j] = b;
         store_bnd32<1>(P, j, b, 0);
     }
+    if (gridDim.x == 1) {
+        __syncthreads();
+        check_bounds(P);
+    }
 }
 
-__global__ void __launch_bounds__(256) k_deinterleave(DevProblem P, double *lb, double *ub) {
+// The result, unless the rounds ended with a device error. lb / ub may be host
+// memory that the device reaches directly.
+__global__ void __launch_bounds__(256) k_finish(DevProblem P, double *lb, double *ub) {
+    if (P.flags[0].error != kErrNone) return;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < P.n; j += gridDim.x * blockDim.x) {
         const double2 b = P.bnd[j];
         lb[j] = b.x;
         ub[j] = b.y;
     }
-}
-
-// Copies n bound pairs into the caller's arrays (host memory the device
-// reaches directly).
-__global__ void __launch_bounds__(256) k_copy_out(const double *lb, const double *ub, double *lb_out,
-                                                  double *ub_out, int n) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        lb_out[j] = lb[j];
-        ub_out[j] = ub[j];
-    }
-}
-
-__global__ void __launch_bounds__(256) k_mark_all(DevProblem P) {
-    const int npos = P.n_srows + P.n_lrows;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npos; p += gridDim.x * blockDim.x) P.mark[p] = 0;
-    if (P.lrow_margin)  // no drift bound carried over from an earlier propagation
-        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < P.n_lrows; r += gridDim.x * blockDim.x) {
-            P.lrow_margin[r] = -1.0;
-            P.lrow_drift[r] = 0.0;
-            P.lrow_skip[r] = 0;
-        }
 }
 
 // ---- megakernel -----------------------------------------------------------
@@ -167,18 +184,27 @@ __device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, 
 // previous round.
 // W warps per CTA; with 24 / W resident CTAs per SM every instance holds about
 // 24 warps per SM under the same register budget.
+// A launch runs the rounds first .. last, or fewer when one changes nothing or
+// turns infeasible; a launch after that one does nothing (flags[0].done), so
+// that a host loop may queue a round before it knows whether the round is
+// needed. Between launches barrier[1] keeps the barrier count and the round's
+// tightenings the next round's mode. mail (may be null): host memory that
+// receives {the round, whether another one follows}.
 template <int W>
-__global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_constant__ DevProblem P) {
+__global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_constant__ DevProblem P, int first,
+                                                               int last, int *mail) {
     WarpSmem *ws = warp_smem();
     const int lane = threadIdx.x & 31;
     WarpSmem &mine = ws[threadIdx.x >> 5];
     int *err = &P.flags[0].error;
-    int last_change = 0;
-    unsigned target = 0;  // grid barrier
+    if (P.flags[0].done || P.flags[0].error != kErrNone) return;
+    int last_change = 0, infeasible = P.flags[0].infeasible;
+    unsigned target = P.barrier[1];  // grid barrier
     stats_zero(mine, lane);
-    bool marked = false;  // round 1 processes every row
-    if (*((volatile int *)&P.flags[0].infeasible) == 0) {
-        for (int round = 1; round <= P.max_rounds; round++) {
+    // round 1 processes every row
+    bool marked = first > 1 && next_round_marked(P, P.flags[1 + ((first - 1) & 1)].tight);
+    if (infeasible == 0) {
+        for (int round = first; round <= last; round++) {
             const int par = round & 1;
             int *change = &P.flags[1 + par].change;
             unsigned *tight = &P.flags[1 + par].tight;
@@ -226,14 +252,21 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_cons
             if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             timer_stamp(P, round, 4);
             last_change = *((volatile int *)change);
-            const int infeasible = *((volatile int *)&P.flags[0].infeasible);
+            infeasible = *((volatile int *)&P.flags[0].infeasible);
             if (!last_change || infeasible) break;
         }
     }
     stats_flush(P, mine, lane);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const bool more = last_change && !infeasible;
         P.flags[0].change = last_change;
-        P.flags[0].done = 1;
+        P.flags[0].done = more ? 0 : 1;
+        P.barrier[1] = target;
+        if (mail) {
+            *((volatile int *)mail + 1) = more ? 1 : 0;
+            __threadfence_system();
+            *((volatile int *)mail) = P.flags[0].rounds;
+        }
     }
 }
 
@@ -269,31 +302,18 @@ int phase_timers_read(unsigned long long *wall, unsigned long long *busy, unsign
 
 // ---- launchers ------------------------------------------------------------
 
-int launch_check_bounds(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (P.n == 0) return 0;
+int launch_start(const DevProblem &P, const double *lb, const double *ub, int blocks, cudaStream_t s) {
+    if (blocks <= 32) {  // up to 8,192 variables or rows: one CTA, one launch
+        k_start<<<1, 1024, 0, s>>>(P, lb, ub);
+        return (int)cudaGetLastError();
+    }
+    k_start<<<blocks, 256, 0, s>>>(P, lb, ub);
     k_check_bounds<<<blocks, 256, 0, s>>>(P);
     return (int)cudaGetLastError();
 }
 
-int launch_interleave(const DevProblem &P, const double *lb, const double *ub, int blocks, cudaStream_t s) {
-    k_interleave<<<blocks, 256, 0, s>>>(P, lb, ub);
-    return (int)cudaGetLastError();
-}
-
-int launch_copy_out(const double *lb, const double *ub, double *lb_out, double *ub_out, int n, int blocks,
-                    cudaStream_t s) {
-    if (n > 0) k_copy_out<<<blocks, 256, 0, s>>>(lb, ub, lb_out, ub_out, n);
-    return (int)cudaGetLastError();
-}
-
-int launch_deinterleave(const DevProblem &P, double *lb, double *ub, int blocks, cudaStream_t s) {
-    k_deinterleave<<<blocks, 256, 0, s>>>(P, lb, ub);
-    return (int)cudaGetLastError();
-}
-
-int launch_mark_all(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (!P.use_marking || P.n_srows + P.n_lrows == 0) return 0;
-    k_mark_all<<<blocks, 256, 0, s>>>(P);
+int launch_finish(const DevProblem &P, double *lb, double *ub, int blocks, cudaStream_t s) {
+    k_finish<<<blocks, 256, 0, s>>>(P, lb, ub);
     return (int)cudaGetLastError();
 }
 
@@ -319,14 +339,8 @@ int launch_exact_phase(const DevProblem &P, int blocks, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int launch_finalize(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (P.n_chg_words == 0) return 0;
-    k_finalize<<<blocks, 256, 0, s>>>(P);
-    return (int)cudaGetLastError();
-}
-
-int launch_condition(const DevProblem &P, unsigned long long handle, cudaStream_t s) {
-    k_condition<<<1, 1, 0, s>>>(P, (cudaGraphConditionalHandle)handle);
+int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, cudaStream_t s) {
+    k_finalize<<<blocks, 256, 0, s>>>(P, (cudaGraphConditionalHandle)handle);
     return (int)cudaGetLastError();
 }
 
@@ -357,9 +371,9 @@ int phase_occupancy(int *act, int *cand, int *mega, int cta_warps) {
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(mega, mk, 32 * cta_warps, mega_smem);
 }
 
-int launch_megakernel(const DevProblem &P, int grid, int cta_warps, cudaStream_t s) {
+int launch_megakernel(const DevProblem &P, int first, int last, int *mail, int grid, int cta_warps, cudaStream_t s) {
     DevProblem Pc = P;
-    void *args[] = {&Pc};
+    void *args[] = {&Pc, &first, &last, &mail};
     return (int)cudaLaunchCooperativeKernel(megakernel_of(cta_warps), dim3(grid), dim3(32 * cta_warps), args,
                                             sizeof(WarpSmem) * (size_t)cta_warps, s);
 }

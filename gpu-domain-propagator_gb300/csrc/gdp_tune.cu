@@ -116,7 +116,7 @@ GDP_RETCODE autotune(int m, int n, int nnz, const int *col, const int *row_ptr, 
             std::copy(lbs, lbs + n, lb.begin());
             std::copy(ubs, ubs + n, ub.begin());
             gdp_stats st{};
-            if (ctx.propagate_host(lb.data(), ub.data(), &st) != GDP_OKAY) return GDP_ERROR;
+            if (ctx.propagate_host(lb.data(), ub.data(), lb.data(), ub.data(), &st) != GDP_OKAY) return GDP_ERROR;
             rounds = st.rounds;
             if (r > 0) t = std::min(t, st.device_ms);
         }
