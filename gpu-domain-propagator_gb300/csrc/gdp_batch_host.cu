@@ -61,6 +61,7 @@ GDP_RETCODE Batch::init_instances(int n_inst, const int *n_cons, const int *n_va
             set_error("instance " + std::to_string(k) + ": " + last_error());
             return GDP_ERROR;
         }
+        inst_[u]->release_host_resources();
     }
     n_units = n_inst;
     nodes = false;

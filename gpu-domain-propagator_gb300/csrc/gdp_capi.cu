@@ -87,6 +87,7 @@ const char *gdp_last_error(void) { return gdp::last_error(); }
 GDP_RETCODE gdp_release_cached_memory(void) {
     return guarded([&]() -> GDP_RETCODE {
         gdp::release_cached_memory();
+        gdp::release_kept_resources();
         return GDP_OKAY;
     });
 }

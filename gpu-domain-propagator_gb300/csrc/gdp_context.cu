@@ -148,6 +148,87 @@ void release_cached_memory() {
     c.bytes = 0;
 }
 
+
+// Streams, events and page-locked memory of destroyed contexts, kept for later
+// ones: creating and destroying them takes about 250 us, half the time of a
+// context of 100 rows. At most kKeptResources sets are kept (any thread takes
+// and gives them back); the object is never destroyed, as above.
+namespace {
+constexpr size_t kKeptResources = 16;
+struct ResourcePool {
+    std::mutex mu;
+    std::vector<HostResources *> free;
+};
+ResourcePool &resource_pool() {
+    static ResourcePool *p = new ResourcePool;
+    return *p;
+}
+void destroy_resources(HostResources *r) {
+    if (r->ev0) cudaEventDestroy(r->ev0);
+    if (r->ev1) cudaEventDestroy(r->ev1);
+    if (r->uploaded) cudaEventDestroy(r->uploaded);
+    if (r->pinned) cudaFreeHost(r->pinned);
+    if (r->stream) cudaStreamDestroy(r->stream);
+    if (r->upload) cudaStreamDestroy(r->upload);
+    delete r;
+}
+}  // namespace
+
+// The caller has set the device; null (and the error) on failure.
+HostResources *take_resources(int device, cudaError_t *err) {
+    ResourcePool &pool = resource_pool();
+    {
+        std::lock_guard<std::mutex> g(pool.mu);
+        for (size_t i = pool.free.size(); i-- > 0;)
+            if (pool.free[i]->device == device) {
+                HostResources *r = pool.free[i];
+                pool.free.erase(pool.free.begin() + (long)i);
+                return r;
+            }
+    }
+    HostResources *r = new HostResources;
+    r->device = device;
+    cudaError_t e = cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&r->upload, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreate(&r->ev0);
+    if (e == cudaSuccess) e = cudaEventCreate(&r->ev1);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->uploaded, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMallocHost(&r->pinned, HostResources::kFlagBytes + HostResources::kStageBytes);
+    if (e != cudaSuccess) {
+        destroy_resources(r);
+        *err = e;
+        return nullptr;
+    }
+    return r;
+}
+
+// Both streams are waited for: a later owner finds them empty.
+void give_resources(HostResources *r) {
+    if (!r) return;
+    const bool idle = cudaStreamSynchronize(r->stream) == cudaSuccess && cudaStreamSynchronize(r->upload) == cudaSuccess;
+    cudaGetLastError();
+    ResourcePool &pool = resource_pool();
+    {
+        std::lock_guard<std::mutex> g(pool.mu);
+        if (idle && pool.free.size() < kKeptResources) {
+            pool.free.push_back(r);
+            return;
+        }
+    }
+    destroy_resources(r);
+}
+
+void release_kept_resources() {
+    ResourcePool &pool = resource_pool();
+    std::vector<HostResources *> free;
+    {
+        std::lock_guard<std::mutex> g(pool.mu);
+        free.swap(pool.free);
+    }
+    for (HostResources *r : free) destroy_resources(r);
+    cudaGetLastError();
+}
+
 Arena::~Arena() { release(); }
 
 void Arena::release() {
@@ -211,6 +292,53 @@ void *Arena::alloc_bytes(size_t bytes) {
     return p;
 }
 
+bool Arena::carve(std::initializer_list<Piece> pieces) {
+    size_t total = 0;
+    for (const Piece &p : pieces) total += (std::max<size_t>(p.bytes, 1) + 255) & ~size_t(255);
+    unsigned char *d = (unsigned char *)alloc_bytes(total);
+    if (!d) return false;
+    for (const Piece &p : pieces) {
+        *p.dst = d;
+        d += (std::max<size_t>(p.bytes, 1) + 255) & ~size_t(255);
+    }
+    return true;
+}
+
+namespace {
+// Host arrays gathered and sent by send(): one device block and, with room in a
+// page-locked stage, one copy.
+struct Uploads {
+    struct Part {
+        const void *src;
+        size_t bytes, at;
+        void **dst;
+    };
+    std::vector<Part> parts;
+    size_t total = 0;
+    template <class T>
+    void add(T *&dst, const void *src, size_t bytes) {
+        parts.push_back(Part{src, bytes, total, (void **)&dst});
+        total += (std::max<size_t>(bytes, 1) + 255) & ~size_t(255);
+    }
+    // false: no memory, or a copy failed
+    bool send(Arena &arena, cudaStream_t s, unsigned char *stage, size_t stage_bytes) {
+        unsigned char *d = (unsigned char *)arena.alloc_bytes(total);
+        if (!d) return false;
+        const bool packed = stage && total <= stage_bytes;
+        for (const Part &p : parts) {
+            *p.dst = d + p.at;
+            if (!p.bytes) continue;
+            if (packed) std::memcpy(stage + p.at, p.src, p.bytes);
+            else if (cudaMemcpyAsync(d + p.at, p.src, p.bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) return false;
+        }
+        if (packed && cudaMemcpyAsync(d, stage, total, cudaMemcpyHostToDevice, s) != cudaSuccess) return false;
+        parts.clear();
+        total = 0;
+        return true;
+    }
+};
+}  // namespace
+
 // ---------------------------------------------------------------------------
 // The checks that make the raw arrays safe to copy: sizes, pointers and the
 // row pointer's end points.
@@ -225,15 +353,27 @@ static GDP_RETCODE validate_shape(int m, int n, int nnz, const int *col, const i
     return GDP_OKAY;
 }
 
+// Host threads for a loop over `items` rows or variables: one per 32K, so a
+// small problem starts none (waking 15 threads takes 10 to 50 us a loop, and
+// milliseconds when one of them is descheduled); one core is left to the
+// upload's helper thread.
+static int host_threads_for(long long items) {
+#ifdef _OPENMP
+    return (int)std::max(1LL, std::min<long long>(items >> 15, omp_get_max_threads() - 1));
+#else
+    return 1;
+#endif
+}
+
 GDP_RETCODE validate_csr(int m, int n, int nnz, const int *col, const int *row_ptr,
                          const double *val, const int *vartype) {
     if (validate_shape(m, n, nnz, col, row_ptr, val, vartype) != GDP_OKAY) return GDP_ERROR;
     int bad_row = INT_MAX, bad_var = INT_MAX;
-#pragma omp parallel for reduction(min : bad_row) schedule(static)
+#pragma omp parallel for reduction(min : bad_row) schedule(static) num_threads(host_threads_for(m))
     for (int i = 0; i < m; i++)
         if (row_ptr[i + 1] < row_ptr[i]) bad_row = std::min(bad_row, i);
     if (bad_row != INT_MAX) { set_error("csr_row_ptrs is not monotone"); return GDP_ERROR; }
-#pragma omp parallel for reduction(min : bad_var) schedule(static)
+#pragma omp parallel for reduction(min : bad_var) schedule(static) num_threads(host_threads_for(n))
     for (int j = 0; j < n; j++)
         if (vartype[j] != 0 && vartype[j] != 1 && vartype[j] != 3) bad_var = std::min(bad_var, j);
     if (bad_var != INT_MAX) {
@@ -286,10 +426,15 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
 
     GDP_CUDA(cudaSetDevice(opts.device));
     cudaGetLastError();  // every call below is checked; start from a clean error state
-    GDP_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    GDP_CUDA(cudaEventCreate(&ev0));
-    GDP_CUDA(cudaEventCreate(&ev1));
-    GDP_CUDA(cudaMallocHost(&h_flags, sizeof(RoundFlags) * 3));
+    {
+        cudaError_t e = cudaSuccess;
+        res = take_resources(opts.device, &e);
+        if (!res) GDP_CUDA(e);
+    }
+    stream = res->stream;
+    ev0 = res->ev0;
+    ev1 = res->ev1;
+    h_flags = reinterpret_cast<RoundFlags *>(res->pinned);
     int sms = 0;
     GDP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opts.device));
     n_sms = sms;
@@ -306,18 +451,21 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
     // waits for them on the device (an event), after the join. The element
     // checks (column range, finite coefficients) run on the device over the
     // copies.
+    // A small problem takes no helper: its arrays and the layout's are packed
+    // into the page-locked stage and go up in one copy.
     stamps.mark(1);
+    const size_t raw_bytes = sizeof(int) * (size_t)nnz + sizeof(double) * (size_t)nnz + sizeof(int) * ((size_t)m + 1) +
+                             2 * sizeof(double) * (size_t)m;
+    // the layout's arrays are at most about 100 bytes per row and tile, and a byte per variable
+    const bool small = raw_bytes + 128 * (size_t)m + 2 * (size_t)n + 16384 <= HostResources::kStageBytes;
     Arena raw;  // raw CSR and row sides, released when the build is done
     int *dcol = nullptr, *drp = nullptr;
     double *dval = nullptr, *dlhs = nullptr, *drhs = nullptr;
     std::string up_err;
-    struct UploadStream {  // the helper's stream and its completion event
+    struct UploadStream {  // the helper's stream
         cudaStream_t s = nullptr;
-        cudaEvent_t done = nullptr;
         ~UploadStream() {
             if (s) cudaStreamSynchronize(s);  // before the raw buffers can be freed
-            if (done) cudaEventDestroy(done);
-            if (s) cudaStreamDestroy(s);
         }
     } ups;
     // marking index (variable -> row positions, |a| rounded up): the helper
@@ -337,49 +485,42 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
             if (t.joinable()) t.join();
         }
     } uploader;  // declared after everything the thread touches: joined first
-    uploader.t = std::thread([&, dev = opts.device] {
-        auto fail = [&](const char *what, cudaError_t e) {
-            up_err = std::string(what) + ": " + cudaGetErrorString(e);
-            cudaGetLastError();
-        };
-        cudaError_t e = cudaSetDevice(dev);
-        if (e != cudaSuccess) return fail("cudaSetDevice", e);
-        const size_t nz = (size_t)std::max(nnz, 1);
-        dcol = (int *)raw.alloc_bytes(sizeof(int) * nz);
-        dval = (double *)raw.alloc_bytes(sizeof(double) * nz);
-        drp = (int *)raw.alloc_bytes(sizeof(int) * ((size_t)m + 1));
-        dlhs = (double *)raw.alloc_bytes(sizeof(double) * (size_t)std::max(m, 1));
-        drhs = (double *)raw.alloc_bytes(sizeof(double) * (size_t)std::max(m, 1));
-        if (!dcol || !dval || !drp || !dlhs || !drhs) {
-            up_err = "device allocation failed (raw CSR)";
-            return;
-        }
-        e = cudaStreamCreateWithFlags(&ups.s, cudaStreamNonBlocking);
-        if (e != cudaSuccess) return fail("cudaStreamCreate", e);
-        e = cudaEventCreateWithFlags(&ups.done, cudaEventDisableTiming);
-        if (e != cudaSuccess) return fail("cudaEventCreate", e);
-        cudaStream_t us = ups.s;
-        stamps.record(0, us);
-        if (nnz) e = cudaMemcpyAsync(dcol, col, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, us);
-        if (e == cudaSuccess && nnz)
-            e = cudaMemcpyAsync(dval, val, sizeof(double) * (size_t)nnz, cudaMemcpyHostToDevice, us);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(drp, row_ptr, sizeof(int) * ((size_t)m + 1), cudaMemcpyHostToDevice, us);
-        if (e == cudaSuccess && m) e = cudaMemcpyAsync(dlhs, lhs, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, us);
-        if (e == cudaSuccess && m) e = cudaMemcpyAsync(drhs, rhs, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, us);
-        stamps.record(1, us);
-        if (e == cudaSuccess) e = (cudaError_t)build_marking_counts(dcol, nnz, n, vp, vcur, vscan, us);
-        if (e == cudaSuccess) e = cudaEventRecord(ups.done, us);
-        if (e != cudaSuccess) fail("raw CSR upload", e);
-    });
+    if (!small) {
+        ups.s = res->upload;
+        uploader.t = std::thread([&, dev = opts.device] {
+            auto fail = [&](const char *what, cudaError_t e) {
+                up_err = std::string(what) + ": " + cudaGetErrorString(e);
+                cudaGetLastError();
+            };
+            cudaError_t e = cudaSetDevice(dev);
+            if (e != cudaSuccess) return fail("cudaSetDevice", e);
+            const size_t nz = (size_t)std::max(nnz, 1);
+            dcol = (int *)raw.alloc_bytes(sizeof(int) * nz);
+            dval = (double *)raw.alloc_bytes(sizeof(double) * nz);
+            drp = (int *)raw.alloc_bytes(sizeof(int) * ((size_t)m + 1));
+            dlhs = (double *)raw.alloc_bytes(sizeof(double) * (size_t)std::max(m, 1));
+            drhs = (double *)raw.alloc_bytes(sizeof(double) * (size_t)std::max(m, 1));
+            if (!dcol || !dval || !drp || !dlhs || !drhs) {
+                up_err = "device allocation failed (raw CSR)";
+                return;
+            }
+            cudaStream_t us = ups.s;
+            stamps.record(0, us);
+            if (nnz) e = cudaMemcpyAsync(dcol, col, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, us);
+            if (e == cudaSuccess && nnz)
+                e = cudaMemcpyAsync(dval, val, sizeof(double) * (size_t)nnz, cudaMemcpyHostToDevice, us);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(drp, row_ptr, sizeof(int) * ((size_t)m + 1), cudaMemcpyHostToDevice, us);
+            if (e == cudaSuccess && m) e = cudaMemcpyAsync(dlhs, lhs, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, us);
+            if (e == cudaSuccess && m) e = cudaMemcpyAsync(drhs, rhs, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice, us);
+            stamps.record(1, us);
+            if (e == cudaSuccess) e = (cudaError_t)build_marking_counts(dcol, nnz, n, vp, vcur, vscan, us);
+            if (e == cudaSuccess) e = cudaEventRecord(res->uploaded, us);
+            if (e != cudaSuccess) fail("raw CSR upload", e);
+        });
+    }
 
-    // host threads while the helper runs: one core stays free for it, so
-    // that no parallel region waits for a descheduled thread
-#ifdef _OPENMP
-    const int host_threads = std::max(1, omp_get_max_threads() - 1);
-#else
-    const int host_threads = 1;
-#endif
+    const int host_threads = host_threads_for(m);
     // ---- row binning (SELL-g) ----
     // g = 1 for rows up to thread_row_max; g = smallest power of two >= len/32
     // (2..32) up to split_tile; longer rows are split into warp tiles.
@@ -585,32 +726,24 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         }
     }
     // ---- upload ----
-    auto up = [&](const void *src, size_t bytes) -> void * {
-        void *d = arena.alloc_bytes(bytes);
-        if (!d) return nullptr;
-        if (bytes && cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, stream) != cudaSuccess)
-            return nullptr;
-        return d;
-    };
-#define GDP_UP(dst, T, vec)                                                                         \
-    do {                                                                                           \
-        dst = (T *)up((vec).data(), sizeof((vec)[0]) * (vec).size());                              \
-        if (!dst) { set_error("device allocation/upload failed for " #vec); return GDP_ERROR; }     \
-    } while (0)
+    Uploads ups1, ups2;  // what the layout build reads; the rest
+    unsigned char *stage = small ? (unsigned char *)res->pinned + HostResources::kFlagBytes : nullptr;
+#define GDP_UP(dst, vec) ups1.add(dst, (vec).data(), sizeof((vec)[0]) * (vec).size())
     std::memset(&P, 0, sizeof(P));
     P.n = n;
     P.n_srows = n_srows;
     P.n_slices = n_slices;
-    GDP_UP(P.slice_ptr, const long long, slice_ptr);
-    GDP_UP(P.slice_row0, const int, slice_row0);
-    GDP_UP(P.slice_lg, const int, slice_lg);
+    GDP_UP(P.slice_ptr, slice_ptr);
+    GDP_UP(P.slice_row0, slice_row0);
+    GDP_UP(P.slice_lg, slice_lg);
     stamps.mark(2);
-    int *d_srow_len = (int *)arena.alloc_bytes(sizeof(int) * (size_t)std::max(ns, 1));
-    int *d_xptr = (int *)arena.alloc_bytes(sizeof(int) * (size_t)std::max(ns, 1));
-    int *d_pos_slice = (int *)arena.alloc_bytes(sizeof(int) * (size_t)std::max(ns, 1));
-    double *d_srow_lhs = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(ns, 1));
-    double *d_srow_rhs = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(ns, 1));
-    if (!d_srow_len || !d_xptr || !d_pos_slice || !d_srow_lhs || !d_srow_rhs) {
+    int *d_srow_len, *d_xptr, *d_pos_slice;
+    double *d_srow_lhs, *d_srow_rhs;
+    if (!arena.carve({{(void **)&d_srow_len, sizeof(int) * (size_t)ns},
+                      {(void **)&d_xptr, sizeof(int) * (size_t)ns},
+                      {(void **)&d_pos_slice, sizeof(int) * (size_t)ns},
+                      {(void **)&d_srow_lhs, sizeof(double) * (size_t)ns},
+                      {(void **)&d_srow_rhs, sizeof(double) * (size_t)ns}})) {
         set_error("device allocation failed (row positions)");
         return GDP_ERROR;
     }
@@ -621,13 +754,13 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
     P.srow_rhs = d_srow_rhs;
     P.n_lrows = n_lrows;
     P.n_tiles = n_tiles;
-    GDP_UP(P.lrow_lhs, const double, lrow_lhs);
-    GDP_UP(P.lrow_rhs, const double, lrow_rhs);
-    GDP_UP(P.lrow_tile0, const int, lrow_tile0);
+    GDP_UP(P.lrow_lhs, lrow_lhs);
+    GDP_UP(P.lrow_rhs, lrow_rhs);
+    GDP_UP(P.lrow_tile0, lrow_tile0);
     if (tile_row.empty()) { tile_row.push_back(0); tile_begin.push_back(0); tile_end.push_back(0); }
-    GDP_UP(P.tile_row, const int, tile_row);
-    GDP_UP(P.tile_begin, const int, tile_begin);
-    GDP_UP(P.tile_end, const int, tile_end);
+    GDP_UP(P.tile_row, tile_row);
+    GDP_UP(P.tile_begin, tile_begin);
+    GDP_UP(P.tile_end, tile_end);
     // The device builds the layout and then the marking index while this
     // thread prepares the rest (row origins, work lists, variable types) and
     // sends it up on the helper's stream; one synchronisation at the end, then
@@ -640,61 +773,69 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         const size_t n_sell = (size_t)std::max<long long>(sell_elems, 1);
         const size_t n_x = (size_t)std::max<long long>(x_elems, 1);
         const size_t n_l = (size_t)std::max<long long>(lnnz, 1);
-        int *sc = (int *)arena.alloc_bytes(sizeof(int) * n_sell);
-        double *sv = (double *)arena.alloc_bytes(sizeof(double) * n_sell);
-        int *xc = (int *)arena.alloc_bytes(sizeof(int) * n_x);
-        double *xv = (double *)arena.alloc_bytes(sizeof(double) * n_x);
-        int *lc = (int *)arena.alloc_bytes(sizeof(int) * n_l);
-        double *lv = (double *)arena.alloc_bytes(sizeof(double) * n_l);
-        float *sa = (float *)arena.alloc_bytes(sizeof(float) * n_sell);
-        float *xa = (float *)arena.alloc_bytes(sizeof(float) * n_x);
-        float *la = (float *)arena.alloc_bytes(sizeof(float) * n_l);
-        if (!sc || !sv || !xc || !xv || !lc || !lv || !sa || !xa || !la) {
+        int *sc, *xc, *lc;
+        double *xv, *lv;
+        float *sa, *la;
+        // the arrays with padding slots first: cleared together
+        size_t cleared = 0;
+        if (!arena.carve({{(void **)&sc, sizeof(int) * n_sell},
+                          {(void **)&sa, sizeof(float) * n_sell},
+                          {(void **)&xc, sizeof(int) * n_x},
+                          {(void **)&xv, sizeof(double) * n_x},
+                          {(void **)&lc, sizeof(int) * n_l},
+                          {(void **)&lv, sizeof(double) * n_l},
+                          {(void **)&la, sizeof(float) * n_l}})) {
             set_error("device allocation failed (layout element arrays)");
             return GDP_ERROR;
         }
-        GDP_CUDA(cudaMemsetAsync(sc, 0, sizeof(int) * n_sell, stream));  // padding slots
-        GDP_CUDA(cudaMemsetAsync(sv, 0, sizeof(double) * n_sell, stream));
-        GDP_CUDA(cudaMemsetAsync(sa, 0, sizeof(float) * n_sell, stream));
-        GDP_CUDA(cudaMemsetAsync(xc, 0, sizeof(int) * n_x, stream));  // row padding of the copy
-        GDP_CUDA(cudaMemsetAsync(xv, 0, sizeof(double) * n_x, stream));
-        GDP_CUDA(cudaMemsetAsync(xa, 0, sizeof(float) * n_x, stream));
-        int *dord = (int *)tmp.alloc_bytes(sizeof(int) * (size_t)std::max(ns, 1));
-        int *dspl = (int *)tmp.alloc_bytes(sizeof(int) * (size_t)std::max(n_lrows, 1));
-        long long *dlrp = (long long *)tmp.alloc_bytes(sizeof(long long) * ((size_t)n_lrows + 1));
-        int *dls = (int *)tmp.alloc_bytes(sizeof(int) * len_start.size());
-        long long *dlb = (long long *)tmp.alloc_bytes(sizeof(long long) * len_base.size());
-        int *dbad = (int *)tmp.alloc_bytes(sizeof(int) * 2);
-        if (!dord || !dspl || !dlrp || !dls || !dlb || !dbad) {
-            set_error("device allocation failed (row maps)");
-            return GDP_ERROR;
-        }
-        uploader.t.join();
-        stamps.mark(3);
-        if (!up_err.empty()) {
-            set_error(up_err);
-            return GDP_ERROR;
-        }
-        GDP_CUDA(cudaStreamWaitEvent(stream, ups.done, 0));
-        stamps.record(2, stream);
-        if (ns) GDP_CUDA(cudaMemcpyAsync(dord, order, sizeof(int) * (size_t)ns, cudaMemcpyHostToDevice, stream));
-        if (n_lrows)
-            GDP_CUDA(cudaMemcpyAsync(dspl, split_rows.data(), sizeof(int) * (size_t)n_lrows, cudaMemcpyHostToDevice,
-                                     stream));
-        GDP_CUDA(cudaMemcpyAsync(dlrp, lrow_ptr.data(), sizeof(long long) * ((size_t)n_lrows + 1),
-                                 cudaMemcpyHostToDevice, stream));
-        GDP_CUDA(cudaMemcpyAsync(dls, len_start.data(), sizeof(int) * len_start.size(), cudaMemcpyHostToDevice,
-                                 stream));
-        GDP_CUDA(cudaMemcpyAsync(dlb, len_base.data(), sizeof(long long) * len_base.size(), cudaMemcpyHostToDevice,
-                                 stream));
+        cleared = (size_t)((unsigned char *)(xv + n_x) - (unsigned char *)sc);
+        GDP_CUDA(cudaMemsetAsync(sc, 0, cleared, stream));
+        int *dord, *dspl, *dls, *dbad;
+        long long *dlrp, *dlb;
         const int no_bad[2] = {INT_MAX, INT_MAX};
-        GDP_CUDA(cudaMemcpyAsync(dbad, no_bad, sizeof(no_bad), cudaMemcpyHostToDevice, stream));
+        Uploads maps;
+        Uploads &um = small ? ups1 : maps;  // a small problem's row maps stay with its other arrays
+        um.add(dord, order, sizeof(int) * (size_t)ns);
+        um.add(dspl, split_rows.data(), sizeof(int) * (size_t)n_lrows);
+        um.add(dlrp, lrow_ptr.data(), sizeof(long long) * ((size_t)n_lrows + 1));
+        um.add(dls, len_start.data(), sizeof(int) * len_start.size());
+        um.add(dlb, len_base.data(), sizeof(long long) * len_base.size());
+        um.add(dbad, no_bad, sizeof(no_bad));
+        if (small) {
+            ups1.add(dcol, col, sizeof(int) * (size_t)nnz);
+            ups1.add(dval, val, sizeof(double) * (size_t)nnz);
+            ups1.add(drp, row_ptr, sizeof(int) * ((size_t)m + 1));
+            ups1.add(dlhs, lhs, sizeof(double) * (size_t)m);
+            ups1.add(drhs, rhs, sizeof(double) * (size_t)m);
+        }
+        const size_t sent = ups1.total;
+        if (!ups1.send(arena, stream, stage, HostResources::kStageBytes)) {
+            set_error("device allocation or upload failed (layout)");
+            return GDP_ERROR;
+        }
+        if (stage) stage += std::min(sent, HostResources::kStageBytes);
+        if (small) {
+            GDP_CUDA(build_marking_counts(dcol, nnz, n, vp, vcur, vscan, stream));
+        } else {
+            uploader.t.join();
+            stamps.mark(3);
+            if (!up_err.empty()) {
+                set_error(up_err);
+                return GDP_ERROR;
+            }
+            GDP_CUDA(cudaStreamWaitEvent(stream, res->uploaded, 0));
+            stamps.record(2, stream);
+            if (!maps.send(tmp, stream, nullptr, 0)) {
+                set_error("device allocation or upload failed (row maps)");
+                return GDP_ERROR;
+            }
+        }
         GDP_CUDA(check_csr_elements(dcol, dval, nnz, n, dbad, 8 * n_sms, stream));
         LayoutBuild L;
         L.col = dcol; L.row_ptr = drp; L.val = dval;
         L.n_srows = ns; L.order = dord; L.pos_slice = P.pos_slice; L.slice_row0 = P.slice_row0;
         L.slice_lg = P.slice_lg; L.xptr = P.xptr; L.slice_ptr = P.slice_ptr;
-        L.sell_col = sc; L.xcol = xc; L.sell_val = sv; L.xval = xv; L.sell_a32 = sa; L.xa32 = xa;
+        L.sell_col = sc; L.xcol = xc; L.xval = xv; L.sell_a32 = sa;
         L.g1_begin = g1_begin; L.la32 = la;
         L.n_lrows = n_lrows; L.split_rows = dspl; L.lrow_ptr = dlrp; L.lcol = lc; L.lval = lv;
         L.lhs = dlhs; L.rhs = drhs; L.len_start = dls; L.len_base = dlb; L.n_slices = n_slices;
@@ -709,8 +850,8 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         stamps.record(3, stream);
         stamps.mark(4);
         GDP_CUDA(cudaMemcpyAsync(hbad, dbad, sizeof(int) * 2, cudaMemcpyDeviceToHost, stream));
-        P.sell_col = sc; P.sell_val = sv; P.sell_a32 = sa;
-        P.xcol = xc; P.xval = xv; P.xa32 = xa;
+        P.sell_col = sc; P.sell_a32 = sa;
+        P.xcol = xc; P.xval = xv;
         P.lcol = lc; P.lval = lv; P.la32 = la;
     }
     vec_blocks = std::max(1, std::min((std::max(n, std::max(ns + n_lrows, 1)) + 255) / 256, 8 * n_sms));
@@ -718,82 +859,74 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
     // never mark) was filled with the layout
     P.var_ptr = vp;
     P.var_ent = vent;
-    // the rest goes up on the helper's stream while the device builds
-    auto up_aux = [&](const void *src, size_t bytes) -> void * {
-        void *d = arena.alloc_bytes(bytes);
-        if (!d) return nullptr;
-        if (bytes && cudaMemcpyAsync(d, src, bytes, cudaMemcpyHostToDevice, ups.s) != cudaSuccess) return nullptr;
-        return d;
-    };
-#define GDP_UP_AUX(dst, T, vec)                                                                     \
-    do {                                                                                           \
-        dst = (T *)up_aux((vec).data(), sizeof((vec)[0]) * (vec).size());                          \
-        if (!dst) { set_error("device allocation/upload failed for " #vec); return GDP_ERROR; }     \
-    } while (0)
     // row-side infeasibility names a position's original row: the split rows
     // follow the SELL positions (the row order uploaded above is staged already)
     std::copy(split_rows.begin(), split_rows.end(), pos_row.begin() + ns);
     if (ns + n_lrows == 0) pos_row[0] = 0;
-    P.pos_row = (const int *)up_aux(pos_row.data(), sizeof(int) * (size_t)std::max(ns + n_lrows, 1));
-    if (!P.pos_row) { set_error("device allocation/upload failed for pos_row"); return GDP_ERROR; }
+    ups2.add(P.pos_row, pos_row.data(), sizeof(int) * (size_t)std::max(ns + n_lrows, 1));
     std::vector<int> mtiles;
     for (int r = 0; r < n_lrows; r++)
         if (lrow_tile0[r + 1] - lrow_tile0[r] > 1)
             for (int t = lrow_tile0[r]; t < lrow_tile0[r + 1]; t++) mtiles.push_back(t);
     P.n_mtiles = (int)mtiles.size();
     if (mtiles.empty()) mtiles.push_back(0);
-    GDP_UP_AUX(P.mtiles, const int, mtiles);
+    ups2.add(P.mtiles, mtiles.data(), sizeof(int) * mtiles.size());
     P.n_items = (int)items.size();
     if (items.empty()) items.push_back(0);
-    GDP_UP_AUX(P.items, const int, items);
+    ups2.add(P.items, items.data(), sizeof(int) * items.size());
     P.use_marking = opts.use_marking < 0 ? 1 : (opts.use_marking > 2 ? 2 : opts.use_marking);
     // adaptive marking: mark when a round tightened fewer bounds than 1/16 of the variables
     P.mark_threshold = (unsigned)std::max(1, n / 16);
     RawVec<unsigned char> is_cont((size_t)std::max(n, 1));
     is_cont[0] = 0;
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) num_threads(host_threads_for(n))
     for (int j = 0; j < n; j++) is_cont[j] = vartype[j] == GDP_CONTINUOUS ? 1 : 0;
-    GDP_UP_AUX(P.is_cont, const unsigned char, is_cont);
-#undef GDP_UP_AUX
+    ups2.add(P.is_cont, is_cont.data(), is_cont.size());
 #undef GDP_UP
+    // the rest goes up on the helper's stream while the device builds
+    if (!ups2.send(arena, small ? stream : ups.s, stage,
+                   stage ? (size_t)((unsigned char *)res->pinned + HostResources::kFlagBytes +
+                                    HostResources::kStageBytes - stage)
+                         : 0)) {
+        set_error("device allocation or upload failed (work lists)");
+        return GDP_ERROR;
+    }
     const int npos = std::max(ns + n_lrows, 1);
     const int n_words = (n + 31) / 32;
-    P.tile_part = (TilePart *)arena.alloc_bytes(sizeof(TilePart) * (size_t)std::max(n_tiles, 1));
-    P.tile_scr = (TileScr *)arena.alloc_bytes(sizeof(TileScr) * (size_t)std::max(n_tiles, 1));
     // deferred exact pass: per-class row queues (classes are contiguous position ranges)
     for (int c = 0; c < 6; c++) { P.cls_begin[c] = 0; P.cls_end[c] = 0; }
     for (int sl = n_slices - 1; sl >= 0; sl--) P.cls_begin[slice_lg[sl]] = slice_row0[sl];
     for (int sl = 0; sl < n_slices; sl++) P.cls_end[slice_lg[sl]] = slice_row0[sl + 1];
-    P.xrow = (XRow *)arena.alloc_bytes(sizeof(XRow) * (size_t)std::max(ns, 1));
-    P.xctr = (unsigned *)arena.alloc_bytes(sizeof(unsigned) * 32);
-    P.row_exact = (int *)arena.alloc_bytes(sizeof(int) * (size_t)std::max(n_lrows, 1));
-    P.lrow_margin = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(n_lrows, 1));
-    P.lrow_drift = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(n_lrows, 1));
-    P.lrow_skip = (int *)arena.alloc_bytes(sizeof(int) * (size_t)std::max(n_lrows, 1));
-    P.mark = (int *)arena.alloc_bytes(sizeof(int) * (size_t)npos);
-    P.bnd = (double2 *)arena.alloc_bytes(sizeof(double2) * (size_t)std::max(n, 1));
-    P.bnd_nxt = (double2 *)arena.alloc_bytes(sizeof(double2) * (size_t)std::max(n, 1));
-    P.bnd32 = (float2 *)arena.alloc_bytes(sizeof(BndScr) * (size_t)std::max(n, 1));  // stamped records
-    P.chg = (unsigned *)arena.alloc_bytes(sizeof(unsigned) * (size_t)std::max(n_words, 1));
     P.n_chg_words = n_words;
-    P.flags = (RoundFlags *)arena.alloc_bytes(sizeof(RoundFlags) * 3);
-    P.barrier = (unsigned *)arena.alloc_bytes(sizeof(unsigned) * 2);
-    P.queue = (unsigned *)arena.alloc_bytes(sizeof(unsigned) * 8);
     P.max_rounds = opts.max_rounds;
     P.spin_limit = opts.barrier_wait_kcycles > 0 ? 1000LL * opts.barrier_wait_kcycles : 4000000000LL;
-    if (!host_direct) {
-        d_lb = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(n, 1));
-        d_ub = (double *)arena.alloc_bytes(sizeof(double) * (size_t)std::max(n, 1));
-    }
-    if (!P.tile_part || !P.tile_scr || !P.row_exact || !P.lrow_margin || !P.lrow_drift || !P.lrow_skip || !P.xrow || !P.xctr || !P.mark || !P.bnd || !P.bnd_nxt || !P.bnd32 || !P.chg || !P.flags || !P.barrier || !P.queue ||
-        (!host_direct && (!d_lb || !d_ub))) {
+    const size_t nl = (size_t)n_lrows, nt = (size_t)n_tiles, nv = (size_t)n;
+    const size_t staged = host_direct ? 0 : sizeof(double) * nv;
+    if (!arena.carve({{(void **)&P.tile_part, sizeof(TilePart) * nt},
+                      {(void **)&P.tile_scr, sizeof(TileScr) * nt},
+                      {(void **)&P.xrow, sizeof(XRow) * (size_t)ns},
+                      {(void **)&P.xctr, sizeof(unsigned) * 32},
+                      {(void **)&P.row_exact, sizeof(int) * nl},
+                      {(void **)&P.lrow_margin, sizeof(double) * nl},
+                      {(void **)&P.lrow_drift, sizeof(double) * nl},
+                      {(void **)&P.lrow_skip, sizeof(int) * nl},
+                      {(void **)&P.mark, sizeof(int) * (size_t)npos},
+                      {(void **)&P.bnd, sizeof(double2) * nv},
+                      {(void **)&P.bnd_nxt, sizeof(double2) * nv},
+                      {(void **)&P.bnd32, sizeof(BndScr) * nv},  // stamped records
+                      {(void **)&P.chg, sizeof(unsigned) * (size_t)n_words},
+                      {(void **)&P.flags, sizeof(RoundFlags) * 3},
+                      {(void **)&P.barrier, sizeof(unsigned) * 2},
+                      {(void **)&P.queue, sizeof(unsigned) * 8},
+                      {(void **)&d_lb, staged},
+                      {(void **)&d_ub, staged}})) {
         set_error("device allocation failed");
         return GDP_ERROR;
     }
 
     if (set_schedule(opts.sync_type, opts.ctas_per_sm, opts.cta_threads) != GDP_OKAY) return GDP_ERROR;
     stamps.mark(5);
-    GDP_CUDA(cudaStreamSynchronize(ups.s));
+    if (ups.s) GDP_CUDA(cudaStreamSynchronize(ups.s));
     GDP_CUDA(cudaStreamSynchronize(stream));  // before the raw CSR is freed and the verdict is read
     stamps.mark(6);
     stamps.report();
@@ -822,8 +955,7 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     }
     // no more CTAs than a phase has work for a warp each: screen items, exact
     // items (a slice's rows make up to two), quarters of exact tiles, words of
-    // the change bitmap. Every barrier waits for every CTA, and a launch costs
-    // less with fewer: 100 rows take 0.36 ms on 1 CTA, 0.45 on 456.
+    // the change bitmap. A grid barrier takes 1.6 us with 456 CTAs, 0.7 with 8.
     const long long cand_work = std::max(2LL * P.n_items, 4LL * P.n_mtiles);
     auto ctas_for = [](long long work, int w, int most) {
         return (int)std::max(1LL, std::min<long long>(most, (work + w - 1) / w));
@@ -844,14 +976,19 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     return GDP_OKAY;
 }
 
+void Context::release_host_resources() {
+    give_resources(res);
+    res = nullptr;
+    stream = nullptr;
+    ev0 = ev1 = nullptr;
+    h_flags = nullptr;
+}
+
 Context::~Context() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph) cudaGraphDestroy(graph);
-    if (ev0) cudaEventDestroy(ev0);
-    if (ev1) cudaEventDestroy(ev1);
-    if (h_flags) cudaFreeHost(h_flags);
-    if (stream) cudaStreamDestroy(stream);
+    give_resources(res);
 }
 
 // ---- drivers ---------------------------------------------------------------

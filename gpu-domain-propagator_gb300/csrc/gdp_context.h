@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -26,10 +27,32 @@ struct Arena {
         int dev;
     };
     std::vector<Block> blocks;
+    struct Piece {
+        void **dst;
+        size_t bytes;
+    };
     ~Arena();
     void *alloc_bytes(size_t bytes);
+    bool carve(std::initializer_list<Piece> pieces);  // one block for all pieces, 256-byte aligned
     void release();  // waits for the device, then returns every block to the cache
 };
+
+// What a context needs besides device memory: two streams (its own, and one
+// for uploads during the build), events, and page-locked memory for the round
+// flags and a stage for small uploads. Taken from and given back to a bounded
+// process-wide pool.
+struct HostResources {
+    static constexpr size_t kFlagBytes = 4096;
+    static constexpr size_t kStageBytes = 1 << 20;
+    int device = 0;
+    cudaStream_t stream = nullptr, upload = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, uploaded = nullptr;
+    void *pinned = nullptr;
+};
+static_assert(3 * sizeof(RoundFlags) <= HostResources::kFlagBytes, "the flags fit their part");
+HostResources *take_resources(int device, cudaError_t *err);
+void give_resources(HostResources *r);
+void release_kept_resources();  // destroys the sets that the pool keeps
 
 // Frees the cached device memory of released arenas (all devices).
 void release_cached_memory();
@@ -56,6 +79,9 @@ public:
     // Loop driver, resident CTAs per SM (0: as many as fit) and megakernel CTA
     // size of later propagations; the layout stays.
     GDP_RETCODE set_schedule(int sync_type, int ctas_per_sm, int cta_threads);
+    // Gives the streams, events and page-locked memory back: a batch member's
+    // context is only a layout once it is built.
+    void release_host_resources();
     // Learned marking with model m (NULL: off), logit threshold and the
     // shortest row length the model decides for.
     GDP_RETCODE set_model(const Mlp *m, float threshold, int min_len);
@@ -65,7 +91,8 @@ public:
 
     int m = 0, n = 0, nnz = 0;
     gdp_options opts{};
-    cudaStream_t stream = nullptr;
+    HostResources *res = nullptr;
+    cudaStream_t stream = nullptr;  // this and the next three: res's
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     RoundFlags *h_flags = nullptr;  // pinned
     Arena arena;

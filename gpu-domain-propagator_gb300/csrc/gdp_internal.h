@@ -123,15 +123,13 @@ struct DevProblem {
     const int *slice_row0;       // n_slices + 1: first row position of each slice
     const int *slice_lg;         // n_slices: log2 of the lanes per row (SELL-g)
     const int *sell_col;
-    const double *sell_val;
-    const float *sell_a32;       // FP32 screen copies of sell_val (coef_screen)
+    const float *sell_a32;       // FP32 screen copies of the coefficients (coef_screen)
     const int *srow_len;         // n_srows
     // row-contiguous copy of the SELL rows for the deferred exact pass: the
     // elements of position p at xptr[p] .. xptr[p] + srow_len[p] - 1
     const int *xptr;             // n_srows
     const int *xcol;
     const double *xval;
-    const float *xa32;           // screen copies of xval
     const double *srow_lhs, *srow_rhs;
     // original row index of each position (SELL positions, then split rows)
     const int *pos_row;
@@ -245,8 +243,8 @@ struct LayoutBuild {
     const int *pos_slice, *slice_row0, *slice_lg, *xptr;
     const long long *slice_ptr;
     int *sell_col, *xcol;
-    double *sell_val, *xval;
-    float *sell_a32, *xa32;  // FP32 screen copies (coef_screen)
+    double *xval;
+    float *sell_a32;         // FP32 screen copies (coef_screen)
     int g1_begin;            // first position of the one-lane rows (n_srows: none)
     int n_lrows;
     const int *split_rows;     // split-row slot -> row

@@ -128,11 +128,9 @@ __global__ void __launch_bounds__(256) k_build_sell(LayoutBuild L) {
             const float a = coef_screen(v);
             const long long e = base + 32LL * k;
             L.sell_col[e] = c;
-            L.sell_val[e] = v;
             L.sell_a32[e] = a;
             L.xcol[xb + k] = c;
             L.xval[xb + k] = v;
-            L.xa32[xb + k] = a;
             index_element(L, c, v, p);
         }
     }
@@ -152,11 +150,9 @@ __global__ void __launch_bounds__(256) k_build_sell(LayoutBuild L) {
             const float a = coef_screen(v);
             const long long e = base + 32LL * (k >> lg) + (k & (g - 1));
             L.sell_col[e] = c;
-            L.sell_val[e] = v;
             L.sell_a32[e] = a;
             L.xcol[xb + k] = c;
             L.xval[xb + k] = v;
-            L.xa32[xb + k] = a;
             index_element(L, c, v, p);
         }
     }
