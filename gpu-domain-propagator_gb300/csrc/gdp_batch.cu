@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
                         push_tile(B.cq, B.tail + 2, B.cap_tiles, B.error, u, -it - 1);
                     }
                 } else if (it >= 0) {
-                    sell_slice<0>(Pu, it, lane, r, marked, change, tight, mine);
+                    sell_slice<0, false>(Pu, it, lane, r, marked, change, tight, mine);
                 } else if (split_partial<0>(Pu, -it - 1, lane, r, marked, change, tight, mine) && lane == 0) {
                     push_tile(B.cq, B.tail + 2, B.cap_tiles, B.error, u, -it - 1);
                 }

@@ -414,8 +414,7 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         set_error("Unknown sync type");
         return GDP_ERROR;
     }
-    if (opts.cta_threads == 0) opts.cta_threads = 256;
-    if (opts.cta_threads != 128 && opts.cta_threads != 256 && opts.cta_threads != 512) {
+    if (opts.cta_threads != 0 && opts.cta_threads != 128 && opts.cta_threads != 256 && opts.cta_threads != 512) {
         set_error("cta_threads must be 128, 256 or 512");
         return GDP_ERROR;
     }
@@ -935,19 +934,30 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
 }
 
 // Grid sizes of the loop drivers for the schedule (the layout is untouched).
+// cta_threads 0: the default, 256, or one CTA of 512 threads for up to
+// kOneCtaSlices slices of one-lane rows: its barrier is __syncthreads and its
+// L1 stays valid from round to round (400 rows: 0.38 ms against 0.57 on 4 CTAs
+// of 256 threads; 800 rows, 25 slices: 0.61 against 0.60).
+constexpr int kOneCtaSlices = 16;
 GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_threads) {
     if (sync_type < CPU_LOOP || sync_type > MEGAKERNEL) {
         set_error("Unknown sync type");
         return GDP_ERROR;
     }
-    if (cta_threads != 128 && cta_threads != 256 && cta_threads != 512) {
+    if (cta_threads != 0 && cta_threads != 128 && cta_threads != 256 && cta_threads != 512) {
         set_error("cta_threads must be 128, 256 or 512");
         return GDP_ERROR;
     }
     GDP_CUDA(cudaSetDevice(opts.device));
+    const bool one_lane = n_lrows == 0 && P.cls_end[0] == n_srows && P.cls_begin[0] == 0;
+    const bool one_cta = cta_threads == 0 && one_lane && P.n_items <= kOneCtaSlices;
+    if (cta_threads == 0) cta_threads = one_cta ? 512 : 256;
     const int warps = cta_threads / 32;
     int act_bps = 0, cand_bps = 0, mega_bps = 0;
-    GDP_CUDA(phase_occupancy(&act_bps, &cand_bps, &mega_bps, warps));
+    // one-lane rows alone, and a warp for each slice (24 warps per SM, fewer
+    // with a limit): the exact pass in place
+    P.in_place = one_lane && P.n_items <= n_sms * (ctas_per_sm > 0 ? std::min(24, ctas_per_sm * warps) : 24);
+    GDP_CUDA(phase_occupancy(&act_bps, &cand_bps, &mega_bps, warps, P.in_place != 0));
     if (ctas_per_sm > 0) {
         act_bps = std::min(act_bps, ctas_per_sm);
         cand_bps = std::min(cand_bps, ctas_per_sm);
@@ -962,7 +972,8 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     };
     act_blocks = ctas_for(P.n_items, kWarpsPerCta, act_bps * n_sms);
     cand_blocks = ctas_for(cand_work, kWarpsPerCta, cand_bps * n_sms);  // the exact-rows phase shares this launch
-    mega_grid = ctas_for(std::max(cand_work, (long long)P.n_chg_words), warps, std::max(1, mega_bps) * n_sms);
+    mega_grid = one_cta ? 1
+                        : ctas_for(std::max(cand_work, (long long)P.n_chg_words), warps, std::max(1, mega_bps) * n_sms);
     mega_warps = warps;
     if (graph_exec && (opts.ctas_per_sm != ctas_per_sm)) {  // the GPU_LOOP graph holds the old grids
         cudaGraphExecDestroy(graph_exec);

@@ -164,6 +164,7 @@ struct DevProblem {
     // the next phase, so the FP64 pipe sees full warps.
     // Class lg's queue is xrow[cls_begin[lg] .. cls_end[lg]) (its row positions
     // are exactly that range, slices being sorted by g).
+    int in_place;          // the screen's warp runs its rows' exact pass (the round loop's choice)
     int cls_begin[6], cls_end[6];
     XRow *xrow;            // n_srows
     unsigned *xctr;        // [parity * 16 + lg]: queue tails, [parity * 16 + 8]: claimed items
@@ -229,7 +230,8 @@ int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, 
 // whether another one follows} at the end of the launch. cta_warps: 4, 8 or 16
 // warps per CTA.
 int launch_megakernel(const DevProblem &P, int first, int last, int *mail, int grid, int cta_warps, cudaStream_t s);
-int phase_occupancy(int *act_blocks_per_sm, int *cand_blocks_per_sm, int *mega_blocks_per_sm, int cta_warps);
+int phase_occupancy(int *act_blocks_per_sm, int *cand_blocks_per_sm, int *mega_blocks_per_sm, int cta_warps,
+                    bool in_place);
 // Phase timers of the megakernel (a library built with GDP_PHASE_TIMERS):
 // 0 or a CUDA error; -1 when the library was built without them.
 int phase_timers_clear();

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_activity(const __grid_consta
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible) return;
     stats_zero(ws[threadIdx.x >> 5], threadIdx.x & 31);
-    activity_phase(P, round, P.flags[0].mark_cur != 0, P.queue + 0, &P.flags[0].change, &P.flags[0].tight,
+    activity_phase<true>(P, round, P.flags[0].mark_cur != 0, P.queue + 0, &P.flags[0].change, &P.flags[0].tight,
                    ws[threadIdx.x >> 5], threadIdx.x & 31);
     stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
@@ -190,7 +190,12 @@ __device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, 
 // needed. Between launches barrier[1] keeps the barrier count and the round's
 // tightenings the next round's mode. mail (may be null): host memory that
 // receives {the round, whether another one follows}.
-template <int W>
+// kInPlace (P.in_place): a small problem of one-lane rows only, with a warp for
+// each slice: the screen's warp takes its rows through the exact pass at once,
+// which saves the queue, a phase and a barrier (2,000 rows of 2 to 16: 0.50 ->
+// 0.42 ms). With wide rows in the problem their items would follow one another
+// on one warp (2,000 power-law rows: 1.86 -> 2.34 ms), and they are deferred.
+template <int W, bool kInPlace>
 __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_constant__ DevProblem P, int first,
                                                                int last, int *mail) {
     WarpSmem *ws = warp_smem();
@@ -212,7 +217,7 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_cons
             unsigned *q = P.queue + 4 * par;
             timer_stamp(P, round, 0);
             unsigned long long t0 = timer_now();
-            activity_phase(P, round, marked, q + 0, change, tight, mine, lane, par);
+            activity_phase<!kInPlace>(P, round, marked, q + 0, change, tight, mine, lane, par);
             timer_busy(P, mine, lane, round, 0, t0);
             if (!grid_barrier(P.barrier, err, P.spin_limit, target)) return;
             timer_stamp(P, round, 1);
@@ -226,8 +231,8 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_cons
                 if (P.xctr)
                     for (int i = 0; i < 16; i++) P.xctr[16 * (par ^ 1) + i] = 0u;
             }
-            const bool xrows = exact_rows_queued(P, par);
-            if (xrows || P.n_mtiles) {
+            const bool xrows = !kInPlace && exact_rows_queued(P, par);
+            if (!kInPlace && (xrows || P.n_mtiles)) {
                 t0 = timer_now();
                 if (P.n_mtiles) candidate_phase(P, round, marked, exact, mine, lane);  // heavy items first
                 timer_busy(P, mine, lane, round, 1, t0);
@@ -345,17 +350,17 @@ int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, 
 }
 
 namespace {
-const void *megakernel_of(int cta_warps) {
+const void *megakernel_of(int cta_warps, bool in_place) {
     switch (cta_warps) {
-        case 4: return (const void *)k_megakernel<4>;
-        case 16: return (const void *)k_megakernel<16>;
-        default: return (const void *)k_megakernel<8>;
+        case 4: return in_place ? (const void *)k_megakernel<4, true> : (const void *)k_megakernel<4, false>;
+        case 16: return in_place ? (const void *)k_megakernel<16, true> : (const void *)k_megakernel<16, false>;
+        default: return in_place ? (const void *)k_megakernel<8, true> : (const void *)k_megakernel<8, false>;
     }
 }
 }  // namespace
 
-int phase_occupancy(int *act, int *cand, int *mega, int cta_warps) {
-    const void *mk = megakernel_of(cta_warps);
+int phase_occupancy(int *act, int *cand, int *mega, int cta_warps, bool in_place) {
+    const void *mk = megakernel_of(cta_warps, in_place);
     const size_t mega_smem = sizeof(WarpSmem) * (size_t)cta_warps;
     cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mega_smem);
     for (const void *k : {(const void *)k_activity, (const void *)k_candidates, (const void *)k_exact})
@@ -374,7 +379,7 @@ int phase_occupancy(int *act, int *cand, int *mega, int cta_warps) {
 int launch_megakernel(const DevProblem &P, int first, int last, int *mail, int grid, int cta_warps, cudaStream_t s) {
     DevProblem Pc = P;
     void *args[] = {&Pc, &first, &last, &mail};
-    return (int)cudaLaunchCooperativeKernel(megakernel_of(cta_warps), dim3(grid), dim3(32 * cta_warps), args,
+    return (int)cudaLaunchCooperativeKernel(megakernel_of(cta_warps, P.in_place != 0), dim3(grid), dim3(32 * cta_warps), args,
                                             sizeof(WarpSmem) * (size_t)cta_warps, s);
 }
 
