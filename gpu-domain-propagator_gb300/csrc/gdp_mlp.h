@@ -34,6 +34,7 @@ public:
     MlpDev dev() const;
 
     int device = 0;
+    bool host_direct = false;  // kernels read and write pageable host memory (coherent access)
     cudaStream_t stream = nullptr;
     float *p = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *loss = nullptr;
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w2t = nullptr, *w3 = nullptr;
