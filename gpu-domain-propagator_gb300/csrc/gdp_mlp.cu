@@ -14,8 +14,10 @@
 //   dh1     = bf16(da2) @ W2          (tensor cores, W2^T as the B operand)
 //   da1     = dh1 [a1 > 0]
 //   g_W1   += da1^T x,                g_b1 += da1        (FP32, CUDA cores)
-// Weight gradients of a CTA accumulate in shared memory and reach global
-// memory with one atomic per parameter per CTA.
+// Each warp adds its tiles' weight gradients to sums of its own in shared
+// memory, a CTA writes the sum over its warps to its row of a partial array, and
+// the optimizer step (or the gradient call) adds up the rows: no atomics, and
+// every sum in a fixed order, so equal calls give equal bits.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -31,28 +33,43 @@ namespace {
 constexpr int kMlpWarps = 4;
 constexpr int kMlpThreads = 32 * kMlpWarps;
 
-// Per-warp tile scratch (FP32): da2, h1 (bf16-rounded relu(a1)), da1, x.
-// Rows of 64 values are padded to 72 floats: the fragment-layout stores and
-// loads (lanes 4g + t at row g, column 2t + c) then meet at most 2 lanes per
-// bank instead of 8.
+// Per-warp scratch of a tile (FP32) and the warp's gradient sums. da holds da2
+// and then da1, transposed: the 16 samples of a column are 64 consecutive bytes,
+// four 16-byte loads that every lane of the warp shares (rows of 20 floats:
+// aligned, and the stores of a fragment's columns fall in different banks).
 constexpr int kTileLd = kMlpH + 8;
 struct TileSmem {
-    float da2[16][kTileLd];
+    float da[kMlpH][20];
     float h1[16][kTileLd];
-    float da1[16][kTileLd];
     float x[16][kMlpIn];
+    float sum[(kMlpParams + 4) & ~3];  // parameters, then the loss
 };
+constexpr int kPartLd = kMlpParams + 1;  // a CTA's row of the partial sums: gradient, loss
+constexpr int kGradWarpsFew = 4, kGradWarpsMany = 7;  // 32 KB of shared memory per warp
 
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// A registers of rows [r0, r0 + 16) of a row-major BF16 [n][16] array (zero past n).
-__device__ __forceinline__ void load_a_global(const __nv_bfloat16 *X, int n, int r0, int lane, unsigned (&a)[4]) {
+// Samples [r0, r0 + 16) of [0, n), sample r being number perm[r] (perm null: r)
+// of a row-major BF16 [.][16] array: A registers, labels and weights of rows g
+// and g + 8, zero past n.
+__device__ __forceinline__ void load_samples(const __nv_bfloat16 *X, const int *perm, const float *y, const float *w,
+                                             int n, int r0, int lane, unsigned (&a)[4], float (&yy)[2],
+                                             float (&ww)[2]) {
     const int g = lane >> 2, t = lane & 3;
-    const int ra = r0 + g, rb = r0 + g + 8;
-    a[0] = ra < n ? __ldg(reinterpret_cast<const unsigned *>(X + (size_t)ra * 16 + 2 * t)) : 0u;
-    a[1] = rb < n ? __ldg(reinterpret_cast<const unsigned *>(X + (size_t)rb * 16 + 2 * t)) : 0u;
-    a[2] = ra < n ? __ldg(reinterpret_cast<const unsigned *>(X + (size_t)ra * 16 + 2 * t + 8)) : 0u;
-    a[3] = rb < n ? __ldg(reinterpret_cast<const unsigned *>(X + (size_t)rb * 16 + 2 * t + 8)) : 0u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int r = r0 + g + 8 * h;
+        a[h] = a[2 + h] = 0u;
+        yy[h] = ww[h] = 0.f;
+        if (r < n) {
+            const int k = perm ? __ldg(perm + r) : r;
+            const unsigned *x = reinterpret_cast<const unsigned *>(X + (size_t)k * kMlpIn) + t;
+            a[h] = __ldg(x);
+            a[2 + h] = __ldg(x + 4);
+            yy[h] = __ldg(y + k);
+            ww[h] = __ldg(w + k);
+        }
+    }
 }
 
 // Logits of n rows of FP32 features. X and z may be host memory that the device
@@ -98,45 +115,78 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(MlpDev M, const flo
     }
 }
 
-// Gradient of the weighted BCE over samples [0, n); grad (kMlpParams floats,
-// zeroed by the caller) and loss (1 float) receive atomic adds.
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_grad(MlpDev M, const __nv_bfloat16 *X, const float *y,
-                                                           const float *w, int n, float inv_wsum, float *grad,
-                                                           float *loss) {
+// Gradient of the weighted BCE over samples [0, n) (sample r is perm[r], or r):
+// row blockIdx.x of part receives the CTA's sums and its loss. W warps per CTA,
+// one CTA per SM. A minibatch of 8,192 is 512 tiles, one per warp of 128 CTAs:
+// what bounds it is the time of one tile on one warp -- forward, 64 x 64 and
+// 64 x 16 FP32 outer products of 16 samples -- 11 us, of which the FP32
+// multiply-adds need 1.4. The outer products keep four rows in flight, and their
+// row values come four to a load. Gradients added by shared and global atomics
+// took 24 us and 19 on clearing them, the Adam step and the BF16 copies; a step
+// of this kernel and k_mlp_step is 16 us (46 before).
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_mlp_grad(MlpDev M, const __nv_bfloat16 *X, const int *perm, const float *y,
+                                                     const float *w, int n, float inv_wsum, float *part) {
     extern __shared__ float4 smem_raw[];
-    float *acc = reinterpret_cast<float *>(smem_raw);  // kMlpParams
-    TileSmem *tiles = reinterpret_cast<TileSmem *>(acc + ((kMlpParams + 3) & ~3));
+    TileSmem *tiles = reinterpret_cast<TileSmem *>(smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     TileSmem &S = tiles[wid];
-    for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) acc[i] = 0.f;
-    __syncthreads();
-    float *gW1 = acc + kOffW1, *gb1 = acc + kOffB1, *gW2 = acc + kOffW2, *gb2 = acc + kOffB2, *gw3 = acc + kOffW3,
-          *gb3 = acc + kOffB3;
+    for (int i = lane; i < kPartLd; i += 32) S.sum[i] = 0.f;
+    float *gW1 = S.sum + kOffW1, *gb1 = S.sum + kOffB1, *gW2 = S.sum + kOffW2, *gb2 = S.sum + kOffB2,
+          *gw3 = S.sum + kOffW3;
     const int g = lane >> 2, t = lane & 3;
-    const int warp = blockIdx.x * kMlpWarps + wid, nwarps = gridDim.x * kMlpWarps;
-    float lsum = 0.f;
-    for (int r0 = warp * 16; r0 < n; r0 += nwarps * 16) {
+    const int ntiles = (n - 1) / 16 + 1;
+    float lsum = 0.f, b3sum = 0.f;
+    __syncwarp();
+    int tile = blockIdx.x * W + wid;
+    unsigned an[4];  // the next tile's samples
+    float yn[2], wn[2];
+    load_samples(X, perm, y, w, tile < ntiles ? n : 0, 16 * (tile < ntiles ? tile : 0), lane, an, yn, wn);
+    // up to here the kernel may run while the optimizer step before it ends
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    while (tile < ntiles) {
+        const int r0 = 16 * tile;
         unsigned a[4];
-        load_a_global(X, n, r0, lane, a);
+        float yy[2], ww[2];
+#pragma unroll
+        for (int q = 0; q < 4; q++) a[q] = an[q];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            yy[h] = yn[h];
+            ww[h] = wn[h];
+        }
+        tile = ntiles - tile > gridDim.x * W ? tile + gridDim.x * W : ntiles;
+        if (tile < ntiles) load_samples(X, perm, y, w, n, 16 * tile, lane, an, yn, wn);
         MlpTile T;
         mlp_forward_tile(M, a, lane, T);
+        // the tile's inputs (FP32 copy of the A registers)
+        {
+            const __nv_bfloat162 *v = reinterpret_cast<const __nv_bfloat162 *>(a);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float2 f = __bfloat1622float2(v[q]);
+                *reinterpret_cast<float2 *>(&S.x[g + 8 * (q & 1)][2 * t + 8 * (q >> 1)]) = f;
+            }
+        }
         // per-row dz (rows g and g + 8)
         float dz[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int r = r0 + g + 8 * h;
             dz[h] = 0.f;
-            if (r < n) {
-                const float zz = T.z[h], yy = __ldg(y + r), ww = __ldg(w + r);
-                const float p = 1.f / (1.f + __expf(-zz));
-                dz[h] = ww * (p - yy) * inv_wsum;
+            if (r0 + g + 8 * h < n) {
+                const float zz = T.z[h], p = 1.f / (1.f + __expf(-zz));
+                dz[h] = ww[h] * (p - yy[h]) * inv_wsum;
                 // BCE with logits: max(z, 0) - z y + log(1 + exp(-|z|))
-                if (t == 0) lsum += ww * (fmaxf(zz, 0.f) - zz * yy + log1pf(__expf(-fabsf(zz)))) * inv_wsum;
+                if (t == 0) lsum += ww[h] * (fmaxf(zz, 0.f) - zz * yy[h] + log1pf(__expf(-fabsf(zz)))) * inv_wsum;
             }
         }
-        // layer 3 and da2
+        if (t == 0) b3sum += dz[0] + dz[1];
+        // layer 3, da2 and the layer-1 activations; da2's A registers for dh1
+        unsigned da[4][4];
 #pragma unroll
         for (int nt = 0; nt < 8; nt++) {
+            float d[4];
 #pragma unroll
             for (int c = 0; c < 2; c++) {
                 const int col = nt * 8 + 2 * t + c;
@@ -146,33 +196,67 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_grad(MlpDev M, const __nv_b
                 gw += __shfl_xor_sync(0xffffffffu, gw, 4);
                 gw += __shfl_xor_sync(0xffffffffu, gw, 8);
                 gw += __shfl_xor_sync(0xffffffffu, gw, 16);
-                if (g == 0) atomicAdd(gw3 + col, gw);
-                S.da2[g][col] = T.a2[nt][c] > 0.f ? dz[0] * w3 : 0.f;
-                S.da2[g + 8][col] = T.a2[nt][2 + c] > 0.f ? dz[1] * w3 : 0.f;
+                if (g == 0) gw3[col] += gw;
+                d[c] = T.a2[nt][c] > 0.f ? dz[0] * w3 : 0.f;
+                d[2 + c] = T.a2[nt][2 + c] > 0.f ? dz[1] * w3 : 0.f;
+                S.da[col][g] = d[c];
+                S.da[col][g + 8] = d[2 + c];
                 S.h1[g][col] = bf16r(fmaxf(T.a1[nt][c], 0.f));
                 S.h1[g + 8][col] = bf16r(fmaxf(T.a1[nt][2 + c], 0.f));
             }
-        }
-        {
-            float gb = (t == 0) ? dz[0] + dz[1] : 0.f;
-            for (int off = 16; off > 0; off >>= 1) gb += __shfl_xor_sync(0xffffffffu, gb, off);
-            if (lane == 0) atomicAdd(gb3, gb);
-        }
-        // x tile (FP32 copy of the BF16 inputs)
-        for (int i = lane; i < 16 * kMlpIn; i += 32) {
-            const int r = i / kMlpIn, k = i % kMlpIn;
-            S.x[r][k] = r0 + r < n ? __bfloat162float(X[(size_t)(r0 + r) * kMlpIn + k]) : 0.f;
+            da[nt >> 1][2 * (nt & 1)] = pack_bf16(d[0], d[1]);
+            da[nt >> 1][2 * (nt & 1) + 1] = pack_bf16(d[2], d[3]);
         }
         __syncwarp();
-        // dh1 = bf16(da2) @ W2 on the tensor cores
-        unsigned da[4][4];
+        // weight gradients of the tile, each a sum over its 16 samples in
+        // sample order: column `row` of da against the samples' inputs
+        auto column = [&](int row, float (&d)[16]) {
 #pragma unroll
-        for (int kt = 0; kt < 4; kt++) {
-            da[kt][0] = pack_bf16(S.da2[g][kt * 16 + 2 * t], S.da2[g][kt * 16 + 2 * t + 1]);
-            da[kt][1] = pack_bf16(S.da2[g + 8][kt * 16 + 2 * t], S.da2[g + 8][kt * 16 + 2 * t + 1]);
-            da[kt][2] = pack_bf16(S.da2[g][kt * 16 + 2 * t + 8], S.da2[g][kt * 16 + 2 * t + 9]);
-            da[kt][3] = pack_bf16(S.da2[g + 8][kt * 16 + 2 * t + 8], S.da2[g + 8][kt * 16 + 2 * t + 9]);
+            for (int q = 0; q < 4; q++) {
+                const float4 v = *reinterpret_cast<const float4 *>(&S.da[row][4 * q]);
+                d[4 * q] = v.x; d[4 * q + 1] = v.y; d[4 * q + 2] = v.z; d[4 * q + 3] = v.w;
+            }
+        };
+        {  // W2: lane owns columns lane and lane + 32 of every row; b2: rows lane and lane + 32
+            float hl[16], hh[16];
+#pragma unroll
+            for (int s = 0; s < 16; s++) {
+                hl[s] = S.h1[s][lane];
+                hh[s] = S.h1[s][lane + 32];
+            }
+            for (int row = 0; row < kMlpH; row += 4) {  // four rows' chains in flight
+                float d[4][16], vl[4], vh[4], ol[4], oh[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    column(row + u, d[u]);
+                    ol[u] = gW2[(row + u) * kMlpH + lane];
+                    oh[u] = gW2[(row + u) * kMlpH + lane + 32];
+                    vl[u] = vh[u] = 0.f;
+                }
+#pragma unroll
+                for (int s = 0; s < 16; s++)
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        vl[u] = fmaf(d[u][s], hl[s], vl[u]);
+                        vh[u] = fmaf(d[u][s], hh[s], vh[u]);
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    gW2[(row + u) * kMlpH + lane] = ol[u] + vl[u];
+                    gW2[(row + u) * kMlpH + lane + 32] = oh[u] + vh[u];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                float d[16], v = 0.f;
+                column(lane + 32 * q, d);
+#pragma unroll
+                for (int s = 0; s < 16; s++) v += d[s];
+                gb2[lane + 32 * q] += v;
+            }
         }
+        // dh1 = bf16(da2) @ W2 on the tensor cores; da1 takes da2's place
+        __syncwarp();
 #pragma unroll
         for (int nt = 0; nt < 8; nt++) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
@@ -185,94 +269,135 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_grad(MlpDev M, const __nv_b
 #pragma unroll
             for (int cc = 0; cc < 2; cc++) {
                 const int col = nt * 8 + 2 * t + cc;
-                S.da1[g][col] = T.a1[nt][cc] > 0.f ? c[cc] : 0.f;
-                S.da1[g + 8][col] = T.a1[nt][2 + cc] > 0.f ? c[2 + cc] : 0.f;
+                S.da[col][g] = T.a1[nt][cc] > 0.f ? c[cc] : 0.f;
+                S.da[col][g + 8] = T.a1[nt][2 + cc] > 0.f ? c[2 + cc] : 0.f;
             }
         }
         __syncwarp();
-        // weight gradients of the tile, each a sum over its 16 samples in
-        // sample order. Lanes own columns: a row's reads are broadcasts and
-        // the 32 shared-memory adds of one instruction go to 32 banks.
-        //   b2, b1: lane owns rows lane and lane + 32
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int row = lane + 32 * q;
-            float sb2 = 0.f, sb1 = 0.f;
-            for (int s = 0; s < 16; s++) {
-                sb2 += S.da2[s][row];
-                sb1 += S.da1[s][row];
-            }
-            atomicAdd(gb2 + row, sb2);
-            atomicAdd(gb1 + row, sb1);
-        }
-        {  // W2: lane owns columns lane and lane + 32 of every row
-            float hl[16], hh[16];
-#pragma unroll
-            for (int s = 0; s < 16; s++) {
-                hl[s] = S.h1[s][lane];
-                hh[s] = S.h1[s][lane + 32];
-            }
-            for (int row = 0; row < kMlpH; row++) {
-                float vl = 0.f, vh = 0.f;
-#pragma unroll
-                for (int s = 0; s < 16; s++) {
-                    const float d = S.da2[s][row];
-                    vl = fmaf(d, hl[s], vl);
-                    vh = fmaf(d, hh[s], vh);
-                }
-                atomicAdd(gW2 + row * kMlpH + lane, vl);
-                atomicAdd(gW2 + row * kMlpH + lane + 32, vh);
-            }
-        }
-        {  // W1: lane owns column lane & 15 of the rows of parity lane >> 4
+        {  // W1: lane owns column lane & 15 of the rows of parity lane >> 4; b1 as b2
             const int k = lane & 15;
             float xs[16];
 #pragma unroll
             for (int s = 0; s < 16; s++) xs[s] = S.x[s][k];
-            for (int rr = 0; rr < kMlpH / 2; rr++) {
-                const int row = 2 * rr + (lane >> 4);
-                float v = 0.f;
+            for (int r = lane >> 4; r < kMlpH; r += 8) {
+                float d[4][16], v[4], o[4];
 #pragma unroll
-                for (int s = 0; s < 16; s++) v = fmaf(S.da1[s][row], xs[s], v);
-                atomicAdd(gW1 + row * kMlpIn + k, v);
+                for (int u = 0; u < 4; u++) {
+                    column(r + 2 * u, d[u]);
+                    o[u] = gW1[(r + 2 * u) * kMlpIn + k];
+                    v[u] = 0.f;
+                }
+#pragma unroll
+                for (int s = 0; s < 16; s++)
+#pragma unroll
+                    for (int u = 0; u < 4; u++) v[u] = fmaf(d[u][s], xs[s], v[u]);
+#pragma unroll
+                for (int u = 0; u < 4; u++) gW1[(r + 2 * u) * kMlpIn + k] = o[u] + v[u];
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                float d[16], v = 0.f;
+                column(lane + 32 * q, d);
+#pragma unroll
+                for (int s = 0; s < 16; s++) v += d[s];
+                gb1[lane + 32 * q] += v;
             }
         }
         __syncwarp();
     }
-    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-    if (lane == 0) atomicAdd(loss, lsum);
+    for (int off = 16; off > 0; off >>= 1) {
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+        b3sum += __shfl_xor_sync(0xffffffffu, b3sum, off);
+    }
+    if (lane == 0) {
+        S.sum[kOffB3] = b3sum;
+        S.sum[kMlpParams] = lsum;
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x)
-        if (acc[i] != 0.f) atomicAdd(grad + i, acc[i]);
-}
-
-// Adam step on the FP32 master parameters, then the BF16 copies.
-__global__ void k_mlp_adam(float *p, float *m1, float *m2, const float *grad, int step, float lr, float beta1,
-                           float beta2, float eps) {
-    const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParams; i += gridDim.x * blockDim.x) {
-        const float gr = grad[i];
-        const float a = beta1 * m1[i] + (1.f - beta1) * gr;
-        const float b = beta2 * m2[i] + (1.f - beta2) * gr * gr;
-        m1[i] = a;
-        m2[i] = b;
-        p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+    for (int i = threadIdx.x; i < kPartLd; i += 32 * W) {
+        float v = tiles[0].sum[i];
+#pragma unroll
+        for (int q = 1; q < W; q++) v += tiles[q].sum[i];
+        part[(size_t)blockIdx.x * kPartLd + i] = v;
     }
 }
 
-// BF16 copies of the master weights, W1, W2 and W2 transposed in fragment
-// order (frag_index).
+// Adds up column i of the `rows` partial rows, in order within 8 interleaved
+// groups of rows and over the groups: 8 threads per column (threadIdx.y), whose
+// loads are coalesced across columns. Every thread of threadIdx.y == 0 returns
+// the sum.
+constexpr int kSumCols = 32, kSumGroups = 8;
+__device__ __forceinline__ float sum_partials(const float *part, int rows, int i, float (&sh)[kSumGroups][kSumCols]) {
+    float v = 0.f;
+    if (i < kPartLd) {
+#pragma unroll 8
+        for (int r = threadIdx.y; r < rows; r += kSumGroups) v += __ldcg(part + (size_t)r * kPartLd + i);
+    }
+    sh[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+        v = sh[0][threadIdx.x];
+#pragma unroll
+        for (int q = 1; q < kSumGroups; q++) v += sh[q][threadIdx.x];
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(kSumCols *kSumGroups) k_mlp_sum(const float *part, int rows, float *grad, float *loss) {
+    __shared__ float sh[kSumGroups][kSumCols];
+    const int i = blockIdx.x * kSumCols + threadIdx.x;
+    const float v = sum_partials(part, rows, i, sh);
+    if (threadIdx.y == 0 && i < kMlpParams) grad[i] = v;
+    if (threadIdx.y == 0 && i == kMlpParams) *loss = v;
+}
+
+// BF16 copies of master parameter i: W1, W2, W2 transposed in fragment order
+// (frag_index), w3.
+__device__ __forceinline__ void cast_param(int i, float v, __nv_bfloat16 *w1, __nv_bfloat16 *w2, __nv_bfloat16 *w2t,
+                                           __nv_bfloat16 *w3) {
+    static_assert(kMlpIn == 16 && kMlpH % 16 == 0, "one k-tile for layer 1, whole k-tiles for layer 2");
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    if (i < kOffB1) {
+        w1[frag_index(i / kMlpIn, i % kMlpIn, 1)] = b;
+    } else if (i >= kOffW2 && i < kOffB2) {
+        const int r = (i - kOffW2) / kMlpH, c = (i - kOffW2) % kMlpH;
+        w2[frag_index(r, c, kMlpH / 16)] = b;
+        w2t[frag_index(c, r, kMlpH / 16)] = b;
+    } else if (i >= kOffW3 && i < kOffB3) {
+        w3[i - kOffW3] = b;
+    }
+}
+
+// One optimizer step from the partial rows: gradient sums, Adam on the FP32
+// master parameters, their BF16 copies, the minibatch's loss. Bound by its chain
+// of loads from L2 (4.5 us for 152 rows, 3.2 MB); a last CTA of the gradient
+// kernel doing this would read them through one SM.
+__global__ void __launch_bounds__(kSumCols *kSumGroups)
+        k_mlp_step(const float *part, int rows, float *p, float *m1, float *m2, int step, float lr, float beta1,
+                   float beta2, float eps, __nv_bfloat16 *w1, __nv_bfloat16 *w2, __nv_bfloat16 *w2t,
+                   __nv_bfloat16 *w3, float *loss) {
+    __shared__ float sh[kSumGroups][kSumCols];
+    const int i = blockIdx.x * kSumCols + threadIdx.x;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const float gr = sum_partials(part, rows, i, sh);
+    if (threadIdx.y != 0) return;
+    if (i == kMlpParams) *loss = gr;
+    if (i >= kMlpParams) return;
+    const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
+    const float a = beta1 * m1[i] + (1.f - beta1) * gr;
+    const float b = beta2 * m2[i] + (1.f - beta2) * gr * gr;
+    m1[i] = a;
+    m2[i] = b;
+    const float v = p[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    p[i] = v;
+    cast_param(i, v, w1, w2, w2t, w3);
+}
+
 __global__ void k_mlp_cast(const float *p, __nv_bfloat16 *w1, __nv_bfloat16 *w2, __nv_bfloat16 *w2t,
                            __nv_bfloat16 *w3) {
-    static_assert(kMlpIn == 16 && kMlpH % 16 == 0, "one k-tile for layer 1, whole k-tiles for layer 2");
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpH * kMlpH; i += gridDim.x * blockDim.x) {
-        const int r = i / kMlpH, c = i % kMlpH;
-        const __nv_bfloat16 v = __float2bfloat16_rn(p[kOffW2 + i]);
-        w2[frag_index(r, c, kMlpH / 16)] = v;
-        w2t[frag_index(c, r, kMlpH / 16)] = v;
-        if (i < kMlpH * kMlpIn) w1[frag_index(i / kMlpIn, i % kMlpIn, 1)] = __float2bfloat16_rn(p[kOffW1 + i]);
-        if (i < kMlpH) w3[i] = __float2bfloat16_rn(p[kOffW3 + i]);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParams; i += gridDim.x * blockDim.x)
+        cast_param(i, p[i], w1, w2, w2t, w3);
 }
 
 __global__ void k_to_bf16(const float *x, __nv_bfloat16 *y, long long n) {
@@ -293,7 +418,6 @@ __global__ void k_to_bf16(const float *x, __nv_bfloat16 *y, long long n) {
     } while (0)
 
 namespace {
-constexpr size_t kGradSmem = sizeof(float) * ((kMlpParams + 3) & ~3) + sizeof(TileSmem) * kMlpWarps;
 
 unsigned long long splitmix(unsigned long long &s) {
     unsigned long long z = (s += 0x9E3779B97F4A7C15ULL);
@@ -310,10 +434,42 @@ int device_sms() {
     return sms;
 }
 
-// Gradient: two CTAs per SM (its registers allow no more), at most one per 4 tiles.
-int grad_grid(int n) {
-    const int tiles = (n + 15) / 16;
-    return std::max(1, std::min(2 * device_sms(), (tiles + kMlpWarps - 1) / kMlpWarps));
+constexpr int kSumBlocks = (kPartLd + kSumCols - 1) / kSumCols;
+
+// A launch whose blocks may become resident, and run up to their grid
+// dependency, while the kernel before it ends (early): the two kernels of a
+// training step alternate, each reads what the other wrote only after that.
+struct LaunchNext {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    LaunchNext(int grid, dim3 block, size_t smem, bool early, cudaStream_t s) {
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = early;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+// Rows of the partial array: at most one CTA per SM.
+int grad_rows_max() { return device_sms(); }
+
+// Enqueues the gradient of samples [0, n): one CTA per SM, 4 warps while that
+// gives every tile a warp of its own, else 7, what the shared memory holds (most
+// warps then have a second one on their SM quarter to overlap with: 2M samples
+// take 1.1 ms instead of 1.8).
+cudaError_t launch_grad(const MlpDev &M, const __nv_bfloat16 *X, const int *perm, const float *y, const float *w, int n,
+                        float inv_wsum, float *part, int *rows, bool early, cudaStream_t s) {
+    const int tiles = (n - 1) / 16 + 1, sms = device_sms();
+    const bool few = tiles <= sms * kGradWarpsFew;
+    const int warps = few ? kGradWarpsFew : kGradWarpsMany;
+    *rows = std::min(sms, (tiles + warps - 1) / warps);
+    LaunchNext L(*rows, 32 * warps, sizeof(TileSmem) * warps, early, s);
+    return few ? cudaLaunchKernelEx(&L.cfg, k_mlp_grad<kGradWarpsFew>, M, X, perm, y, w, n, inv_wsum, part)
+               : cudaLaunchKernelEx(&L.cfg, k_mlp_grad<kGradWarpsMany>, M, X, perm, y, w, n, inv_wsum, part);
 }
 
 // Forward: every CTA that fits on an SM (the loop waits on its loads, and more
@@ -366,7 +522,10 @@ GDP_RETCODE Mlp::init(unsigned long long seed, int dev_index) {
     GDP_MCUDA(cudaMalloc(&w2, sizeof(__nv_bfloat16) * kMlpH * kMlpH));
     GDP_MCUDA(cudaMalloc(&w2t, sizeof(__nv_bfloat16) * kMlpH * kMlpH));
     GDP_MCUDA(cudaMalloc(&w3, sizeof(__nv_bfloat16) * kMlpH));
-    GDP_MCUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem));
+    GDP_MCUDA(cudaFuncSetAttribute(k_mlp_grad<kGradWarpsFew>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(TileSmem) * kGradWarpsFew));
+    GDP_MCUDA(cudaFuncSetAttribute(k_mlp_grad<kGradWarpsMany>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(TileSmem) * kGradWarpsMany));
     // He-uniform weights, zero biases
     std::vector<float> h(kMlpParams, 0.f);
     unsigned long long s = seed;
@@ -399,22 +558,36 @@ GDP_RETCODE Mlp::get(float *params) const {
 }
 
 namespace {
-// Uploads n x 16 FP32 features as BF16 (device buffer owned by the caller).
-GDP_RETCODE upload_x(const float *x, int n, __nv_bfloat16 **out, cudaStream_t s) {
-    float *tmp = nullptr;
+// A call's kernels and copies use its host memory: one that fails waits for
+// them before its buffers are given back.
+struct Drained {
+    cudaStream_t s;
+    ~Drained() { cudaStreamSynchronize(s); }
+};
+}  // namespace
+
+// Samples on the device: features as BF16, labels, weights (device memory of
+// `mem`). With coherent access the features are read from host memory by the
+// conversion kernel, which does not hold up the calling thread.
+GDP_RETCODE Mlp::upload(Arena &mem, int n, const float *x, const float *y, const float *w, __nv_bfloat16 **xb,
+                        float **dy, float **dw) {
     const size_t cnt = (size_t)n * kMlpIn;
-    GDP_MCUDA(cudaMalloc(&tmp, sizeof(float) * std::max<size_t>(cnt, 1)));
-    GDP_MCUDA(cudaMalloc(out, sizeof(__nv_bfloat16) * std::max<size_t>(cnt, 1)));
-    if (cnt) {
-        GDP_MCUDA(cudaMemcpyAsync(tmp, x, sizeof(float) * cnt, cudaMemcpyHostToDevice, s));
-        k_to_bf16<<<256, 256, 0, s>>>(tmp, *out, (long long)cnt);
-        GDP_MCUDA(cudaGetLastError());
+    *xb = (__nv_bfloat16 *)mem.alloc_bytes(sizeof(__nv_bfloat16) * cnt);
+    *dy = (float *)mem.alloc_bytes(sizeof(float) * (size_t)n);
+    *dw = (float *)mem.alloc_bytes(sizeof(float) * (size_t)n);
+    const float *src = x;
+    if (!host_direct || reinterpret_cast<uintptr_t>(x) % alignof(float)) {
+        float *up = (float *)mem.alloc_bytes(sizeof(float) * cnt);
+        if (up) GDP_MCUDA(cudaMemcpyAsync(up, x, sizeof(float) * cnt, cudaMemcpyHostToDevice, stream));
+        src = up;
     }
-    GDP_MCUDA(cudaStreamSynchronize(s));
-    cudaFree(tmp);
+    if (!*xb || !*dy || !*dw || !src) { set_error("device allocation failed (samples)"); return GDP_ERROR; }
+    GDP_MCUDA(cudaMemcpyAsync(*dy, y, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream));
+    GDP_MCUDA(cudaMemcpyAsync(*dw, w, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, stream));
+    k_to_bf16<<<4 * device_sms(), 256, 0, stream>>>(src, *xb, (long long)cnt);
+    GDP_MCUDA(cudaGetLastError());
     return GDP_OKAY;
 }
-}  // namespace
 
 GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     if (n < 0 || (n && (!x || !z))) { set_error("bad forward arguments"); return GDP_ERROR; }
@@ -442,28 +615,26 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
 
 GDP_RETCODE Mlp::gradient(int n, const float *x, const float *y, const float *w, float *g, float *lossv) {
     if (n <= 0 || !x || !y || !w || !g) { set_error("bad gradient arguments"); return GDP_ERROR; }
-    __nv_bfloat16 *xb = nullptr;
-    float *dy = nullptr, *dw = nullptr;
-    if (upload_x(x, n, &xb, stream) != GDP_OKAY) return GDP_ERROR;
-    GDP_MCUDA(cudaMalloc(&dy, sizeof(float) * n));
-    GDP_MCUDA(cudaMalloc(&dw, sizeof(float) * n));
-    GDP_MCUDA(cudaMemcpyAsync(dy, y, sizeof(float) * n, cudaMemcpyHostToDevice, stream));
-    GDP_MCUDA(cudaMemcpyAsync(dw, w, sizeof(float) * n, cudaMemcpyHostToDevice, stream));
+    GDP_MCUDA(cudaSetDevice(device));
+    Arena mem;
+    const Drained drained{stream};
+    __nv_bfloat16 *xb;
+    float *dy, *dw;
+    if (upload(mem, n, x, y, w, &xb, &dy, &dw) != GDP_OKAY) return GDP_ERROR;
+    float *part = (float *)mem.alloc_bytes(sizeof(float) * kPartLd * (size_t)grad_rows_max());
+    if (!part) { set_error("device allocation failed (gradient)"); return GDP_ERROR; }
     double ws = 0.0;
     for (int i = 0; i < n; i++) ws += w[i];
-    GDP_MCUDA(cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, stream));
-    GDP_MCUDA(cudaMemsetAsync(loss, 0, sizeof(float), stream));
-    k_mlp_grad<<<grad_grid(n), kMlpThreads, kGradSmem, stream>>>(dev(), xb, dy, dw, n,
-                                                                   ws > 0 ? (float)(1.0 / ws) : 0.f, grad, loss);
+    int rows = 0;
+    GDP_MCUDA(launch_grad(dev(), xb, nullptr, dy, dw, n, ws > 0 ? (float)(1.0 / ws) : 0.f, part, &rows, false,
+                          stream));
+    k_mlp_sum<<<kSumBlocks, dim3(kSumCols, kSumGroups), 0, stream>>>(part, rows, grad, loss);
     GDP_MCUDA(cudaGetLastError());
     GDP_MCUDA(cudaMemcpyAsync(g, grad, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, stream));
     float l = 0.f;
     GDP_MCUDA(cudaMemcpyAsync(&l, loss, sizeof(float), cudaMemcpyDeviceToHost, stream));
     GDP_MCUDA(cudaStreamSynchronize(stream));
     if (lossv) *lossv = l;
-    cudaFree(xb);
-    cudaFree(dy);
-    cudaFree(dw);
     return GDP_OKAY;
 }
 
@@ -473,66 +644,52 @@ GDP_RETCODE Mlp::train(int n, const float *x, const float *y, const float *w, in
         set_error("bad training arguments");
         return GDP_ERROR;
     }
+    GDP_MCUDA(cudaSetDevice(device));
     // one shuffle of the samples; epochs walk contiguous minibatches from a
-    // rotating start
+    // rotating start. The samples go up in their order while the shuffle is
+    // drawn; the gradient kernel reads them through it.
     std::vector<int> perm(n);
+    std::vector<double> wpre(n + 1, 0.0);
+    Arena mem;
+    const Drained drained{stream};
+    __nv_bfloat16 *xb;
+    float *dy, *dw;
+    if (upload(mem, n, x, y, w, &xb, &dy, &dw) != GDP_OKAY) return GDP_ERROR;
     for (int i = 0; i < n; i++) perm[i] = i;
     unsigned long long s = seed;
     for (int i = n - 1; i > 0; i--) std::swap(perm[i], perm[(int)(splitmix(s) % (unsigned long long)(i + 1))]);
-    std::vector<float> xs((size_t)n * kMlpIn), ys(n), wsv(n);
-    std::vector<double> wpre(n + 1, 0.0);
-    for (int i = 0; i < n; i++) {
-        const int k = perm[i];
-        std::memcpy(&xs[(size_t)i * kMlpIn], x + (size_t)k * kMlpIn, sizeof(float) * kMlpIn);
-        ys[i] = y[k];
-        wsv[i] = w[k];
-        wpre[i + 1] = wpre[i] + w[k];
-    }
-    __nv_bfloat16 *xb = nullptr;
-    float *dy = nullptr, *dw = nullptr;
-    if (upload_x(xs.data(), n, &xb, stream) != GDP_OKAY) return GDP_ERROR;
-    GDP_MCUDA(cudaMalloc(&dy, sizeof(float) * n));
-    GDP_MCUDA(cudaMalloc(&dw, sizeof(float) * n));
-    GDP_MCUDA(cudaMemcpyAsync(dy, ys.data(), sizeof(float) * n, cudaMemcpyHostToDevice, stream));
-    GDP_MCUDA(cudaMemcpyAsync(dw, wsv.data(), sizeof(float) * n, cudaMemcpyHostToDevice, stream));
-    const int nb = (n + batch - 1) / batch;
+    const int nb = (n - 1) / batch + 1;
+    int *dperm = (int *)mem.alloc_bytes(sizeof(int) * (size_t)n);
+    float *part = (float *)mem.alloc_bytes(sizeof(float) * kPartLd * (size_t)grad_rows_max());
+    float *d_losses = (float *)mem.alloc_bytes(sizeof(float) * (size_t)nb);
+    if (!dperm || !part || !d_losses) { set_error("device allocation failed (training)"); return GDP_ERROR; }
+    GDP_MCUDA(cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, stream));
+    for (int i = 0; i < n; i++) wpre[i + 1] = wpre[i] + w[perm[i]];
     double last = 0.0;
-    int last_cnt = 0;
     std::vector<float> lh(nb);
-    float *d_losses = nullptr;
-    GDP_MCUDA(cudaMalloc(&d_losses, sizeof(float) * nb));
+    const int step0 = step;
     for (int e = 0; e < epochs; e++) {
-        GDP_MCUDA(cudaMemsetAsync(d_losses, 0, sizeof(float) * nb, stream));
         const int rot = (int)(splitmix(s) % (unsigned long long)nb);
         for (int b = 0; b < nb; b++) {
             const int bi = (b + rot) % nb;
             const int r0 = bi * batch, cnt = std::min(batch, n - r0);
             const double ws = wpre[r0 + cnt] - wpre[r0];
-            GDP_MCUDA(cudaMemsetAsync(grad, 0, sizeof(float) * kMlpParams, stream));
-            k_mlp_grad<<<grad_grid(cnt), kMlpThreads, kGradSmem, stream>>>(
-                dev(), xb + (size_t)r0 * kMlpIn, dy + r0, dw + r0, cnt, ws > 0 ? (float)(1.0 / ws) : 0.f, grad,
-                d_losses + bi);
+            int rows = 0;
+            GDP_MCUDA(launch_grad(dev(), xb, dperm + r0, dy, dw, cnt, ws > 0 ? (float)(1.0 / ws) : 0.f, part, &rows,
+                                  step0 != step, stream));
             step++;
-            k_mlp_adam<<<8, 256, 0, stream>>>(p, m1, m2, grad, step, lr, 0.9f, 0.999f, 1e-8f);
-            k_mlp_cast<<<16, 256, 0, stream>>>(p, w1, w2, w2t, w3);
-            GDP_MCUDA(cudaGetLastError());
-        }
-        if (e == epochs - 1) {
-            GDP_MCUDA(cudaMemcpyAsync(lh.data(), d_losses, sizeof(float) * nb, cudaMemcpyDeviceToHost, stream));
-            GDP_MCUDA(cudaStreamSynchronize(stream));
-            for (int b = 0; b < nb; b++) {
-                const int r0 = b * batch, cnt = std::min(batch, n - r0);
-                last += lh[b] * (wpre[r0 + cnt] - wpre[r0]);
-                last_cnt++;
-            }
+            LaunchNext L(kSumBlocks, dim3(kSumCols, kSumGroups), 0, true, stream);
+            GDP_MCUDA(cudaLaunchKernelEx(&L.cfg, k_mlp_step, (const float *)part, rows, p, m1, m2, step, lr, 0.9f,
+                                         0.999f, 1e-8f, w1, w2, w2t, w3, d_losses + bi));
         }
     }
+    GDP_MCUDA(cudaMemcpyAsync(lh.data(), d_losses, sizeof(float) * (size_t)nb, cudaMemcpyDeviceToHost, stream));
     GDP_MCUDA(cudaStreamSynchronize(stream));
+    for (int b = 0; b < nb; b++) {
+        const int r0 = b * batch, cnt = std::min(batch, n - r0);
+        last += lh[b] * (wpre[r0 + cnt] - wpre[r0]);
+    }
     if (final_loss) *final_loss = wpre[n] > 0 ? (float)(last / wpre[n]) : 0.f;
-    cudaFree(xb);
-    cudaFree(dy);
-    cudaFree(dw);
-    cudaFree(d_losses);
     return GDP_OKAY;
 }
 

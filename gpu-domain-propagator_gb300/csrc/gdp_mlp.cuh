@@ -61,7 +61,7 @@ __host__ __device__ __forceinline__ int frag_index(int n, int k, int kts) {
 // order with kts k-tiles (a warp reads 256 consecutive bytes).
 __device__ __forceinline__ void load_bfrag(const __nv_bfloat16 *Wf, int kts, int nt, int kt, int lane, unsigned &b0,
                                            unsigned &b1) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(Wf) + (nt * kts + kt) * 32 + lane);
+    const uint2 v = reinterpret_cast<const uint2 *>(Wf)[(nt * kts + kt) * 32 + lane];
     b0 = v.x;
     b1 = v.y;
 }
@@ -78,7 +78,7 @@ __device__ __forceinline__ void mlp_forward_tile(const MlpDev &M, const unsigned
     const int t = lane & 3;
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
-        const float bl = __ldg(M.b1 + nt * 8 + 2 * t), bh = __ldg(M.b1 + nt * 8 + 2 * t + 1);
+        const float bl = M.b1[nt * 8 + 2 * t], bh = M.b1[nt * 8 + 2 * t + 1];
         T.a1[nt][0] = bl; T.a1[nt][1] = bh; T.a1[nt][2] = bl; T.a1[nt][3] = bh;
         unsigned b0, b1;
         load_bfrag(M.w1, 1, nt, 0, lane, b0, b1);
@@ -96,7 +96,7 @@ __device__ __forceinline__ void mlp_forward_tile(const MlpDev &M, const unsigned
     }
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
-        const float bl = __ldg(M.b2 + nt * 8 + 2 * t), bh = __ldg(M.b2 + nt * 8 + 2 * t + 1);
+        const float bl = M.b2[nt * 8 + 2 * t], bh = M.b2[nt * 8 + 2 * t + 1];
         T.a2[nt][0] = bl; T.a2[nt][1] = bh; T.a2[nt][2] = bl; T.a2[nt][3] = bh;
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
@@ -119,7 +119,7 @@ __device__ __forceinline__ void mlp_forward_tile(const MlpDev &M, const unsigned
     z0 += __shfl_xor_sync(0xffffffffu, z0, 2);
     z1 += __shfl_xor_sync(0xffffffffu, z1, 1);
     z1 += __shfl_xor_sync(0xffffffffu, z1, 2);
-    const float b3 = __ldg(M.b3);
+    const float b3 = M.b3[0];
     T.z[0] = z0 + b3;
     T.z[1] = z1 + b3;
 }
@@ -136,7 +136,7 @@ __device__ __forceinline__ void mlp_infer_tile(const MlpDev &M, const unsigned (
 #pragma unroll
         for (int half = 0; half < 2; half++) {
             const int nt = 2 * kt + half;
-            const float bl = __ldg(M.b1 + nt * 8 + 2 * t), bh = __ldg(M.b1 + nt * 8 + 2 * t + 1);
+            const float bl = M.b1[nt * 8 + 2 * t], bh = M.b1[nt * 8 + 2 * t + 1];
             float c[4] = {bl, bh, bl, bh};
             unsigned b0, b1;
             load_bfrag(M.w1, 1, nt, 0, lane, b0, b1);
@@ -148,7 +148,7 @@ __device__ __forceinline__ void mlp_infer_tile(const MlpDev &M, const unsigned (
     float s0 = 0.f, s1 = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
-        const float bl = __ldg(M.b2 + nt * 8 + 2 * t), bh = __ldg(M.b2 + nt * 8 + 2 * t + 1);
+        const float bl = M.b2[nt * 8 + 2 * t], bh = M.b2[nt * 8 + 2 * t + 1];
         float c[4] = {bl, bh, bl, bh};
 #pragma unroll
         for (int kt = 0; kt < 4; kt++) {
@@ -166,7 +166,7 @@ __device__ __forceinline__ void mlp_infer_tile(const MlpDev &M, const unsigned (
     s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
     s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
     s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-    const float b3 = __ldg(M.b3);
+    const float b3 = M.b3[0];
     z0 = s0 + b3;
     z1 = s1 + b3;
 }

@@ -18,6 +18,8 @@ constexpr int kOffW3 = kOffB2 + kMlpH;
 constexpr int kOffB3 = kOffW3 + kMlpH;
 constexpr int kMlpParams = kOffB3 + 1;  // 5313
 
+struct Arena;
+
 class Mlp {
 public:
     ~Mlp();
@@ -42,6 +44,8 @@ public:
 
 private:
     GDP_RETCODE refresh_bf16();
+    GDP_RETCODE upload(Arena &mem, int n, const float *x, const float *y, const float *w, __nv_bfloat16 **xb,
+                       float **dy, float **dw);
 };
 
 }  // namespace gdp
