@@ -988,26 +988,39 @@ __device__ __forceinline__ void flush_changed(const DevProblem &P, unsigned long
 // recorded infeasible in this round, a variable whose bounds cross), mark the
 // rows of changed variables for the next round, clear the bitmap.
 // One warp per word of the bitmap: lane l commits variable 32 w + l, then the
-// warp pushes the marks of each changed variable's rows together, 32 per step
-// (a thread walking its word's variables and their rows alone leaves the
-// commit of a round with many changes to a few long serial chains). tid /
-// nthreads: a grid of whole warps.
+// warp pushes the marks of each changed variable's rows together, 32 per step,
+// with the first steps of four variables in flight: what bounds it is the
+// latency of the index entries, most of which come from HBM (2M rows, 72 rounds:
+// 29.88 -> 29.42 ms against one variable after the other; a thread walking its word's variables and their rows alone
+// leaves the commit of a round with many changes to a few long serial chains).
+// tid / nthreads: a grid of whole warps.
 __device__ __forceinline__ void finalize_words(const DevProblem &P, int round, bool push_marks, int tid,
                                                int nthreads) {
     const int lane = tid & 31;
     unsigned long long changed = 0;
+    auto push = [&](int2 e, double dj) {  // e: {pos, acoef}
+        P.mark[e.x] = round + 1;
+        // a split row's slack moves by at most |a| (lb' - lb + ub - ub')
+        if (e.x >= P.n_srows && P.lrow_drift)
+            atomicAdd(P.lrow_drift + (e.x - P.n_srows), __dmul_ru((double)__int_as_float(e.y), dj));
+    };
     if (tid == 0 && *((volatile int *)&P.flags[0].infeasible_row) != INT_MAX) P.flags[0].infeasible = 1;
     for (int w = tid >> 5; w < P.n_chg_words; w += nthreads >> 5) {
         const unsigned bits = __ldcg(P.chg + w);
         if (!bits) continue;  // warp-uniform
         double delta = 0.0;  // upper bound of (lb' - lb) + (ub - ub') of my variable
+        int p0 = 0, p1 = 0;  // its rows
         if ((bits >> lane) & 1u) {
             const int j = w * 32 + lane;
             const double2 b = __ldcg(P.bnd_nxt + j);
             const double2 o = P.bnd[j];
-            delta = (neginf_bits(dbits(o.x)) || posinf_bits(dbits(o.y)))
-                            ? __longlong_as_double(0x7FF0000000000000LL)  // an infinite bound became finite
-                            : __dadd_ru(__dsub_ru(b.x, o.x), __dsub_ru(o.y, b.y));
+            if (push_marks) {
+                p0 = __ldg(P.var_ptr + j);
+                p1 = __ldg(P.var_ptr + j + 1);
+                delta = (neginf_bits(dbits(o.x)) || posinf_bits(dbits(o.y)))
+                                ? __longlong_as_double(0x7FF0000000000000LL)  // an infinite bound became finite
+                                : __dadd_ru(__dsub_ru(b.x, o.x), __dsub_ru(o.y, b.y));
+            }
             P.bnd[j] = b;
             store_bnd32<1>(P, j, b, round);
             if (var_infeasible(b.x, b.y)) {
@@ -1020,18 +1033,26 @@ __device__ __forceinline__ void finalize_words(const DevProblem &P, int round, b
             P.chg[w] = 0u;
             changed += __popc(bits);
         }
-        if (!push_marks) continue;
-        for (unsigned rem = bits; rem; rem &= rem - 1) {
-            const int bit = __ffs(rem) - 1;
-            const int j = w * 32 + bit;
-            const double dj = __shfl_sync(kFull, delta, bit);
-            for (int p = __ldg(P.var_ptr + j) + lane; p < __ldg(P.var_ptr + j + 1); p += 32) {
-                const int2 e = __ldg(reinterpret_cast<const int2 *>(P.var_ent) + p);  // {pos, acoef}
-                const int pos = e.x;
-                P.mark[pos] = round + 1;
-                // a split row's slack moves by at most |a| (lb' - lb + ub - ub')
-                if (pos >= P.n_srows && P.lrow_drift)
-                    atomicAdd(P.lrow_drift + (pos - P.n_srows), __dmul_ru((double)__int_as_float(e.y), dj));
+        constexpr int kVars = 4;
+        for (unsigned rem = __ballot_sync(kFull, p0 < p1); rem;) {
+            int q[kVars], q1[kVars];
+            double dj[kVars];
+            int2 e[kVars];
+#pragma unroll
+            for (int i = 0; i < kVars; i++) {
+                const int bit = rem ? __ffs(rem) - 1 : 0;
+                q[i] = __shfl_sync(kFull, p0, bit) + lane;
+                q1[i] = __shfl_sync(kFull, p1, bit);
+                dj[i] = __shfl_sync(kFull, delta, bit);
+                if (!rem) q1[i] = 0;
+                rem &= rem - 1;
+                if (q[i] < q1[i]) e[i] = __ldg(reinterpret_cast<const int2 *>(P.var_ent) + q[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < kVars; i++) {
+                if (q[i] < q1[i]) push(e[i], dj[i]);
+                for (int p = q[i] + 32; p < q1[i]; p += 32)
+                    push(__ldg(reinterpret_cast<const int2 *>(P.var_ent) + p), dj[i]);
             }
         }
     }
