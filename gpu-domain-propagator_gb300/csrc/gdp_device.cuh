@@ -24,14 +24,44 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
 
+// ---- integer-domain forms (no FP64 pipe) ----------------------------------
+// A double's bit pattern orders like a signed integer when the sign bit is 0,
+// and in reverse as an unsigned integer when it is 1. A compare of doubles is an
+// FP64 instruction like any other (72 cycles a warp); these are not.
+constexpr long long kBitsEps = 0x3E112E0BE826D695LL;          // 1e-9
+constexpr long long kBitsPosInf = 0x4415AF1D78B58C40LL;       // 1e20
+constexpr unsigned long long kBitsNegInf = 0xC415AF1D78B58C40ULL;  // -1e20
+constexpr long long kBitsIeeeInf = 0x7FF0000000000000LL;
+
+__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+// key(x) < key(y) iff x < y for non-NaN doubles of different value (NaN keys
+// lie above +inf's and below -inf's; -0.0 below +0.0)
+__device__ __forceinline__ long long order_key(long long b) {
+    return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
+}
+__device__ __forceinline__ bool nan_bits(long long b) { return (b & 0x7FFFFFFFFFFFFFFFLL) > kBitsIeeeInf; }
+// v > c and v <= c for c > 0 given by its bits (false for a NaN)
+__device__ __forceinline__ bool gt_bits(double v, long long c) { return dbits(v) > c && dbits(v) <= kBitsIeeeInf; }
+__device__ __forceinline__ bool le_bits(double v, long long c) { return dbits(v) <= c && !nan_bits(dbits(v)); }
+
 // reference src/def.h:68-79
-__device__ __forceinline__ bool eps_gt(double x, double y) { return dsub(x, y) > kEps; }
-__device__ __forceinline__ bool eps_lt(double x, double y) { return dsub(x, y) < -kEps; }
-__device__ __forceinline__ bool eps_le(double x, double y) { return dsub(x, y) <= kEps; }
+__device__ __forceinline__ bool eps_gt(double x, double y) { return gt_bits(dsub(x, y), kBitsEps); }
+__device__ __forceinline__ bool eps_le(double x, double y) { return le_bits(dsub(x, y), kBitsEps); }
 __device__ __forceinline__ bool is_posinf(double x) { return x >= kInf; }
 __device__ __forceinline__ bool is_neginf(double x) { return x <= -kInf; }
-__device__ __forceinline__ double eps_floor(double x) { return floor(dadd(x, kEps)); }
-__device__ __forceinline__ double eps_ceil(double x) { return ceil(dsub(x, kEps)); }
+// The tightened bound's value and whether it is EPS-better than `old`: floor(nb
+// + EPS) for an upper bound, ceil(nb - EPS) for a lower one (is_int), then nb <
+// old - EPS or nb > old + EPS. Both sides take the same three instructions:
+// ceil(x) = -floor(-x), signs by bits.
+__device__ __forceinline__ double flip_sign(double x, bool on) {
+    return __longlong_as_double(dbits(x) ^ (on ? (long long)(1ULL << 63) : 0LL));
+}
+__device__ __forceinline__ double eps_round(double nb, bool lower) {
+    return flip_sign(floor(flip_sign(dadd(nb, lower ? -kEps : kEps), lower)), lower);
+}
+__device__ __forceinline__ bool eps_better(double nb, double old, bool lower) {
+    return gt_bits(flip_sign(dsub(nb, old), !lower), kBitsEps);
+}
 
 // FP64 max / min as one integer atomic each: for sign bit 0 the bit pattern
 // orders like a signed integer; for sign bit 1 it orders in reverse as an
@@ -47,15 +77,6 @@ __device__ __forceinline__ void atomic_min_f64(double *addr, double v) {
     else atomicMax(reinterpret_cast<unsigned long long *>(addr), static_cast<unsigned long long>(b));
 }
 
-// ---- integer-domain forms (no FP64 pipe) ----------------------------------
-// Exact for every non-NaN double: a double's bit pattern orders like a signed
-// integer when the sign bit is 0, and in reverse as an unsigned integer when
-// it is 1.
-constexpr long long kBitsEps = 0x3E112E0BE826D695LL;          // 1e-9
-constexpr long long kBitsPosInf = 0x4415AF1D78B58C40LL;       // 1e20
-constexpr unsigned long long kBitsNegInf = 0xC415AF1D78B58C40ULL;  // -1e20
-
-__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 // x > 1e-9 (the reference's EPSGT(x, 0))
 __device__ __forceinline__ bool gt_eps_bits(long long b) { return b > kBitsEps; }
 // x > 0
@@ -64,10 +85,6 @@ __device__ __forceinline__ bool gt0_bits(long long b) { return b > 0; }
 __device__ __forceinline__ bool neginf_bits(long long b) { return (unsigned long long)b >= kBitsNegInf; }
 // x >= 1e20 (ISPOSINF)
 __device__ __forceinline__ bool posinf_bits(long long b) { return b >= kBitsPosInf; }
-// key(x) < key(y) iff x < y for non-NaN doubles (NaN keys sort above +inf)
-__device__ __forceinline__ long long order_key(long long b) {
-    return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
-}
 // EPSGT(x, y) with the FP64 subtraction only when x > y.
 __device__ __forceinline__ bool eps_gt_fast(double x, double y) {
     return order_key(dbits(x)) > order_key(dbits(y)) && eps_gt(x, y);
@@ -161,16 +178,16 @@ __device__ __forceinline__ void acc_combine(Acc &a, const Acc &b) {
 // below 2 EPS). m >= 1e20 exactly when M >= 1e20 (doubles near 1e20 are 16384
 // apart). So, with v = fl(M - mn):
 //   v <= EPS                      -> fl(m - mn) <= v: the reference skips;
-//   v > kGoClear (2.00001e-9)     -> m - mn > 1.00001e-9: it processes the row;
+//   v > 2.00001e-9                -> m - mn > 1.00001e-9: it processes the row;
 //   in between                    -> only m itself decides (seq_eps_max).
 // Returns 0 (skip), 1 (process) or 2 (undecided: compute m).
-constexpr double kGoClear = 2.00001e-9;
+constexpr long long kBitsGoClear = 0x3E212E11894DB83DLL;  // 2.00001e-9
 __device__ __forceinline__ int row_go_from_max(int minf, int maxf, double M, double mn) {
     if (minf > 1 && maxf > 1) return 0;
-    if (M >= kInf) return 1;
+    if (posinf_bits(dbits(M))) return 1;  // M is no NaN
     const double v = dsub(M, mn);
-    if (v <= kEps) return 0;
-    return (v > kGoClear || v != v) ? 1 : 2;  // NaN: the reference's !EPSLE(m, NaN) holds
+    if (le_bits(v, kBitsEps)) return 0;
+    return (gt_bits(v, kBitsGoClear) || nan_bits(dbits(v))) ? 1 : 2;  // NaN: the reference's !EPSLE(m, NaN) holds
 }
 
 // Row-side infeasibility: the reference's isConsInfeasible

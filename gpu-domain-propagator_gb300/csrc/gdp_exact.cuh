@@ -126,8 +126,8 @@ __device__ __forceinline__ void exact_drain(const T &t, ExactSmem &xs, ExactQueu
             const bool lower = q.code & 1u;
             double nb = ddiv(q.num, a);
             if (q.code & 2u) nb = dadd(nb, lower ? b.y : b.x);
-            if (!t.cont(j)) nb = lower ? eps_ceil(nb) : eps_floor(nb);
-            if (lower ? eps_gt(nb, b.x) : eps_lt(nb, b.y)) {
+            if (!t.cont(j)) nb = eps_round(nb, lower);
+            if (eps_better(nb, lower ? b.x : b.y, lower)) {
                 t.apply(j, nb, lower);
                 Q.tight++;
                 if (row_tight) atomicAdd(row_tight + (q.code >> 2), 1);
@@ -383,7 +383,8 @@ __device__ __forceinline__ int exact_decide(const ExactRow &R, const ExactSums &
                                             bool &bad) {
     s = dsub(R.rhs, S.minact);
     t = dsub(S.maxact, R.lhs);
-    mn = (t < s) ? t : s;
+    const long long ks = order_key(dbits(s)), kt = order_key(dbits(t));
+    mn = kt < ks && !nan_bits(dbits(s)) && !nan_bits(dbits(t)) ? t : s;  // t < s ? t : s
     // a row with both slacks >= 0 is feasible
     bad = (dbits(s) < 0 || dbits(t) < 0) && row_infeasible(S.minact, S.maxact, R.minf, R.maxf, R.lhs, R.rhs);
     return row_go_from_max(R.minf, R.maxf, __longlong_as_double(S.km), mn);
