@@ -154,14 +154,8 @@ __device__ __forceinline__ bool sell_slice_learned(const DevProblem &P, int slic
     Scr c;
     scr_init(c);
     {
-        const int *col = P.sell_col + base;
-        const float *val = P.sell_a32 + base;
-#pragma unroll 4
-        for (int i = 0; i < cnt; i++) {
-            const int j = __ldcs(col + 32 * i);
-            const float a = __ldcs(val + 32 * i);
-            scr_add(c, a, load_bnd32<kRec>(P, j));
-        }
+        int chg = 0;
+        screen_elements<kRec, 32>(P, P.sell_col + base, P.sell_a32 + base, cnt, round, c, chg);
     }
     if (g > 1) scr_group_reduce(c, g);
     bool exact = false;
