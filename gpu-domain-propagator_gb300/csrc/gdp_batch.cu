@@ -270,12 +270,10 @@ namespace {
 // round r in flags[1 + (r & 1)].kind; a slice whose marked rows the model
 // deferred is queued again for the next round, and a unit ends only with a FULL
 // round that changes nothing, exactly as in its single-problem learned run.
-// Both instantiations run 5 CTAs per SM (48 registers, spills served by L1):
-// the round work is latency-bound, and on 128 chain instances the learned
-// loop took 2,093 / 912 / 866 / 844 / 1,269 ms at 2 / 3 / 4 / 5 / 6 CTAs per
-// SM, the plain one 590 / 567 / 561 / 566 ms at 3 / 4 / 5 / 6.
-template <bool kLearned>
-__global__ void __launch_bounds__(kCtaThreads, 3) k_batch_loop(BatchDev B) {
+// kCtas per SM: 3 (80 registers), or 2 (128) for batches with little work in a
+// round (Batch::size_grid).
+template <bool kLearned, int kCtas>
+__global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
     WarpSmem *ws = warp_smem();
     __shared__ LearnSmem ls[kLearned ? kWarpsPerCta : 1];
     const int lane = threadIdx.x & 31;
@@ -572,8 +570,15 @@ __global__ void __launch_bounds__(256) k_batch_fini(BatchDev B, double *lb, doub
 }  // namespace
 
 // ---- launchers --------------------------------------------------------------
-int batch_occupancy(int *blocks_per_sm, bool learned) {
-    const void *k = learned ? (const void *)k_batch_loop<true> : (const void *)k_batch_loop<false>;
+namespace {
+const void *batch_loop(bool learned, bool little) {
+    if (learned) return (const void *)k_batch_loop<true, 3>;
+    return little ? (const void *)k_batch_loop<false, 2> : (const void *)k_batch_loop<false, 3>;
+}
+}  // namespace
+
+int batch_occupancy(int *blocks_per_sm, bool learned, bool little) {
+    const void *k = batch_loop(learned, little);
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaSmem);
     if (e != cudaSuccess) return (int)e;
     return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, kCtaThreads, kCtaSmem);
@@ -581,7 +586,7 @@ int batch_occupancy(int *blocks_per_sm, bool learned) {
 
 int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub, double *lb_out,
                  double *ub_out, const long long *var_base, int max_unit_n, const double2 *ref,
-                 const int *seed_mode, bool learned, cudaStream_t s) {
+                 const int *seed_mode, bool learned, bool little, cudaStream_t s) {
     const dim3 vgrid((unsigned)std::max(1, std::min((max_unit_n + 255) / 256, 64)), (unsigned)B.n_units);
     k_batch_init<<<vgrid, 256, 0, s>>>(B, lb, ub, var_base);
     cudaError_t e = cudaGetLastError();
@@ -594,8 +599,7 @@ int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
     BatchDev Bc = B;
     void *args[] = {&Bc};
-    e = cudaLaunchCooperativeKernel(learned ? (const void *)k_batch_loop<true> : (const void *)k_batch_loop<false>,
-                                    dim3(grid), dim3(kCtaThreads), args, kCtaSmem, s);
+    e = cudaLaunchCooperativeKernel(batch_loop(learned, little), dim3(grid), dim3(kCtaThreads), args, kCtaSmem, s);
     if (e != cudaSuccess) return (int)e;
     k_batch_fini<<<vgrid, 256, 0, s>>>(B, lb_out, ub_out, var_base);
     return (int)cudaGetLastError();

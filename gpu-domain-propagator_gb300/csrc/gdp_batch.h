@@ -34,8 +34,8 @@ struct BatchDev {
 
 int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub, double *lb_out,
                  double *ub_out, const long long *var_base, int max_unit_n, const double2 *ref,
-                 const int *seed_mode, bool learned, cudaStream_t s);
-int batch_occupancy(int *blocks_per_sm, bool learned);
+                 const int *seed_mode, bool learned, bool little, cudaStream_t s);
+int batch_occupancy(int *blocks_per_sm, bool learned, bool little);
 
 class Batch {
 public:
@@ -60,6 +60,7 @@ public:
     bool use_graph = true;   // capture the device part once and replay it
     bool graph_ok = false;   // the graph was captured and is used
     int grid = 1;
+    bool little_ = false;  // little work in a round
     int max_rounds = GDP_MAX_NUM_ROUNDS;
 
 private:

@@ -11,11 +11,14 @@ namespace gdp {
 
 namespace {
 
-// Shared memory of 24 warps (and 1 KB the system keeps per CTA) as a share of
+// Shared memory of 16 warps (and 1 KB the system keeps per CTA) as a share of
 // the 228 KB per SM, in percent.
-constexpr int kCarveout = (int)((24 * sizeof(WarpSmem) + 6 * 1024) * 100 / (228 * 1024) + 1);
+constexpr int kCarveout = (int)((16 * sizeof(WarpSmem) + 6 * 1024) * 100 / (228 * 1024) + 1);
 
 // ---- phase kernels (GPU_LOOP) -----------------------------------
+// The screen alone needs few registers: 32 warps per SM. The exact passes take
+// 16 with 128 registers, as in the megakernel (60,001 rows: 4.9 ms with 4 CTAs of
+// 64 registers for all three, 4.0 with these).
 __global__ void __launch_bounds__(kCtaThreads, 4) k_activity(const __grid_constant__ DevProblem P) {
     WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
@@ -26,7 +29,7 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_activity(const __grid_consta
     stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
-__global__ void __launch_bounds__(kCtaThreads, 4) k_candidates(const __grid_constant__ DevProblem P) {
+__global__ void __launch_bounds__(kCtaThreads, 2) k_candidates(const __grid_constant__ DevProblem P) {
     WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible) return;
@@ -40,7 +43,7 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_candidates(const __grid_cons
     stats_flush(P, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
-__global__ void __launch_bounds__(kCtaThreads, 4) k_exact(const __grid_constant__ DevProblem P) {
+__global__ void __launch_bounds__(kCtaThreads, 2) k_exact(const __grid_constant__ DevProblem P) {
     WarpSmem *ws = warp_smem();
     const int round = P.flags[0].rounds;
     if (P.flags[0].infeasible || P.flags[0].exact == 0) return;
@@ -182,8 +185,11 @@ __device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, 
 // so that nothing a CTA may still read is cleared: the next round's slots are cleared after the current
 // round's first barrier, which every CTA passes only after finishing the
 // previous round.
-// W warps per CTA; with 24 / W resident CTAs per SM every instance holds about
-// 24 warps per SM under the same register budget.
+// W warps per CTA; with 16 / W resident CTAs per SM every instance holds 16
+// warps per SM with 128 registers each. 24 warps with 80 registers spill around
+// the exact pass, and six warps share an SM quarter's FP64 unit instead of four:
+// 60,001 rows 4.29 -> 3.62 ms with 16, 300,000 6.45 -> 6.07, 2,000 0.333 -> 0.314,
+// 2M rows 27.0 either way (12 warps: 3.5, 6.3, 0.31 and 31.5).
 // A launch runs the rounds first .. last, or fewer when one changes nothing or
 // turns infeasible; a launch after that one does nothing (flags[0].done), so
 // that a host loop may queue a round before it knows whether the round is
@@ -196,7 +202,7 @@ __device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, 
 // 0.42 ms). With wide rows in the problem their items would follow one another
 // on one warp (2,000 power-law rows: 1.86 -> 2.34 ms), and they are deferred.
 template <int W, bool kInPlace>
-__global__ void __launch_bounds__(32 * W, 24 / W) k_megakernel(const __grid_constant__ DevProblem P, int first,
+__global__ void __launch_bounds__(32 * W, 16 / W) k_megakernel(const __grid_constant__ DevProblem P, int first,
                                                                int last, int *mail) {
     WarpSmem *ws = warp_smem();
     const int lane = threadIdx.x & 31;
@@ -365,7 +371,7 @@ int phase_occupancy(int *act, int *cand, int *mega, int cta_warps, bool in_place
     cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mega_smem);
     for (const void *k : {(const void *)k_activity, (const void *)k_candidates, (const void *)k_exact})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaSmem);
-    // a carveout that just holds 24 warps' shared memory, the rest of the
+    // a carveout that just holds 16 warps' shared memory, the rest of the
     // 256 KB per SM serving as L1 for the element streams
     if (e == cudaSuccess) e = cudaFuncSetAttribute(mk, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout);
     if (e != cudaSuccess) return (int)e;
