@@ -583,7 +583,6 @@ __device__ __forceinline__ void sell_slice(const DevProblem &P, int slice, int l
 // only 64..128 non-zeros: alone, its chain of dependent loads leaves the warp
 // waiting), and the exact rows of all K slices are queued with one counter
 // update. Decisions and queue contents equal those of K sell_slice calls.
-constexpr int kScreenGroup = 2;
 template <int K, int kRec>
 __device__ __forceinline__ void sell_slices_g1(const DevProblem &P, const int (&sl)[K], int lane, int round,
                                                bool marked, WarpSmem &ws, int par) {
@@ -1110,40 +1109,46 @@ __device__ __forceinline__ void activity_item(const DevProblem &P, int it, int l
     else split_partial<1>(P, -it - 1, lane, round, marked, change, tight_ctr, ws);
 }
 
-// Items are claimed kScreenGroup at a time when there are several claims per
-// warp (one at a time otherwise: two items on one warp are twice its latency);
-// a claim of one-lane-row slices (the light end of the heaviest-first order) is
-// screened as a group, other claims item by item.
+// Items are claimed one, two or three at a time: from 8 items per warp on in
+// pairs, from 32 on in threes (two items on one warp are twice its latency, but
+// the light end of the heaviest-first order, slices of one-lane rows, is screened
+// as a group with all its loads in flight). One at a time against pairs, 300,000
+// rows (6.6 items per warp): 5.6 against 6.1 ms; 600,000 (13): 10.4 against 10.2;
+// pairs against threes, 1M rows (22): 15.6 and 15.6; 2M rows (44): 27.4 against
+// 26.8. Other claims run item by item.
+template <int K>
+__device__ __forceinline__ bool screen_group(const DevProblem &P, const int (&it)[3], int lane, int round, bool marked,
+                                             WarpSmem &ws, int par) {
+    int sl[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (it[k] < 0 || __ldg(P.slice_lg + it[k]) != 0) return false;
+        sl[k] = it[k];
+    }
+    sell_slices_g1<K, 1>(P, sl, lane, round, marked, ws, par);
+    return true;
+}
 template <bool kDefer>
 __device__ __forceinline__ void activity_phase(const DevProblem &P, int round, bool marked, unsigned *ctr,
                                                int *change, unsigned *tight_ctr, WarpSmem &ws, int lane,
                                                int par = 0) {
-    constexpr int K = kScreenGroup;
     const int nw = grid_warps();
-    const int take = P.n_items >= 2 * K * nw ? K : 1;  // items of a claim
+    const int take = P.n_items >= 32 * nw ? 3 : P.n_items >= 8 * nw ? 2 : 1;  // items of a claim
     WarpCursor<true> cur;
     cur.start(ctr, take, nw, P.n_items);
     for (;;) {
         const int i = cur.next(lane);
         if (i >= P.n_items) break;
-        int it[K];
-        bool group = kDefer && take == K && i + K <= P.n_items;
+        int it[3];
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            it[k] = i + k < P.n_items ? __ldg(P.items + i + k) : -1;
-            group = group && it[k] >= 0;
+        for (int k = 0; k < 3; k++) it[k] = k < take && i + k < P.n_items ? __ldg(P.items + i + k) : -1;
+        if (kDefer && i + take <= P.n_items) {
+            if (take == 3 && screen_group<3>(P, it, lane, round, marked, ws, par)) continue;
+            if (take == 2 && screen_group<2>(P, it, lane, round, marked, ws, par)) continue;
         }
-        if (group) {
-#pragma unroll
-            for (int k = 0; k < K; k++) group = group && __ldg(P.slice_lg + it[k]) == 0;
-        }
-        if (group) {
-            sell_slices_g1<K, 1>(P, it, lane, round, marked, ws, par);
-        } else {
 #pragma unroll 1
-            for (int k = 0; k < take && i + k < P.n_items; k++)
-                activity_item<kDefer>(P, it[k], lane, round, marked, change, tight_ctr, ws, par);
-        }
+        for (int k = 0; k < take && i + k < P.n_items; k++)
+            activity_item<kDefer>(P, it[k], lane, round, marked, change, tight_ctr, ws, par);
     }
 }
 
