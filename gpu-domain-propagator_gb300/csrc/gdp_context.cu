@@ -954,9 +954,11 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     if (cta_threads == 0) cta_threads = one_cta ? 512 : 256;
     const int warps = cta_threads / 32;
     int act_bps = 0, cand_bps = 0, mega_bps = 0;
-    // one-lane rows alone, and a warp for each slice (24 warps per SM, fewer
-    // with a limit): the exact pass in place
-    P.in_place = one_lane && P.n_items <= n_sms * (ctas_per_sm > 0 ? std::min(24, ctas_per_sm * warps) : 24);
+    // one-lane rows alone, and at most three slices per warp (16 warps per SM, fewer
+    // with a limit): the exact pass in place. Megakernel, 130,000 rows of 2 to 16:
+    // 0.86 ms in place, 1.04 queued; 200,000 0.99 and 1.06; 300,000 1.34 and 1.345;
+    // 600,000 2.21 and 2.04
+    P.in_place = one_lane && P.n_items <= n_sms * 3 * (ctas_per_sm > 0 ? std::min(16, ctas_per_sm * warps) : 16);
     GDP_CUDA(phase_occupancy(&act_bps, &cand_bps, &mega_bps, warps, P.in_place != 0));
     if (ctas_per_sm > 0) {
         act_bps = std::min(act_bps, ctas_per_sm);

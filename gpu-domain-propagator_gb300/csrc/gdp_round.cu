@@ -196,11 +196,11 @@ __device__ __forceinline__ void timer_busy(const DevProblem &, WarpSmem &, int, 
 // needed. Between launches barrier[1] keeps the barrier count and the round's
 // tightenings the next round's mode. mail (may be null): host memory that
 // receives {the round, whether another one follows}.
-// kInPlace (P.in_place): a small problem of one-lane rows only, with a warp for
-// each slice: the screen's warp takes its rows through the exact pass at once,
-// which saves the queue, a phase and a barrier (2,000 rows of 2 to 16: 0.50 ->
-// 0.42 ms). With wide rows in the problem their items would follow one another
-// on one warp (2,000 power-law rows: 1.86 -> 2.34 ms), and they are deferred.
+// kInPlace (P.in_place): a problem of one-lane rows only, with at most three slices
+// per warp: the screen's warp takes its rows through the exact pass at once,
+// which saves the queue, a phase and a barrier. With wide rows in the problem their
+// items would follow one another on one warp (2,000 power-law rows: 1.86 -> 2.34
+// ms), and they are deferred.
 template <int W, bool kInPlace>
 __global__ void __launch_bounds__(32 * W, 16 / W) k_megakernel(const __grid_constant__ DevProblem P, int first,
                                                                int last, int *mail) {
