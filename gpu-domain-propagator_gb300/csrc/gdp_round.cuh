@@ -327,10 +327,10 @@ struct WarpCursor {
     int step, first, base;
     bool more;      // the grid's first claims do not cover the items
     unsigned pre;   // kAhead, lane 0: the claim in flight
-    __device__ __forceinline__ void start(unsigned *c, int stp, int warps, int n) {
+    __device__ __forceinline__ void start(unsigned *c, int stp, int warps, int n, bool from_last = false) {
         ctr = c;
         step = stp;
-        first = grid_warp_striped() * stp;
+        first = (from_last ? warps - 1 - grid_warp_striped() : grid_warp_striped()) * stp;
         base = warps * stp;
         more = n > base;
         pre = 0;
@@ -683,9 +683,14 @@ __device__ __forceinline__ void sell_slices_g1(const DevProblem &P, const int (&
 // Exact-rows phase: the rows the screen queued, in items of 32 / g rows per
 // warp, or of fewer rows with more lanes per chain (up to 8: a row's sums then
 // take a quarter of the FP64 instructions) as long as the grid has a warp for
-// each item. The items of all classes are one list, widest class first; warp w
-// takes item w and claims further ones from a counter only when there are more
-// items than warps.
+// each item. The items of all classes are one list, widest class first; a warp
+// takes one by its own number and claims further ones from a counter only when
+// there are more items than warps. The first warps come from the tiles of the
+// candidate phase: with tiles for up to half of the warps the widest items go to
+// the last ones (the same warps had the tiles and the widest items before: 5,000
+// rows 1.45 -> 1.35 ms, 20,000 rows 2.28 -> 2.10, 60,001 rows 3.57 -> 3.52); with
+// tiles for all of them the order is a coin toss (150,000 rows 4.08, 4.24 from the
+// last).
 __device__ __forceinline__ void exact_rows_phase(const DevProblem &P, int par, int *change, unsigned *tight_ctr,
                                                  WarpSmem &ws, int lane) {
     const int nw = grid_warps();
@@ -707,7 +712,7 @@ __device__ __forceinline__ void exact_rows_phase(const DevProblem &P, int par, i
     const CtxTarget T = sell_target(P);
     ExactQueue Q{0, 0, 0};
     WarpCursor<false> cur;
-    cur.start(P.xctr + 16 * par + 8, 1, nw, total);
+    cur.start(P.xctr + 16 * par + 8, 1, nw, total, 2 * P.n_mtiles <= nw);
     for (;;) {
         const int it = cur.next(lane);
         if (it >= total) break;
