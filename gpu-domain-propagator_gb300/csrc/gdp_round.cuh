@@ -987,6 +987,7 @@ __device__ __forceinline__ bool split_cand(const DevProblem &P, int t, int lane,
     return true;
 }
 
+constexpr int kTileParts = 4;  // candidates of a tile in quarters: a long tile is no phase's long pole
 // Exact phase, tile t of a multi-tile row flagged this round: the row's exact
 // partials combined in tile order, then the decision and this tile's candidates.
 template <int kRec>
@@ -1186,21 +1187,20 @@ __device__ __forceinline__ void candidate_phase(const DevProblem &P, int round, 
 // phase's long pole while the rest of the grid waited at its barrier.
 __device__ __forceinline__ void exact_phase(const DevProblem &P, int round, int *change, unsigned *tight_ctr,
                                             WarpSmem &ws, int lane) {
-    constexpr int kParts = 4;  // candidates of a tile in quarters: a long tile is no phase's long pole
     const int nw = grid_warps();
-    const int n_items = P.n_mtiles * kParts;
+    const int n_items = P.n_mtiles * kTileParts;
     for (int i0 = grid_warp_striped(); i0 < n_items; i0 += 32 * nw) {
         const int i = i0 + lane * nw;
         int t = 0;
         bool live = false;
         if (i < n_items) {
-            t = __ldg(P.mtiles + i / kParts);
+            t = __ldg(P.mtiles + i / kTileParts);
             live = P.row_exact[__ldg(P.tile_row + t)] == round;
         }
         for (unsigned bal = __ballot_sync(kFull, live); bal; bal &= bal - 1) {
             const int src = __ffs(bal) - 1;
             split_exact<1>(P, __shfl_sync(kFull, t, src), lane, round, change, tight_ctr, ws,
-                           (i0 + src * nw) % kParts, kParts);
+                           (i0 + src * nw) % kTileParts, kTileParts);
         }
     }
 }
