@@ -165,6 +165,7 @@ struct DevProblem {
     // Class lg's queue is xrow[cls_begin[lg] .. cls_end[lg]) (its row positions
     // are exactly that range, slices being sorted by g).
     int in_place;          // the screen's warp runs its rows' exact pass (the round loop's choice)
+    int parts;             // in place: warps that screen a slice, each running a share of its exact rows
     int cls_begin[6], cls_end[6];
     XRow *xrow;            // n_srows
     unsigned *xctr;        // [parity * 16 + lg]: queue tails, [parity * 16 + 8]: claimed items

@@ -523,7 +523,8 @@ __device__ __forceinline__ int pack_inf(const Scr &c) { return min(c.minf, 3) | 
 // with a warp for each slice of nothing but one-lane rows).
 template <int kRec, bool kDefer>
 __device__ __forceinline__ void sell_slice(const DevProblem &P, int slice, int lane, int round, bool marked,
-                                           int *change, unsigned *tight_ctr, WarpSmem &ws, int par = 0) {
+                                           int *change, unsigned *tight_ctr, WarpSmem &ws, int par = 0, int part = 0,
+                                           int parts = 1) {
     const int lg = __ldg(P.slice_lg + slice);
     const int g = 1 << lg;
     const int row0 = __ldg(P.slice_row0 + slice);
@@ -564,7 +565,12 @@ __device__ __forceinline__ void sell_slice(const DevProblem &P, int slice, int l
             }
         }
     }
-    count_work(ws, lane, leader ? 1 : 0, leader ? len : 0, (leader && exact) ? len : 0);
+    if (!kDefer && parts > 1) {  // my share of the exact rows
+        const unsigned rows = __ballot_sync(kFull, exact);
+        exact = exact && __popc(rows & ((1u << lane) - 1u)) % parts == part;
+    }
+    const bool counted = leader && part == 0;
+    count_work(ws, lane, counted ? 1 : 0, counted ? len : 0, (leader && exact) ? len : 0);
     if (kDefer) {
         const unsigned bal = __ballot_sync(kFull, exact);
         if (!bal) return;
@@ -1110,8 +1116,9 @@ __device__ __forceinline__ void finalize_words(const DevProblem &P, int round, b
 // ---- work distribution ----------------------------------------------------
 template <bool kDefer>
 __device__ __forceinline__ void activity_item(const DevProblem &P, int it, int lane, int round, bool marked,
-                                              int *change, unsigned *tight_ctr, WarpSmem &ws, int par) {
-    if (it >= 0) sell_slice<1, kDefer>(P, it, lane, round, marked, change, tight_ctr, ws, par);
+                                              int *change, unsigned *tight_ctr, WarpSmem &ws, int par, int part = 0,
+                                              int parts = 1) {
+    if (it >= 0) sell_slice<1, kDefer>(P, it, lane, round, marked, change, tight_ctr, ws, par, part, parts);
     else split_partial<1>(P, -it - 1, lane, round, marked, change, tight_ctr, ws);
 }
 
@@ -1139,6 +1146,13 @@ __device__ __forceinline__ void activity_phase(const DevProblem &P, int round, b
                                                int *change, unsigned *tight_ctr, WarpSmem &ws, int lane,
                                                int par = 0) {
     const int nw = grid_warps();
+    if (!kDefer && P.parts > 1) {  // a warp for each part of each slice
+        const int i = grid_warp_striped();
+        if (i < P.n_items * P.parts)
+            activity_item<kDefer>(P, __ldg(P.items + i / P.parts), lane, round, marked, change, tight_ctr, ws, par,
+                                  i % P.parts, P.parts);
+        return;
+    }
     const int take = P.n_items >= 32 * nw ? 3 : P.n_items >= 8 * nw ? 2 : 1;  // items of a claim
     WarpCursor<true> cur;
     cur.start(ctr, take, nw, P.n_items);
