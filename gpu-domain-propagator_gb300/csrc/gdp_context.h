@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <initializer_list>
 #include <string>
 #include <vector>
@@ -113,7 +114,8 @@ private:
     GDP_RETCODE run(const double *lb_in, const double *ub_in, double *lb_out, double *ub_out,
                     cudaStream_t s, gdp_stats *st);
     GDP_RETCODE build_graph(cudaStream_t s);
-    GDP_RETCODE rounds_cpu_loop(cudaStream_t s, int *launches);
+    // meanwhile: host work to do once the first rounds are queued
+    GDP_RETCODE rounds_cpu_loop(cudaStream_t s, int *launches, const std::function<void()> &meanwhile);
     GDP_RETCODE rounds_gpu_loop(cudaStream_t s);
     void copy_bounds(const double *lbs_in, const double *ubs_in, double *lbs_out, double *ubs_out) const;
     GDP_RETCODE rounds_megakernel(cudaStream_t s, int *launches);
