@@ -18,6 +18,9 @@
 // memory, a CTA writes the sum over its warps to its row of a partial array, and
 // the optimizer step (or the gradient call) adds up the rows: no atomics, and
 // every sum in a fixed order, so equal calls give equal bits.
+#include <omp.h>
+
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -76,9 +79,9 @@ __device__ __forceinline__ void load_samples(const __nv_bfloat16 *X, const int *
 // reaches directly: the features are read once, where they are, 1 KB per warp
 // and tile in whole lines with the next tile in flight, rounded to BF16 on the
 // way and passed to the fragment layout through shared memory; a copy to the
-// device, a conversion pass and a copy back are left out. What bounds it is
-// the rate of those reads (1M rows, 64 MB: 0.40 ms, 170 GB/s
-// over NVLink-C2C, against 0.93 ms with the copies).
+// device and a conversion pass are left out. What bounds it is
+// the rate of those reads over NVLink-C2C (1M rows, 64 MB: 0.41 ms, 165 GB/s,
+// against 0.93 ms with the copies).
 __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(MlpDev M, const float *__restrict__ X, int n, float *z) {
     __shared__ __align__(16) __nv_bfloat16 tile[kMlpWarps][16][kMlpIn];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -400,6 +403,10 @@ __global__ void k_mlp_cast(const float *p, __nv_bfloat16 *w1, __nv_bfloat16 *w2,
         cast_param(i, p[i], w1, w2, w2t, w3);
 }
 
+__global__ void k_copy(const float *x, float *y, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = x[i];
+}
+
 __global__ void k_to_bf16(const float *x, __nv_bfloat16 *y, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         y[i] = __float2bfloat16_rn(x[i]);
@@ -589,26 +596,47 @@ GDP_RETCODE Mlp::upload(Arena &mem, int n, const float *x, const float *y, const
     return GDP_OKAY;
 }
 
+// Host threads that touch `pages` pages.
+static int omp_threads(long long pages) {
+    return (int)std::max(1LL, std::min<long long>(pages >> 8, omp_get_max_threads() - 1));
+}
+
 GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     if (n < 0 || (n && (!x || !z))) { set_error("bad forward arguments"); return GDP_ERROR; }
     if (!n) return GDP_OKAY;
     GDP_MCUDA(cudaSetDevice(device));
     // 16-byte loads need an aligned array (numpy's are); another one is copied
     const bool direct = host_direct && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+    const size_t xb = sizeof(float) * (size_t)n * kMlpIn, zb = sizeof(float) * (size_t)n;
+    // The logits of a small call go straight to host memory. The GPU's first write
+    // to a page that nothing has touched yet is a fault of many microseconds, so
+    // those of a large one (a new array of that size has new pages) go to device
+    // memory, and the host touches the pages while the kernel runs (2M rows into a
+    // new array: 3.6 ms written directly, 0.77 so, 1.9 with every copy; into one
+    // that was written before: 0.79, 0.81).
+    constexpr size_t kDirectBytes = 64 << 10;
     Arena tmp;
+    const Drained drained{stream};
     const float *dx = x;
     float *dz = z;
     if (!direct) {
-        const size_t xb = sizeof(float) * (size_t)n * kMlpIn;
         float *up = (float *)tmp.alloc_bytes(xb);
-        dz = (float *)tmp.alloc_bytes(sizeof(float) * (size_t)n);
-        if (!up || !dz) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
+        if (!up) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
         GDP_MCUDA(cudaMemcpyAsync(up, x, xb, cudaMemcpyHostToDevice, stream));
         dx = up;
     }
+    if (!direct || zb > kDirectBytes) dz = (float *)tmp.alloc_bytes(zb);
+    if (!dz) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
     k_mlp_forward<<<forward_grid(n), kMlpThreads, 0, stream>>>(dev(), dx, n, dz);
     GDP_MCUDA(cudaGetLastError());
-    if (!direct) GDP_MCUDA(cudaMemcpyAsync(z, dz, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, stream));
+    if (dz != z) {
+        const long long pages = (long long)((zb + 4095) / 4096);
+#pragma omp parallel for schedule(static) num_threads(omp_threads(pages))
+        for (long long i = 0; i < pages; i++) *((volatile char *)z + 4096 * i) = 0;
+        if (host_direct) k_copy<<<2 * device_sms(), 256, 0, stream>>>(dz, z, n);
+        else GDP_MCUDA(cudaMemcpyAsync(z, dz, zb, cudaMemcpyDeviceToHost, stream));
+        GDP_MCUDA(cudaGetLastError());
+    }
     GDP_MCUDA(cudaStreamSynchronize(stream));
     return GDP_OKAY;
 }
