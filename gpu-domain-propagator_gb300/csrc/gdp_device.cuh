@@ -257,7 +257,7 @@ __device__ __forceinline__ MagEnc mag_enc(long long bits) {
 // NaN or inf terms make the screen's sums, magnitude sum or U NaN or inf,
 // and every such row is left to the exact pass; the sign test a32 > 0 equals
 // the reference's EPSGT(a, 0) for every coefficient, and a NaN copy keeps the
-// coefficient's sign (so the sign bit tells a > 0, as in candidate_sides).
+// coefficient's sign.
 constexpr float kF32Inf = __builtin_huge_valf();
 __host__ __device__ __forceinline__ float coef_screen(double a) {
     const double m = a < 0 ? -a : a;

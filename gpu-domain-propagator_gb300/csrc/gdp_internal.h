@@ -4,7 +4,7 @@
 //  * SELL-g slices (rows up to split_tile non-zeros): rows sorted by lanes per
 //    row g and length; a slice holds 32/g rows with g lanes each and stores
 //    its elements column-major (step i of lane l at slice_ptr[s] + 32*i + l),
-//    so a warp streams a slice with coalesced 128 B (col) / 256 B (val) loads.
+//    so a warp streams a slice with coalesced 128 B loads (columns, FP32 copies).
 //    Rows up to thread_row_max have g = 1: one lane sums the row left to
 //    right -- the reference's summation order. Longer rows get g = 2..32 lanes
 //    (about 32 elements per lane) and a shuffle-tree combine.
@@ -20,7 +20,7 @@
 //    coefficients with one 16-byte load.
 //  * FP32 screen copies of the coefficients (sell_a32, la32) and of the
 //    current bounds (bnd32): the screen streams 8 B per non-zero and gathers
-//    8 B per bound pair; the FP64 arrays are read only by the exact pass.
+//    one 16-byte record (batch members 8 bytes); the FP64 arrays are read only by the exact pass.
 //  * marking: per row position the round in which it must be processed next,
 //    and the positions of every variable's rows (CSC of positions).
 #pragma once

@@ -48,8 +48,8 @@ typedef struct {
                              (about 2 s at 2 GHz) */
     int cta_threads;      /* threads per CTA of the MEGAKERNEL loop: 128, 256 or 512; 0 (default) = 256,
                              or 512 on one CTA for problems of up to 512 rows of at most thread_row_max.
-                             With ctas_per_sm = 0 as many CTAs run per SM as fit (up to 6, 3 and 1,
-                             about 24 warps per SM) */
+                             With ctas_per_sm = 0 as many CTAs run per SM as fit (up to 4, 2 and 1,
+                             16 warps per SM) */
     int reserved[4];      /* must be zero */
 } gdp_options;
 
