@@ -288,6 +288,9 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
     unsigned target = 0;  // grid barrier
     int unit = -1;        // unit in the warp's cache, which its statistics belong to
     stats_zero(mine, lane);
+    // the round's work: units in the full sweep, their items, queued entries
+    int nfs = *((volatile int *)B.n_fs), fs_items = *((volatile int *)(B.fs_prefix + nfs));
+    int n_entries = (int)min(*((volatile unsigned *)(B.tail + 1)), B.cap_entries);
     for (int r = 1; r <= B.max_rounds; r++) {
         const int par = r & 1;
         unsigned *ctr = B.ctr + 4 * par;
@@ -298,9 +301,6 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
             for (int u = gtid; u < B.n_units; u += gthreads) close_round(B, u, r - 1);
         // ---- A
         {
-            const int nfs = *((volatile int *)B.n_fs);
-            const int fs_items = *((volatile int *)(B.fs_prefix + nfs));
-            const int n_entries = (int)min(*((volatile unsigned *)(B.tail + par)), B.cap_entries);
             const unsigned long long *ent = B.entries + (size_t)par * B.cap_entries;
             const int n_work = fs_items + n_entries;
             WarpCursor<false> cur;
@@ -322,10 +322,11 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
                     marked = true;
                 }
                 const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
-                if (*((volatile int *)&Pu.flags[0].infeasible)) continue;
+                const bool due = *((volatile int *)&Pu.flags[0].infeasible) == 0;
                 int *change = &Pu.flags[1 + par].change;
                 unsigned *tight = &Pu.flags[1 + par].tight;
                 if (kLearned && Pu.learned == 1) {
+                    if (!due) continue;
                     const int kind = Pu.flags[1 + par].kind;
                     if (it >= 0) {
                         if (lane == 0) L.marked = 0;
@@ -341,8 +342,8 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
                         push_tile(B.cq, B.tail + 2, B.cap_tiles, B.error, u, -it - 1);
                     }
                 } else if (it >= 0) {
-                    sell_slice<0, false>(Pu, it, lane, r, marked, change, tight, mine);
-                } else if (split_partial<0>(Pu, -it - 1, lane, r, marked, change, tight, mine) && lane == 0) {
+                    sell_slice<0, false>(Pu, it, lane, r, marked, change, tight, mine, 0, 0, 1, due);
+                } else if (due && split_partial<0>(Pu, -it - 1, lane, r, marked, change, tight, mine) && lane == 0) {
                     push_tile(B.cq, B.tail + 2, B.cap_tiles, B.error, u, -it - 1);
                 }
             }
@@ -477,9 +478,10 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
         }
         if (!grid_barrier(B.barrier, B.error, B.spin_limit, target)) return;
         last = r;
-        const int nfs = *((volatile int *)B.n_fs);
-        const int next = *((volatile int *)(B.fs_prefix + nfs)) +
-                         (int)min(*((volatile unsigned *)(B.tail + (par ^ 1))), B.cap_entries);
+        nfs = *((volatile int *)B.n_fs);
+        n_entries = (int)min(*((volatile unsigned *)(B.tail + (par ^ 1))), B.cap_entries);
+        fs_items = *((volatile int *)(B.fs_prefix + nfs));
+        const int next = fs_items + n_entries;
         const int pending = kLearned ? *((volatile int *)B.n_pending) : 0;
         if (!more || (next == 0 && pending == 0)) break;
     }

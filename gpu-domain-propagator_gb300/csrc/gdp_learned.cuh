@@ -171,7 +171,8 @@ __device__ __forceinline__ bool sell_slice_learned(const DevProblem &P, int slic
     }
     count_work(ws, lane, leader ? 1 : 0, leader ? len : 0, (leader && exact) ? len : 0);
     __syncwarp();
-    exact_slice(P, ws, lg, exact, r, len, slack_lo, c.minf, c.maxf, lhs, rhs, lane, change, tight_ctr, L.tight, L.go);
+    exact_slice(P, ws, lg, exact, r, exact ? __ldg(P.xptr + r) : 0, len, slack_lo, c.minf, c.maxf, lhs, rhs, lane, change,
+                tight_ctr, L.tight, L.go);
     __syncwarp();
     if (leader) {
         const bool tightened = L.tight[rl] != 0;
