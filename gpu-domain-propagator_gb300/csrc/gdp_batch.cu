@@ -170,45 +170,35 @@ __device__ __noinline__ int2 sweep_item(const int *prefix, int nfs, int total, i
     return make_int2(lo, before(p1) - before(p0) + i - below(p0));
 }
 
-// One block builds the list of units swept in full in the next round, in
-// unit order, with the prefix of their work-item counts.
+// One warp builds the list of units swept in full in the next round, in unit
+// order, with the prefix of their work-item counts, while the rest of its CTA
+// commits (with the whole CTA on the list first, a round of few changes waited
+// for it: 8 chain MIPs 31.8 ms, 31.4 so).
 template <class Pred>
-__device__ void build_full_sweep_list(const BatchDev &B, Pred &&pred) {
-    __shared__ int s_cnt[kCtaThreads / 32], s_items[kCtaThreads / 32];
-    __shared__ int s_base_u, s_base_i;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) { s_base_u = 0; s_base_i = 0; }
-    __syncthreads();
-    for (int u0 = 0; u0 < B.n_units; u0 += kCtaThreads) {
-        const int u = u0 + tid;
-        const int f = (u < B.n_units && pred(u)) ? 1 : 0;
+__device__ void build_full_sweep_list(const BatchDev &B, int lane, Pred &&pred) {
+    int units = 0, before = 0;  // listed so far, their items
+    for (int u0 = 0; u0 < B.n_units; u0 += 32) {
+        const int u = u0 + lane;
+        const bool f = u < B.n_units && pred(u);
         const int items = f ? B.units[u].n_items : 0;
-        int cf = f, ci = items;  // inclusive warp scans
+        const unsigned listed = __ballot_sync(kFull, f);
+        int upto = items;  // inclusive scan
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const int a = __shfl_up_sync(kFull, cf, off), b = __shfl_up_sync(kFull, ci, off);
-            if (lane >= off) { cf += a; ci += b; }
-        }
-        if (lane == 31) { s_cnt[wid] = cf; s_items[wid] = ci; }
-        __syncthreads();
-        int wf = 0, wi = 0, tf = 0, ti = 0;
-        for (int w = 0; w < kCtaThreads / 32; w++) {
-            if (w < wid) { wf += s_cnt[w]; wi += s_items[w]; }
-            tf += s_cnt[w];
-            ti += s_items[w];
+            const int v = __shfl_up_sync(kFull, upto, off);
+            if (lane >= off) upto += v;
         }
         if (f) {
-            const int k = s_base_u + wf + cf - 1;
+            const int k = units + __popc(listed & ((1u << lane) - 1u));
             B.fs_unit[k] = u;
-            B.fs_prefix[k] = s_base_i + wi + ci - items;
+            B.fs_prefix[k] = before + upto - items;
         }
-        __syncthreads();
-        if (tid == 0) { s_base_u += tf; s_base_i += ti; }
-        __syncthreads();
+        units += __popc(listed);
+        before += __shfl_sync(kFull, upto, 31);
     }
-    if (tid == 0) {
-        B.fs_prefix[s_base_u] = s_base_i;
-        B.n_fs[0] = s_base_u;
+    if (lane == 0) {
+        B.fs_prefix[units] = before;
+        B.n_fs[0] = units;
     }
 }
 
@@ -398,15 +388,15 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
             if (B.units[u].flags[0].infeasible_row != INT_MAX) B.units[u].flags[0].infeasible = 1;
         const bool more = r < B.max_rounds;
         if (blockIdx.x == 0) {
-            if (more)
-                build_full_sweep_list(B, [&](int u) {
+            if (more && threadIdx.x < 32)
+                build_full_sweep_list(B, lane, [&](int u) {
                     const DevProblem &Pu = B.units[u];
                     if (kLearned && Pu.learned == 1)
                         return !Pu.flags[0].done && !Pu.flags[0].infeasible && !unit_certified(Pu, r) &&
                                unit_next_kind(Pu, r) == kRoundFull;
                     return !Pu.flags[0].done && Pu.flags[1 + par].change && !unit_next_marked(Pu, r);
                 });
-            else if (threadIdx.x == 0) {
+            else if (!more && threadIdx.x == 0) {
                 B.n_fs[0] = 0;
                 B.fs_prefix[0] = 0;
             }
@@ -452,19 +442,20 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
                     const unsigned bits = __shfl_sync(kFull, my, q);
                     const int u = find_unit(B.wbase, B.n_units, w0 + q);
                     const DevProblem &Pu = unit_of(B, cache, mine, unit, u, lane);
+                    const bool on = (bits >> lane) & 1u;
+                    const int j = (w0 + q - __ldg(B.wbase + u)) * 32 + lane;
+                    int k0 = 0, k1 = 0;
+                    double2 b = make_double2(0.0, 0.0);
+                    if (on) {
+                        b = Pu.bnd_nxt[j];
+                        k0 = __ldg(Pu.var_ptr + j);
+                        k1 = __ldg(Pu.var_ptr + j + 1);
+                    }
                     if (lane == 0) atomicAdd(&Pu.flags[0].changed_vars, (unsigned long long)__popc(bits));
                     const bool lrn = kLearned && Pu.learned == 1;
                     const bool push = more && (lrn ? (!unit_certified(Pu, r) && unit_next_kind(Pu, r) != kRoundFull)
                                                    : unit_next_marked(Pu, r));
-                    const bool on = (bits >> lane) & 1u;
-                    int k0 = 0, k1 = 0;
                     if (on) {
-                        const int j = (w0 + q - __ldg(B.wbase + u)) * 32 + lane;
-                        const double2 b = Pu.bnd_nxt[j];
-                        if (push) {
-                            k0 = __ldg(Pu.var_ptr + j);
-                            k1 = __ldg(Pu.var_ptr + j + 1);
-                        }
                         Pu.bnd[j] = b;
                         store_bnd32<0>(Pu, j, b, r);
                         if (var_infeasible(b.x, b.y)) {
@@ -559,7 +550,8 @@ __global__ void __launch_bounds__(kCtaThreads) k_batch_plan(BatchDev B, const in
         }
     }
     __syncthreads();
-    build_full_sweep_list(B, [&](int u) { return seed_mode[u] == 0 && !B.units[u].flags[0].infeasible; });
+    if (threadIdx.x < 32)
+        build_full_sweep_list(B, threadIdx.x, [&](int u) { return seed_mode[u] == 0 && !B.units[u].flags[0].infeasible; });
 }
 
 __global__ void __launch_bounds__(256) k_batch_fini(BatchDev B, double *lb, double *ub, const long long *var_base) {
