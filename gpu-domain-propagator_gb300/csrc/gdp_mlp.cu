@@ -608,34 +608,44 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     // 16-byte loads need an aligned array (numpy's are); another one is copied
     const bool direct = host_direct && reinterpret_cast<uintptr_t>(x) % 16 == 0;
     const size_t xb = sizeof(float) * (size_t)n * kMlpIn, zb = sizeof(float) * (size_t)n;
-    // The logits of a small call go straight to host memory. The GPU's first write
-    // to a page that nothing has touched yet is a fault of many microseconds, so
-    // those of a large one (a new array of that size has new pages) go to device
-    // memory, and the host touches the pages while the kernel runs (2M rows into a
-    // new array: 3.6 ms written directly, 0.77 so, 1.9 with every copy; into one
-    // that was written before: 0.79, 0.81).
-    constexpr size_t kDirectBytes = 64 << 10;
+    // The logits go straight to host memory. The GPU's first write to a page that
+    // nothing has touched yet is a fault of many microseconds, and a new array has new
+    // pages, so the host touches them: up to 1 MB before the launch, of more while the
+    // first quarter of the rows runs, whose logits go by way of device memory (2M rows
+    // into a new array: 3.6 ms written untouched, 0.77 with all of them by way of
+    // device memory, 0.72 so, 1.9 with the features copied too).
+    constexpr size_t kTouchFirst = 1 << 20;
+    const int early = !direct ? n : zb > kTouchFirst ? n / 4 / 16 * 16 : 0;  // rows by way of device memory
     Arena tmp;
     const Drained drained{stream};
     const float *dx = x;
-    float *dz = z;
+    float *dz = nullptr;
     if (!direct) {
         float *up = (float *)tmp.alloc_bytes(xb);
         if (!up) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
         GDP_MCUDA(cudaMemcpyAsync(up, x, xb, cudaMemcpyHostToDevice, stream));
         dx = up;
     }
-    if (!direct || zb > kDirectBytes) dz = (float *)tmp.alloc_bytes(zb);
-    if (!dz) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
-    k_mlp_forward<<<forward_grid(n), kMlpThreads, 0, stream>>>(dev(), dx, n, dz);
-    GDP_MCUDA(cudaGetLastError());
-    if (dz != z) {
-        const long long pages = (long long)((zb + 4095) / 4096);
-#pragma omp parallel for schedule(static) num_threads(omp_threads(pages))
-        for (long long i = 0; i < pages; i++) *((volatile char *)z + 4096 * i) = 0;
-        if (host_direct) k_copy<<<2 * device_sms(), 256, 0, stream>>>(dz, z, n);
-        else GDP_MCUDA(cudaMemcpyAsync(z, dz, zb, cudaMemcpyDeviceToHost, stream));
+    if (early) {
+        dz = (float *)tmp.alloc_bytes(sizeof(float) * (size_t)early);
+        if (!dz) { set_error("device allocation failed (forward)"); return GDP_ERROR; }
+        k_mlp_forward<<<forward_grid(early), kMlpThreads, 0, stream>>>(dev(), dx, early, dz);
         GDP_MCUDA(cudaGetLastError());
+    }
+    const long long pages = (long long)((zb + 4095) / 4096);
+#pragma omp parallel for schedule(static) num_threads(omp_threads(pages)) if (pages > 256)
+    for (long long i = 0; i < pages; i++) *((volatile char *)z + 4096 * i) = 0;
+    *((volatile char *)z + zb - 1) = 0;  // an array that does not start on a page has one more
+    if (early < n) {
+        k_mlp_forward<<<forward_grid(n - early), kMlpThreads, 0, stream>>>(dev(), dx + (size_t)early * kMlpIn, n - early,
+                                                                          z + early);
+        GDP_MCUDA(cudaGetLastError());
+    }
+    if (early && host_direct) {
+        k_copy<<<2 * device_sms(), 256, 0, stream>>>(dz, z, early);
+        GDP_MCUDA(cudaGetLastError());
+    } else if (early) {
+        GDP_MCUDA(cudaMemcpyAsync(z, dz, sizeof(float) * (size_t)early, cudaMemcpyDeviceToHost, stream));
     }
     GDP_MCUDA(cudaStreamSynchronize(stream));
     return GDP_OKAY;
