@@ -605,9 +605,12 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     if (n < 0 || (n && (!x || !z))) { set_error("bad forward arguments"); return GDP_ERROR; }
     if (!n) return GDP_OKAY;
     GDP_MCUDA(cudaSetDevice(device));
-    // 16-byte loads need an aligned array (numpy's are); another one is copied
-    const bool direct = host_direct && reinterpret_cast<uintptr_t>(x) % 16 == 0;
     const size_t xb = sizeof(float) * (size_t)n * kMlpIn, zb = sizeof(float) * (size_t)n;
+    // 16-byte loads need an aligned array (numpy's are), and logits may be written
+    // while features are still read: other features are copied first
+    const uintptr_t xa = reinterpret_cast<uintptr_t>(x), za = reinterpret_cast<uintptr_t>(z);
+    const bool overlap = xa < za + zb && za < xa + xb;
+    const bool direct = host_direct && xa % 16 == 0 && !overlap;
     // The logits go straight to host memory. The GPU's first write to a page that
     // nothing has touched yet is a fault of many microseconds, and a new array has new
     // pages, so the host touches them: up to 1 MB before the launch, of more while the
@@ -632,6 +635,7 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
         k_mlp_forward<<<forward_grid(early), kMlpThreads, 0, stream>>>(dev(), dx, early, dz);
         GDP_MCUDA(cudaGetLastError());
     }
+    if (overlap) GDP_MCUDA(cudaStreamSynchronize(stream));  // the features are read before z changes
     const long long pages = (long long)((zb + 4095) / 4096);
 #pragma omp parallel for schedule(static) num_threads(omp_threads(pages)) if (pages > 256)
     for (long long i = 0; i < pages; i++) *((volatile char *)z + 4096 * i) = 0;

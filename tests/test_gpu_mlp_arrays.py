@@ -1,0 +1,35 @@
+"""The host arrays a caller may give the MLP's forward pass: logits that share
+memory with the features. Results are the bits of the plain call."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import gdp
+
+pytestmark = pytest.mark.gpu
+
+FLOATS = C.POINTER(C.c_float)
+
+
+def _forward_at(model, n, x_addr, z_addr):
+    """gdp_mlp_forward on raw addresses."""
+    rc = model._lib.gdp_mlp_forward(model._h, n, C.cast(x_addr, FLOATS), C.cast(z_addr, FLOATS))
+    assert rc == gdp.GDP_OKAY, gdp.last_error()
+
+
+def _features(n, seed=5):
+    return np.random.default_rng(seed).normal(0, 1, (n, gdp.MLP_FEATURES)).astype(np.float32)
+
+
+# 262,144 rows are the last whose logits (1 MB) are written by one launch
+@pytest.mark.parametrize("n", [1, 17, 5000, 262_144, 262_145])
+@pytest.mark.parametrize("where", ["front", "middle", "last row"])
+def test_logits_over_the_features(n, where):
+    m = gdp.Mlp(seed=3)
+    x = _features(n)
+    z = m.forward(x)
+    buf = np.concatenate([x.ravel(), np.zeros(n, np.float32)])
+    at = {"front": 0, "middle": 16 * (n // 2), "last row": 16 * n - 16}[where]
+    _forward_at(m, n, buf.ctypes.data, buf.ctypes.data + 4 * at)
+    assert np.array_equal(buf[at:at + n], z)
