@@ -900,7 +900,6 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
     P.max_rounds = opts.max_rounds;
     P.spin_limit = opts.barrier_wait_kcycles > 0 ? 1000LL * opts.barrier_wait_kcycles : 4000000000LL;
     const size_t nl = (size_t)n_lrows, nt = (size_t)n_tiles, nv = (size_t)n;
-    const size_t staged = host_direct ? 0 : sizeof(double) * nv;
     if (!arena.carve({{(void **)&P.tile_part, sizeof(TilePart) * nt},
                       {(void **)&P.tile_scr, sizeof(TileScr) * nt},
                       {(void **)&P.xrow, sizeof(XRow) * (size_t)ns},
@@ -916,12 +915,11 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
                       {(void **)&P.chg, sizeof(unsigned) * (size_t)n_words},
                       {(void **)&P.flags, sizeof(RoundFlags) * 3},
                       {(void **)&P.barrier, sizeof(unsigned) * 2},
-                      {(void **)&P.queue, sizeof(unsigned) * 8},
-                      {(void **)&d_lb, staged},
-                      {(void **)&d_ub, staged}})) {
+                      {(void **)&P.queue, sizeof(unsigned) * 8}})) {
         set_error("device allocation failed");
         return GDP_ERROR;
     }
+    if (!host_direct && alloc_staging() != GDP_OKAY) return GDP_ERROR;
 
     if (set_schedule(opts.sync_type, opts.ctas_per_sm, opts.cta_threads) != GDP_OKAY) return GDP_ERROR;
     stamps.mark(5);
@@ -1255,9 +1253,21 @@ GDP_RETCODE Context::trace(double *lbs, double *ubs, int capacity, float *x_out,
     return rc;
 }
 
+// Device copies of host bounds: for contexts without coherent access, and on
+// first use for arrays that are not aligned as the kernels' loads need.
+GDP_RETCODE Context::alloc_staging() {
+    const size_t bytes = sizeof(double) * (size_t)std::max(n, 1);
+    if (d_lb || arena.carve({{(void **)&d_lb, bytes}, {(void **)&d_ub, bytes}})) return GDP_OKAY;
+    set_error("device allocation failed (bounds)");
+    return GDP_ERROR;
+}
+
 GDP_RETCODE Context::propagate_host(const double *lbs_in, const double *ubs_in, double *lbs_out, double *ubs_out,
                                     gdp_stats *st) {
-    if (host_direct) {
+    bool aligned = true;
+    for (const double *a : {lbs_in, ubs_in, (const double *)lbs_out, (const double *)ubs_out})
+        aligned = aligned && reinterpret_cast<uintptr_t>(a) % sizeof(double) == 0;
+    if (host_direct && aligned) {
         // coherent access to pageable memory (NVLink-C2C on Grace hosts): the
         // first kernel reads the caller's bounds where they are, and the last
         // one writes the result to them once the rounds succeeded
@@ -1266,6 +1276,7 @@ GDP_RETCODE Context::propagate_host(const double *lbs_in, const double *ubs_in, 
         return rc;
     }
     copy_bounds(lbs_in, ubs_in, lbs_out, ubs_out);
+    if (alloc_staging() != GDP_OKAY) return GDP_ERROR;
     const size_t bytes = sizeof(double) * (size_t)n;
     GDP_CUDA(cudaMemcpyAsync(d_lb, lbs_in, bytes, cudaMemcpyHostToDevice, stream));
     GDP_CUDA(cudaMemcpyAsync(d_ub, ubs_in, bytes, cudaMemcpyHostToDevice, stream));

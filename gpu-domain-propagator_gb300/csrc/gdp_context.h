@@ -98,7 +98,7 @@ public:
     RoundFlags *h_flags = nullptr;  // pinned
     Arena arena;
     DevProblem P{};
-    double *d_lb = nullptr, *d_ub = nullptr;  // staging for host bounds (not with host_direct)
+    double *d_lb = nullptr, *d_ub = nullptr;  // staging for host bounds (alloc_staging)
     int n_sms = 0, vec_blocks = 1, act_blocks = 1, cand_blocks = 1, mega_grid = 1, learned_grid = 1;
     int mega_warps = 8;  // warps per CTA of the megakernel (opts.cta_threads / 32)
     int n_srows = 0, n_slices = 0, n_lrows = 0, n_tiles = 0;
@@ -121,6 +121,7 @@ private:
     GDP_RETCODE rounds_megakernel(cudaStream_t s, int *launches);
     GDP_RETCODE rounds_learned(cudaStream_t s, int *launches);
     GDP_RETCODE alloc_learned_state();
+    GDP_RETCODE alloc_staging();
 };
 
 }  // namespace gdp
