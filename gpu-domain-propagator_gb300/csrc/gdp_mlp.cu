@@ -611,6 +611,7 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     const uintptr_t xa = reinterpret_cast<uintptr_t>(x), za = reinterpret_cast<uintptr_t>(z);
     const bool overlap = xa < za + zb && za < xa + xb;
     const bool direct = host_direct && xa % 16 == 0 && !overlap;
+    const bool z_direct = host_direct && za % alignof(float) == 0;
     // The logits go straight to host memory. The GPU's first write to a page that
     // nothing has touched yet is a fault of many microseconds, and a new array has new
     // pages, so the host touches them: up to 1 MB before the launch, of more while the
@@ -618,7 +619,8 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
     // into a new array: 3.6 ms written untouched, 0.77 with all of them by way of
     // device memory, 0.72 so, 1.9 with the features copied too).
     constexpr size_t kTouchFirst = 1 << 20;
-    const int early = !direct ? n : zb > kTouchFirst ? n / 4 / 16 * 16 : 0;  // rows by way of device memory
+    // rows by way of device memory
+    const int early = !direct || !z_direct ? n : zb > kTouchFirst ? n / 4 / 16 * 16 : 0;
     Arena tmp;
     const Drained drained{stream};
     const float *dx = x;
@@ -645,7 +647,7 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
                                                                           z + early);
         GDP_MCUDA(cudaGetLastError());
     }
-    if (early && host_direct) {
+    if (early && z_direct) {
         k_copy<<<2 * device_sms(), 256, 0, stream>>>(dz, z, early);
         GDP_MCUDA(cudaGetLastError());
     } else if (early) {

@@ -1,5 +1,6 @@
 """The host arrays a caller may give the MLP's forward pass: logits that share
-memory with the features. Results are the bits of the plain call."""
+memory with the features, features and logits that start on any byte. Results are
+the bits of the plain call."""
 import ctypes as C
 
 import numpy as np
@@ -33,3 +34,18 @@ def test_logits_over_the_features(n, where):
     at = {"front": 0, "middle": 16 * (n // 2), "last row": 16 * n - 16}[where]
     _forward_at(m, n, buf.ctypes.data, buf.ctypes.data + 4 * at)
     assert np.array_equal(buf[at:at + n], z)
+
+
+@pytest.mark.parametrize("n", [1, 17, 5000, 262_145])
+@pytest.mark.parametrize("x_by,z_by", [(0, 1), (0, 2), (4, 3), (2, 0), (3, 3)])
+def test_arrays_off_their_alignment(n, x_by, z_by):
+    m = gdp.Mlp(seed=3)
+    x = _features(n)
+    z = m.forward(x)
+    xraw, zraw = np.zeros(x.nbytes + 32, np.uint8), np.zeros(z.nbytes + 32, np.uint8)
+    x0 = (-xraw.ctypes.data) % 16 + x_by
+    z0 = (-zraw.ctypes.data) % 16 + z_by
+    xraw[x0:x0 + x.nbytes] = x.view(np.uint8).ravel()
+    _forward_at(m, n, xraw.ctypes.data + x0, zraw.ctypes.data + z0)
+    assert zraw[z0:z0 + z.nbytes].tobytes() == z.tobytes()
+    assert not zraw[:z0].any() and not zraw[z0 + z.nbytes:].any()
