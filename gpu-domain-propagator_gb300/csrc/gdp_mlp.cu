@@ -28,6 +28,7 @@
 
 #include "gdp_context.h"
 #include "gdp_mlp.h"
+#include "gdp_pages.h"
 
 namespace gdp {
 
@@ -596,9 +597,9 @@ GDP_RETCODE Mlp::upload(Arena &mem, int n, const float *x, const float *y, const
     return GDP_OKAY;
 }
 
-// Host threads that touch `pages` pages.
-static int omp_threads(long long pages) {
-    return (int)std::max(1LL, std::min<long long>(pages >> 8, omp_get_max_threads() - 1));
+// Host threads that touch the pages of `bytes` bytes: one per MB.
+static int touch_threads(size_t bytes) {
+    return (int)std::max(1LL, std::min<long long>((long long)(bytes >> 20), omp_get_max_threads() - 1));
 }
 
 GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
@@ -637,11 +638,7 @@ GDP_RETCODE Mlp::forward(int n, const float *x, float *z) {
         k_mlp_forward<<<forward_grid(early), kMlpThreads, 0, stream>>>(dev(), dx, early, dz);
         GDP_MCUDA(cudaGetLastError());
     }
-    if (overlap) GDP_MCUDA(cudaStreamSynchronize(stream));  // the features are read before z changes
-    const long long pages = (long long)((zb + 4095) / 4096);
-#pragma omp parallel for schedule(static) num_threads(omp_threads(pages)) if (pages > 256)
-    for (long long i = 0; i < pages; i++) *((volatile char *)z + 4096 * i) = 0;
-    *((volatile char *)z + zb - 1) = 0;  // an array that does not start on a page has one more
+    if (z_direct) touch_pages(z, zb, touch_threads(zb));
     if (early < n) {
         k_mlp_forward<<<forward_grid(n - early), kMlpThreads, 0, stream>>>(dev(), dx + (size_t)early * kMlpIn, n - early,
                                                                           z + early);
