@@ -1300,7 +1300,20 @@ void Context::copy_bounds(const double *lbs_in, const double *ubs_in, double *lb
 }
 
 GDP_RETCODE Context::propagate_device(double *d_lbs, double *d_ubs, cudaStream_t s, gdp_stats *st) {
-    if (!s) s = stream;
+    if (!s) {
+        // Handle 0 is the default stream to whoever fills the bounds (a framework's
+        // current stream): what it has queued there so far comes first. The context's
+        // stream does not wait for it by itself. While a stream that the default
+        // stream waits for is being captured, the default stream takes no work.
+        s = stream;
+        cudaStreamCaptureStatus status;
+        if (cudaStreamIsCapturing(cudaStreamLegacy, &status) == cudaSuccess) {
+            GDP_CUDA(cudaEventRecord(res->uploaded, cudaStreamLegacy));
+            GDP_CUDA(cudaStreamWaitEvent(s, res->uploaded, 0));
+        } else {
+            cudaGetLastError();
+        }
+    }
     return run(d_lbs, d_ubs, d_lbs, d_ubs, s, st);
 }
 

@@ -348,7 +348,8 @@ class Context:
         return x[:k.value].copy(), y[:k.value].copy(), lbo, ubo, st.as_dict()
 
     def propagate_device(self, d_lb_ptr: int, d_ub_ptr: int, stream_ptr: int = 0) -> dict:
-        """Propagates device-resident bounds (raw device pointers, e.g. torch data_ptr())."""
+        """Propagates device-resident bounds (raw device pointers, e.g. torch data_ptr())
+        after what the stream holds so far (0: the default stream)."""
         st = Stats()
         _check(self._lib.gdp_propagate_device(self._h, C.c_void_p(d_lb_ptr), C.c_void_p(d_ub_ptr),
                                               C.c_void_p(stream_ptr or None), C.byref(st)),

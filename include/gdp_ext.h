@@ -121,8 +121,9 @@ GDP_RETCODE gdp_propagate_into(gdp_context *ctx, const double *lbs_in, const dou
                                double *ubs_out, gdp_stats *stats);
 
 /* Same on device-resident bounds (d_lbs/d_ubs: n_vars doubles each in device
- * memory, in/out) on the given CUDA stream (NULL: the context's stream). The
- * call returns after the propagation has finished. */
+ * memory, in/out) on the given CUDA stream (NULL: the context's stream, after
+ * what the legacy default stream holds so far). The call returns after the
+ * propagation has finished. */
 GDP_RETCODE gdp_propagate_device(gdp_context *ctx, double *d_lbs, double *d_ubs, void *stream,
                                  gdp_stats *stats);
 
