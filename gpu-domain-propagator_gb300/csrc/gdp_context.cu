@@ -1021,13 +1021,15 @@ Context::~Context() {
 // host: 100 us a round with five launches, a copy and a synchronisation became
 // 83 us on 60,001 power-law rows, 44 us became 27 us on 2,000 rows.
 GDP_RETCODE Context::rounds_cpu_loop(cudaStream_t s, int *launches, const std::function<void()> &meanwhile) {
+    DevProblem Q = P;
+    Q.spin_limit = kLongSpinLimit;  // a driver of launches: no wait of its rounds is an error to the caller
     volatile int *mail = reinterpret_cast<volatile int *>(h_flags + 2);
     mail[0] = 0;
     mail[1] = 1;
     int queued = 0;
     for (int round = 1; round <= opts.max_rounds; round++) {
         for (; queued < std::min(round + 1, opts.max_rounds); queued++)
-            GDP_CUDA(launch_megakernel(P, queued + 1, queued + 1, const_cast<int *>(mail), mega_grid, mega_warps, s));
+            GDP_CUDA(launch_megakernel(Q, queued + 1, queued + 1, const_cast<int *>(mail), mega_grid, mega_warps, s));
         if (round == 1) meanwhile();
         // the round's mail, or an idle stream: the bounds were infeasible from
         // the start, or a launch ended with an error

@@ -213,6 +213,12 @@ struct DevProblem {
     long long spin_limit;  // clock64 cycles one grid-barrier wait may last (gdp_options.barrier_wait_kcycles)
 };
 
+// clock64 cycles (about 9 minutes at 2 GHz) that a grid-barrier wait may last in
+// loops that gdp_options.barrier_wait_kcycles does not cover. A wait lasts as long as
+// the longest item of its phase, which has no bound of its own (a row of 2^31
+// elements is added up from left to right in 76 s): the limit only ends a fault.
+constexpr long long kLongSpinLimit = 1LL << 40;
+
 constexpr int kWarpsPerCta = 8;
 constexpr int kCtaThreads = 32 * kWarpsPerCta;
 

@@ -45,9 +45,11 @@ typedef struct {
                              learned marking, batches), in thousands of SM clock cycles; a CTA that
                              waits longer records a device error, every CTA leaves at its next
                              barrier and the call returns GDP_ERROR. 0 (default) = 4,000,000
-                             (about 2 s at 2 GHz) */
-    int cta_threads;      /* threads per CTA of the MEGAKERNEL loop: 128, 256 or 512; 0 (default) = 256,
-                             or 512 on one CTA for problems of up to 512 rows of at most thread_row_max.
+                             (about 2 s at 2 GHz). CPU_LOOP and GPU_LOOP are not subject to it
+                             (a wait in CPU_LOOP's rounds ends after 2^40 cycles, 9 minutes) */
+    int cta_threads;      /* threads per CTA of the MEGAKERNEL and CPU_LOOP rounds: 128, 256 or 512;
+                             0 (default) = 256, or 512 on one CTA for problems of up to 512 rows of at
+                             most thread_row_max.
                              With ctas_per_sm = 0 as many CTAs run per SM as fit (up to 4, 2 and 1,
                              16 warps per SM) */
     int reserved[4];      /* must be zero */
