@@ -71,7 +71,6 @@ constexpr int kLongRow = 1024;
 constexpr unsigned kLongCap = 1 << 16;
 constexpr int kNaWarps = 8;
 constexpr int kNaThreads = 32 * kNaWarps;
-constexpr long long kNaSpinLimit = 4000000000LL;  // clock64 cycles of one grid-barrier wait, about 2 s
 
 // Round state: flags.* as in the context path; per-round values by parity.
 struct NaState {
@@ -707,7 +706,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
         }
         exact_drain(T, ws.xs, Q, true, lane);
         if (__any_sync(kFull, Q.tight) && lane == 0) st->tight[par] = 1;
-        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit, target)) return;
+        if (!grid_barrier(st->barrier, &st->flags.error, kLongSpinLimit, target)) return;
         // commit: the caller's arrays hold the round's result
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             st->claim[par ^ 1] = 0u;
@@ -736,7 +735,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
             atomicAdd(&st->changed[par], (unsigned)changed);
             atomicAdd(&st->flags.changed_vars, (unsigned long long)changed);
         }
-        if (!grid_barrier(st->barrier, &st->flags.error, kNaSpinLimit, target)) return;
+        if (!grid_barrier(st->barrier, &st->flags.error, kLongSpinLimit, target)) return;
         last_tight = *((volatile int *)&st->tight[par]);
         if (!last_tight || *((volatile int *)&st->flags.infeasible)) break;
     }

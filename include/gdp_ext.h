@@ -334,7 +334,8 @@ void gdp_mps_free(gdp_mps_problem *p);
  *   - The first call on a device looks up that array's device address (once per
  *     device).
  *   - Every round runs in one cooperative launch; the call synchronizes its
- *     stream once, at its end.
+ *     stream once, at its end. Rounds may take any time (a grid-barrier wait
+ *     returns GDP_ERROR after 2^40 cycles, about 9 minutes).
  *   - Calls share the array: calls that overlap on the GPU race and must be
  *     serialized by the caller. Each call re-initializes it.
  *   - Rows are summed left to right: results equal the context path's for rows
