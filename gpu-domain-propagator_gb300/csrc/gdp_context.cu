@@ -994,7 +994,7 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     }
     opts.sync_type = sync_type;
     opts.ctas_per_sm = ctas_per_sm;
-    opts.cta_threads = cta_threads;
+    opts.cta_threads = one_cta ? 0 : cta_threads;  // what makes the same schedule again: 512 would make several CTAs
     return GDP_OKAY;
 }
 

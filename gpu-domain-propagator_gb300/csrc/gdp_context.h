@@ -100,7 +100,7 @@ public:
     DevProblem P{};
     double *d_lb = nullptr, *d_ub = nullptr;  // staging for host bounds (alloc_staging)
     int n_sms = 0, vec_blocks = 1, act_blocks = 1, cand_blocks = 1, mega_grid = 1, learned_grid = 1;
-    int mega_warps = 8;  // warps per CTA of the megakernel (opts.cta_threads / 32)
+    int mega_warps = 8;  // warps per CTA of the megakernel (opts.cta_threads / 32; 16 where that is 0)
     int n_srows = 0, n_slices = 0, n_lrows = 0, n_tiles = 0;
     long long sell_elems = 0;
     // the last propagation converged feasibly: P.bnd is a fixpoint of the problem

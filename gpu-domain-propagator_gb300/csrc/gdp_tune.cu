@@ -124,7 +124,7 @@ GDP_RETCODE autotune(int m, int n, int nnz, const int *col, const int *row_ptr, 
     };
     auto record = [&](const gdp_options &o, int rounds, double t) {
         out.trials.push_back(gdp_tune_trial{o.thread_row_max, o.split_tile, o.sync_type, o.ctas_per_sm, rounds,
-                                            o.cta_threads ? o.cta_threads : 256, t});
+                                            o.cta_threads, t});
         if (t < out.best_ms) {
             out.best_ms = t;
             out.best = o;

@@ -267,7 +267,8 @@ GDP_RETCODE gdp_context_trace(gdp_context *ctx, double *lbs, double *ubs, int ca
  * Results are cached per problem shape (device, m, n, nnz, the histogram of
  * row lengths in powers of two, base's round cap and marking): a later call
  * for a problem of the same shape returns the cached options and trials at
- * once. gdp_autotune_clear_cache empties the cache. */
+ * once. gdp_autotune_clear_cache empties the cache. cta_threads in *best and the
+ * trials is 0 for the one CTA that small problems run on by default. */
 typedef struct {
     int thread_row_max, split_tile, sync_type, ctas_per_sm, rounds, cta_threads;
     double ms;
