@@ -935,8 +935,14 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
 // cta_threads 0: the default, 256, or one CTA of 512 threads for up to
 // kOneCtaSlices slices of one-lane rows: its barrier is __syncthreads and its
 // L1 stays valid from round to round (400 rows: 0.38 ms against 0.57 on 4 CTAs
-// of 256 threads; 800 rows, 25 slices: 0.61 against 0.60).
+// of 256 threads; 800 rows, 25 slices: 0.61 against 0.60). Its 16 warps also commit
+// every round, a word of the change bitmap per warp and step, so the variables count
+// too, the more the fewer warps the slices leave idle. MEGAKERNEL, one CTA against the
+// grid: 30 rows, 125 words 0.062 and 0.071 ms, 375 words 0.080 and 0.072; 100 rows, 32
+// words 0.082 and 0.086, 125 words 0.104 and 0.098; 400 rows, 10 words 0.29 and 0.34, 63
+// words 0.43 and 0.38, 31,250 words 10.9 and 0.46.
 constexpr int kOneCtaSlices = 16;
+constexpr long long kOneCtaWords = 192;  // slices x words
 // Warps that share a slice in place, up to 4 while that takes no more than
 // kPartWarps warps: each screens the whole slice and runs its share of the exact
 // rows, with more lanes per chain (30 rows: 0.089 -> 0.069 ms, 2,000 0.318 ->
@@ -953,7 +959,8 @@ GDP_RETCODE Context::set_schedule(int sync_type, int ctas_per_sm, int cta_thread
     }
     GDP_CUDA(cudaSetDevice(opts.device));
     const bool one_lane = n_lrows == 0 && P.cls_end[0] == n_srows && P.cls_begin[0] == 0;
-    const bool one_cta = cta_threads == 0 && one_lane && P.n_items <= kOneCtaSlices;
+    const bool one_cta = cta_threads == 0 && one_lane && P.n_items <= kOneCtaSlices &&
+                         (long long)P.n_items * P.n_chg_words <= kOneCtaWords;
     if (cta_threads == 0) cta_threads = one_cta ? 512 : 256;
     const int warps = cta_threads / 32;
     int act_bps = 0, cand_bps = 0, mega_bps = 0;

@@ -49,7 +49,7 @@ typedef struct {
                              (a wait in CPU_LOOP's rounds ends after 2^40 cycles, 9 minutes) */
     int cta_threads;      /* threads per CTA of the MEGAKERNEL and CPU_LOOP rounds: 128, 256 or 512;
                              0 (default) = 256, or 512 on one CTA for problems of up to 512 rows of at
-                             most thread_row_max.
+                             most thread_row_max and not many more variables than rows.
                              With ctas_per_sm = 0 as many CTAs run per SM as fit (up to 4, 2 and 1,
                              16 warps per SM) */
     int reserved[4];      /* must be zero */

@@ -1,5 +1,7 @@
-"""The schedule of small problems, one CTA of 512 threads by default: it survives a
+"""The schedule of small problems, one CTA of 512 threads by default (unless they have
+many variables, whose change bitmap that CTA reads every round): it survives a
 change of options, and the tuner hands back the schedule that it timed."""
+import numpy as np
 import pytest
 
 import gdp
@@ -54,3 +56,22 @@ def test_tuned_schedule_is_the_timed_one():
                                                   "cta_threads")}) as ctx:
         assert (ctx.layout()["mega_grid"] == 1) == (opts["cta_threads"] == 0)
         _exact(mip, ctx, split_len=opts["thread_row_max"])
+
+
+def _spread(mip, n):
+    """The rows of `mip` over n variables, most of them in no row."""
+    at = np.sort(np.random.default_rng(0).choice(n, mip.n, replace=False)).astype(np.int32)
+    lb, ub, vartype = np.zeros(n), np.full(n, 10.0), np.full(n, 3, np.int32)
+    lb[at], ub[at], vartype[at] = mip.lb, mip.ub, mip.vartype
+    return gdp.MIP(mip.row_ptr, at[mip.col], mip.val, mip.lhs, mip.rhs, lb, ub, vartype)
+
+
+@pytest.mark.parametrize("m,n,one", [(30, 6144, True), (30, 6145, False), (100, 1536, True), (100, 1537, False),
+                                     (512, 384, True), (512, 385, False), (400, 1_000_000, False)])
+def test_many_variables_take_the_grid(m, n, one):
+    mip = _spread(gdpgen.random_mip(0, seed=5, m=m, n=min(n, 3 * m // 4)), n)
+    with gdp.Context(mip) as ctx:
+        assert (ctx.layout()["mega_grid"] == 1) == one
+        for sync in (gdp.CPU_LOOP, gdp.MEGAKERNEL):
+            ctx.set_options(sync_type=sync)
+            _exact(mip, ctx)
