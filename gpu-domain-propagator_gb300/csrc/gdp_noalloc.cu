@@ -219,6 +219,7 @@ struct NaWarp {
     double d[kStage];     // |a| (ub - lb)
     int src[32];
     unsigned char own[32];  // lanes of the rows that take the exact pass
+    unsigned long long rows, nnz;  // rows that this warp swept and their non-zeros, kept by lane 0
 };
 constexpr int kScreenStage = 128;  // elements the screen stages at a time
 __device__ __forceinline__ float2 *stage_b(NaWarp &ws) { return reinterpret_cast<float2 *>(ws.t[0]); }
@@ -516,6 +517,12 @@ __device__ __forceinline__ void na_chunk(const Csr &A, const NoallocView &S, con
             hits = hit ? 1u : 0u;
         }
     }
+    const unsigned swept = __ballot_sync(kFull, small || mid);
+    const int swept_nnz = __reduce_add_sync(kFull, small || mid ? len : 0);
+    if (lane == 0) {
+        ws.rows += (unsigned)__popc(swept);
+        ws.nnz += (unsigned)swept_nnz;
+    }
     // round 1 takes every row; later a row without a changed variable was last
     // processed with these bounds and finds nothing
     bool exact = false;
@@ -547,6 +554,10 @@ __device__ __forceinline__ void na_long_row(const Csr &A, const NoallocView &S, 
     const int b = __ldg(A.row_ptr + row);
     const unsigned len = (unsigned)(__ldg(A.row_ptr + row + 1) - b);
     if (sparse && !__syncthreads_or(hit_strided(A, prev, b, len, threadIdx.x, kNaThreads))) return;
+    if (threadIdx.x == 0) {
+        wss[0].rows += 1;
+        wss[0].nnz += len;
+    }
     Scr c;
     scr_init(c);
     int hit = 0;
@@ -688,6 +699,7 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
     const int long_len = n_long == (int)st->n_long ? kLongRow : INT_MAX;
     int last_tight = 0;
     unsigned target = 0;  // grid barrier
+    if (lane == 0) ws.rows = ws.nnz = 0;
     for (int round = 1; round <= max_rounds; round++) {
         const int par = round & 1;
         const unsigned *prev = S.chg[par ^ 1];
@@ -740,6 +752,10 @@ __global__ void __launch_bounds__(kNaThreads, 2) k_noalloc_rounds(Csr A, Noalloc
         if (!last_tight || *((volatile int *)&st->flags.infeasible)) break;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) st->flags.change = last_tight;
+    if (lane == 0 && ws.rows) {
+        atomicAdd(&st->flags.rows_proc, ws.rows);
+        atomicAdd(&st->flags.nnz_proc, ws.nnz);
+    }
 }
 
 #define NA_CUDA(expr)                                                                   \
@@ -849,9 +865,9 @@ GDP_RETCODE propagate_noalloc(int m, int n, int nnz, const int *d_col, const int
         st->converged = (f.infeasible || !f.change) ? 1 : 0;
         st->kernel_launches = 3;
         st->changed_vars = f.changed_vars;
-        st->rows_processed = (long long)f.rounds * m;
-        st->nnz_processed = (long long)f.rounds * nnz;
-        st->bytes_algorithmic = (double)f.rounds * (12.0 * nnz + 20.0 * m + 36.0 * n);
+        st->rows_processed = (long long)f.rows_proc;
+        st->nnz_processed = (long long)f.nnz_proc;
+        st->bytes_algorithmic = 12.0 * (double)f.nnz_proc + 20.0 * (double)f.rows_proc + 36.0 * n * (double)f.rounds;
         st->total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
     return GDP_OKAY;

@@ -342,7 +342,9 @@ void gdp_mps_free(gdp_mps_problem *p);
  *   - Rows are summed left to right: results equal the context path's for rows
  *     up to its thread_row_max non-zeros.
  * stream: CUDA stream (NULL = legacy default stream); the call returns when the
- * propagation has finished. stats may be NULL (device_ms is not measured). */
+ * propagation has finished. stats may be NULL (device_ms is not measured; a row
+ * whose variables are looked up in the previous round's changes and found
+ * unchanged is not counted as processed). */
 #define GDP_NOALLOC_MAX_VARS (1 << 20)
 GDP_RETCODE gdp_propagate_noalloc(int n_cons, int n_vars, int nnz, const int *d_csr_col_indices,
                                   const int *d_csr_row_ptrs, const double *d_csr_vals,
