@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -1044,7 +1045,10 @@ GDP_RETCODE Context::rounds_cpu_loop(cudaStream_t s, int *launches, const std::f
         for (int spin = 1; mail[0] < round && e == cudaErrorNotReady; spin++)
             if (spin % 256 == 0) e = cudaStreamQuery(s);
         if (e != cudaErrorNotReady) GDP_CUDA(e);
-        if (mail[0] < round || !mail[1]) break;
+        if (mail[0] < round) break;
+        // the device wrote mail[1] before mail[0]; an Arm host may read them the other way round
+        std::atomic_thread_fence(std::memory_order_acquire);
+        if (!mail[1]) break;
     }
     *launches += queued;
     return GDP_OKAY;
