@@ -31,6 +31,7 @@
 #include <cstring>
 
 #include "gdp_learned.cuh"
+#include "gdp_sweep.h"
 
 namespace gdp {
 
@@ -142,32 +143,6 @@ __device__ __forceinline__ const DevProblem &unit_of(const BatchDev &B, UnitCach
         unit = u;
     }
     return *reinterpret_cast<const DevProblem *>(c.raw);
-}
-
-// Work item i of the full sweep: every unit's items are ordered heaviest first,
-// and one unit after the other would leave the last unit's heavy items to the
-// end of the phase. So the claims run through the units kSweepParts times, an
-// equal part of each unit's list at a time: part s of unit k holds as many items
-// as [prefix[k], prefix[k + 1]) holds numbers = s mod kSweepParts, which makes
-// the parts' prefixes functions of the units'. 24 mixed instances of up to 60,000 rows: 12.42 -> 11.53
-// ms (of 77 us of screening a round, 29 were the wait for the last items). Not
-// inlined: that cost every other batch 2%.
-constexpr int kSweepParts = 8;
-__device__ __noinline__ int2 sweep_item(const int *prefix, int nfs, int total, int i) {
-    constexpr int K = kSweepParts;
-    const int q = total / K, rem = total % K;
-    const int s = i < rem * (q + 1) ? i / (q + 1) : rem + (i - rem * (q + 1)) / q;
-    i -= s * q + min(s, rem);  // within part s
-    auto below = [&](int x) { return (x + K - 1 - s) / K; };           // numbers under x that are s mod K
-    auto before = [&](int x) { return x / K * s + min(s, x % K); };    // ... that are less than s mod K
-    int lo = 0, hi = nfs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (below(prefix[mid]) <= i) lo = mid;
-        else hi = mid - 1;
-    }
-    const int p0 = prefix[lo], p1 = prefix[lo + 1];
-    return make_int2(lo, before(p1) - before(p0) + i - below(p0));
 }
 
 // One warp builds the list of units swept in full in the next round, in unit
@@ -302,9 +277,9 @@ __global__ void __launch_bounds__(kCtaThreads, kCtas) k_batch_loop(BatchDev B) {
                 int u, it;
                 bool marked;
                 if (i < fs_items) {
-                    const int2 at = sweep_item(B.fs_prefix, nfs, fs_items, i);
-                    u = B.fs_unit[at.x];
-                    it = __ldg(B.units[u].items + at.y);
+                    const SweepItem at = sweep_item(B.fs_prefix, nfs, fs_items, i);
+                    u = B.fs_unit[at.unit];
+                    it = __ldg(B.units[u].items + at.item);
                     marked = false;
                 } else {
                     const unsigned long long e = ent[i - fs_items];
