@@ -2,6 +2,7 @@
 memory with the features, features and logits that start on any byte. Results are
 the bits of the plain call."""
 import ctypes as C
+import mmap
 
 import numpy as np
 import pytest
@@ -49,3 +50,19 @@ def test_arrays_off_their_alignment(n, x_by, z_by):
     _forward_at(m, n, xraw.ctypes.data + x0, zraw.ctypes.data + z0)
     assert zraw[z0:z0 + z.nbytes].tobytes() == z.tobytes()
     assert not zraw[:z0].any() and not zraw[z0 + z.nbytes:].any()
+
+
+# above 262,144 rows the first quarter's logits go by way of device memory
+@pytest.mark.parametrize("n", [262_143, 262_144, 262_145, 262_207, 1_000_003])
+@pytest.mark.parametrize("z_by", [0, 4, 2052])
+def test_split_logits_equal_chunks(n, z_by):
+    m = gdp.Mlp(seed=7)
+    x = _features(n, seed=9)
+    z = np.concatenate([m.forward(x[k:k + 100_000]) for k in range(0, n, 100_000)])
+    pages = mmap.mmap(-1, 4 * n + (1 << 17))  # pages that nothing has touched
+    raw = np.frombuffer(pages, np.uint8)
+    page = mmap.PAGESIZE
+    at = (-raw.ctypes.data) % page + z_by
+    _forward_at(m, n, x.ctypes.data, raw.ctypes.data + at)
+    assert raw[at:at + 4 * n].tobytes() == z.tobytes()
+    assert not raw[:at].any() and not raw[at + 4 * n:].any()
