@@ -1244,9 +1244,10 @@ __device__ __forceinline__ bool next_round_marked(const DevProblem &P, unsigned 
 // Any CTA that waits longer than `limit` clock64 cycles (or sees another
 // CTA's error) records kErrBarrierTimeout and every CTA leaves the round loop
 // at its next barrier. The default limit is 4e9 cycles, about 2 s at 2 GHz.
-// A single CTA needs no fence and keeps its L1 (100 rows: 0.23 -> 0.16 ms): what
-// it reads after its own atomics (the next bounds, the bitmap, round state) is
-// read past L1 everywhere.
+// A single CTA needs no fence and keeps its L1 (100 rows: 0.23 -> 0.16 ms):
+// __syncthreads makes what any of its threads wrote, by atomics or plain stores,
+// what all of them read afterwards, by plain loads too (the change bitmap of the
+// allocation-free loop, the drift bounds of split rows).
 __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *error, long long limit, unsigned &target) {
     __syncthreads();
     if (gridDim.x == 1) return *((volatile int *)error) == kErrNone;
