@@ -541,7 +541,8 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
     // SELL rows (1..Ls non-zeros) by lanes per row (widest first), then length
     // (longest first), stable: lanes_of never decreases with the length, so
     // this is a counting sort by length, longest first -- run in parallel over
-    // contiguous row chunks (per-chunk histograms keep it stable). Split rows
+    // contiguous row chunks (per-chunk histograms keep it stable; a team may have
+    // fewer threads than there are chunks). Split rows
     // (longer than Ls) are collected in row order and sorted by length.
     // pos_row: the original row of every position -- SELL positions first (the
     // row order the layout is built from), then the split rows; uploaded as is
@@ -562,13 +563,8 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         const size_t W = (size_t)lmax + 1;  // keys 0..lmax (0: empty rows, skipped)
         std::vector<int> hist((size_t)nt * W, 0);
         std::vector<int> nsplit(nt + 1, 0);
-#pragma omp parallel num_threads(nt)
-        {
-#ifdef _OPENMP
-            const int t = omp_get_thread_num();
-#else
-            const int t = 0;
-#endif
+#pragma omp parallel for schedule(static, 1) num_threads(nt)
+        for (int t = 0; t < nt; t++) {
             const int i0 = (int)((long long)m * t / nt), i1 = (int)((long long)m * (t + 1) / nt);
             int *h = &hist[(size_t)t * W];
             for (int i = i0; i < i1; i++) {
@@ -591,13 +587,8 @@ GDP_RETCODE Context::init(int m_, int n_, int nnz_, const int *col, const int *r
         for (int t = 0; t < nt; t++) nsplit[t + 1] += nsplit[t];
         n_sell_rows = acc;
         split_rows.resize(nsplit[nt]);
-#pragma omp parallel num_threads(nt)
-        {
-#ifdef _OPENMP
-            const int t = omp_get_thread_num();
-#else
-            const int t = 0;
-#endif
+#pragma omp parallel for schedule(static, 1) num_threads(nt)
+        for (int t = 0; t < nt; t++) {
             const int i0 = (int)((long long)m * t / nt), i1 = (int)((long long)m * (t + 1) / nt);
             int *h = &hist[(size_t)t * W];
             int sp = nsplit[t];
