@@ -1111,6 +1111,15 @@ GDP_RETCODE Context::run(const double *lb_in, const double *ub_in, double *lb_ou
                          cudaStream_t s, gdp_stats *st) {
     P.max_rounds = opts.max_rounds;
     certified = false;
+    // a call that fails leaves nothing of it running: its kernels use the caller's
+    // arrays and the words that a later CPU_LOOP call reads its rounds from
+    struct Drain {
+        cudaStream_t s;
+        bool on;
+        ~Drain() {
+            if (on) cudaStreamSynchronize(s);
+        }
+    } drain{s, true};
     GDP_CUDA(launch_start(P, lb_in, ub_in, vec_blocks, s));
     int launches = vec_blocks <= 32 ? 1 : 2;
     GDP_CUDA(cudaEventRecord(ev0, s));
@@ -1134,6 +1143,7 @@ GDP_RETCODE Context::run(const double *lb_in, const double *ub_in, double *lb_ou
     launches++;
     GDP_CUDA(cudaMemcpyAsync(h_flags, P.flags, sizeof(RoundFlags), cudaMemcpyDeviceToHost, s));
     GDP_CUDA(cudaStreamSynchronize(s));
+    drain.on = false;
     if (!P.learned && opts.sync_type == GPU_LOOP)
         launches += std::max(h_flags[0].rounds, 1) * (2 + (P.n_items > 0) + (P.n_mtiles > 0)) + 1;
     const RoundFlags &f = h_flags[0];
