@@ -108,10 +108,6 @@ __device__ __forceinline__ float f32_dn(long long b) {
 }
 constexpr float kUMargin = 1.00000095367431640625f;  // 1 + 2^-20
 
-// FP32 enclosure lo <= |a| (ub - lb) <= hi of one element (delta_box32).
-struct DeltaBox {
-    float lo, hi;
-};
 // Activity accumulator: the reference's computeActivities terms with integer
 // classification (no FP64 compares), plus the first maximum of the FP64
 // |a| (ub - lb) over the elements seen: km is its order key (order_key of its
@@ -362,21 +358,13 @@ __device__ __forceinline__ void scr_slack(const Scr &c, int n, double lhs, doubl
     mn_lo = fmin_nan(s_lo, t_lo);
     mn_hi = fminf(s_hi, t_hi);  // min(s, t) <= either upper end
 }
-// FP32 enclosure lo <= fl(|a| fl(ub - lb)) <= hi of one element from the
-// screen copies (the copies' errors as in scr_add, widened by 2^-20 relative
-// and 2^-80 absolute, which also covers the two FP64 roundings). A bound coded
-// +-inf is at least 1e20 in magnitude, so the lower end uses +-kInfF32Dn in its
-// place; NaN copies leave both ends NaN, and the comparisons then stay open.
-__device__ __forceinline__ DeltaBox delta_box32(float a, float2 b) {
-    const float aa = fabsf(a);
+// FP32 upper bound of fl(|a| fl(ub - lb)) of one element from the screen copies
+// (the copies' errors as in scr_add, widened by 2^-20 relative and 2^-80
+// absolute, which also covers the two FP64 roundings). NaN copies leave it NaN,
+// and the comparisons then stay open.
+__device__ __forceinline__ float delta_upper32(float a, float2 b) {
     const float d = __fsub_rn(b.y, b.x), w = __fadd_rn(fabsf(b.y), fabsf(b.x));
-    DeltaBox r;
-    r.hi = __fmaf_ru(__fmul_rn(aa, __fmaf_rn(w, 0x1p-21f, d)), kUMargin, 0x1p-80f);
-    const float ubl = fmin_nan(b.y, kInfF32Dn), lbh = fmax_nan(b.x, -kInfF32Dn);
-    const float dl = __fsub_rn(ubl, lbh), wl = __fadd_rn(fabsf(ubl), fabsf(lbh));
-    r.lo = __fmaf_rd(__fmul_rn(fmin_nan(aa, 0x1p40f), __fmaf_rn(wl, -0x1p-21f, dl)), 0.99999904632568359375f,
-                     -0x1p-80f);
-    return r;
+    return __fmaf_ru(__fmul_rn(fabsf(a), __fmaf_rn(w, 0x1p-21f, d)), kUMargin, 0x1p-80f);
 }
 
 // True when the reference's row test certainly skips the row, whatever order

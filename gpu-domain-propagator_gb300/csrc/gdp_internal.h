@@ -270,7 +270,7 @@ struct LayoutBuild {
     // row positions, built before the elements: SELL rows are sorted by
     // length, longest first, so the rows of one length L are the consecutive
     // positions from len_start[L] and their row-contiguous copies start at
-    // len_base[L] + (p - len_start[L]) * L
+    // len_base[L] + (p - len_start[L]) * (L rounded up to a multiple of 4)
     const double *lhs, *rhs;    // raw row sides (m)
     const int *len_start;       // lmax + 1 entries
     const long long *len_base;  // lmax + 1 entries

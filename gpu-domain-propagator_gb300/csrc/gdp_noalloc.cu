@@ -543,7 +543,6 @@ struct NaBlock {
     int p[kNaWarps];
     int hit[kNaWarps];
     int decision;
-    float slack_lo;
     ExactSums sums;
     double s, t;
 };

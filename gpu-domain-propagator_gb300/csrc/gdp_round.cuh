@@ -360,21 +360,8 @@ struct LearnSmem {
     unsigned long long marked;  // marked SELL rows met by this warp in the current phase
 };
 
-// Combines the partial accumulators of a group of g lanes (g a power of two,
+// Combines the partial screens of a group of g lanes (g a power of two,
 // warp-uniform) into its first lane: shuffle tree with offsets g/2, ..., 1.
-__device__ __forceinline__ void acc_group_reduce(Acc &s, int g) {
-    for (int off = g >> 1; off > 0; off >>= 1) {
-        Acc o;
-        o.minact = __shfl_down_sync(kFull, s.minact, off);
-        o.maxact = __shfl_down_sync(kFull, s.maxact, off);
-        o.minf = __shfl_down_sync(kFull, s.minf, off);
-        o.maxf = __shfl_down_sync(kFull, s.maxf, off);
-        o.km = __shfl_down_sync(kFull, s.km, off);
-        o.p = __shfl_down_sync(kFull, s.p, off);
-        acc_combine(s, o);
-    }
-}
-
 __device__ __forceinline__ void scr_group_reduce(Scr &c, int g) {
     for (int off = g >> 1; off > 0; off >>= 1) {
         Scr o;
@@ -519,8 +506,9 @@ __device__ __forceinline__ int pack_inf(const Scr &c) { return min(c.minf, 3) | 
 // l >> lg and its elements sub, sub+g, ... (sub = l & (g-1)), stored
 // column-major (step i of lane l at slice_ptr[slice] + 32 i + l).
 // The FP32 screen runs here; rows it cannot skip are queued for the exact-rows
-// phase (kDefer) or take the exact pass in place (batch members, and contexts
-// with a warp for each slice of nothing but one-lane rows).
+// phase (kDefer) or take the exact pass in place (batch members, and contexts of
+// nothing but one-lane rows with at most three slices per warp, or with up to four
+// warps per slice: `part` of `parts`).
 template <int kRec, bool kDefer>
 __device__ __forceinline__ void sell_slice(const DevProblem &P, int slice, int lane, int round, bool marked,
                                            int *change, unsigned *tight_ctr, WarpSmem &ws, int par = 0, int part = 0,
@@ -846,7 +834,7 @@ __device__ __noinline__ void split_row_candidates(const DevProblem &P, int row, 
         unsigned todo = 0u;  // my elements that may be candidates
 #pragma unroll
         for (int i = 0; i < kSteps; i++)
-            if (j[i] >= 0 && !(delta_box32(a[i], bb[i]).hi <= cut)) todo |= 1u << i;
+            if (j[i] >= 0 && !(delta_upper32(a[i], bb[i]) <= cut)) todo |= 1u << i;
 #pragma unroll 1
         for (int i = 0; i < kSteps; i++) {
             const bool on = (todo >> i) & 1u;
