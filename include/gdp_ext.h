@@ -98,7 +98,8 @@ const char *gdp_last_error(void);
 /* Device memory released by destroyed contexts and batches stays cached (up
  * to 32 GiB) for later contexts of similar size, so that repeated
  * create / destroy cycles allocate nothing; a failed allocation frees the
- * cache and retries. This frees the cache now. */
+ * cache and retries. So do the samples of gdp_mlp_* calls, and up to 16 sets of
+ * streams, events and 1 MB of page-locked memory. This frees all of it now. */
 GDP_RETCODE gdp_release_cached_memory(void);
 
 /* Uploads a MIP (host CSR arrays, reference argument meaning) and builds the
@@ -203,7 +204,11 @@ GDP_RETCODE gdp_mlp_destroy(gdp_mlp *m);
 GDP_RETCODE gdp_mlp_get_params(const gdp_mlp *m, float *params);
 /* Sets the FP32 master parameters (and resets the optimizer state). */
 GDP_RETCODE gdp_mlp_set_params(gdp_mlp *m, const float *params);
-/* logits[i] of the n x 16 host features x (rounded to BF16 on the device). */
+/* logits[i] of the n x 16 host features x (rounded to BF16 on the device). The
+ * arrays may start anywhere and share memory: features that are 16-byte aligned
+ * are read, and logits that are 4-byte aligned written, where they are by GPUs
+ * with coherent access to host memory, others are copied. A call that fails before its
+ * kernels run leaves the logits as they were. */
 GDP_RETCODE gdp_mlp_forward(gdp_mlp *m, int n, const float *x, float *logits);
 /* Gradient (GDP_MLP_PARAMS floats) and value of the weighted binary
  * cross-entropy sum_i w_i BCE(sigmoid(z_i), y_i) / sum_i w_i at the current
