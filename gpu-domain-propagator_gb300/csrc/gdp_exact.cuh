@@ -45,7 +45,7 @@ struct ExactSmem {
     int cand_k[kCandCap];
     int src[kItemRows];                 // element index of the row's flat index 0
     unsigned char cand_s[kCandCap];     // row slot
-    unsigned char info[kItemRows];      // bits 0, 1: usable sides; 2, 3: minf; 4, 5: maxf; 6: candidates wanted
+    unsigned char info[kItemRows];      // bits 0, 1: usable sides; 2, 3: minf; 4, 5: maxf; 6: candidates wanted; 7: lhs is -0.0
 };
 
 // The rows of an item: lane r < n holds row r (in is set for those lanes).
@@ -167,8 +167,10 @@ __device__ __forceinline__ void exact_push(const T &t, ExactSmem &xs, ExactQueue
     }
     const unsigned bu = __ballot_sync(kFull, uo), bl = __ballot_sync(kFull, lo);
     const unsigned lt = (1u << lane) - 1u;
-    // lhs - maxact is -(maxact - lhs) (round-to-nearest is symmetric), +0.0 when they are equal
-    const double surplus = __longlong_as_double((dbits(u) << 1) ? dbits(u) ^ (1LL << 63) : 0LL);
+    // lhs - maxact is -(maxact - lhs) (round-to-nearest is symmetric); when they are equal
+    // it is +0.0, or -0.0 if lhs is (a sum that starts at +0.0 never is)
+    const double surplus = __longlong_as_double((dbits(u) << 1) ? dbits(u) ^ (1LL << 63)
+                                                                : (long long)((unsigned long long)(info & 128u) << 56));
     if (bu) {
         if (uo)
             xs.div[Q.cnt + __popc(bu & lt)] =
@@ -403,7 +405,8 @@ __device__ __forceinline__ void exact_candidates(const T &t, ExactSmem &xs, Exac
         xs.slack[lane] = s;
         xs.nsur[lane] = u;
         xs.info[lane] = (unsigned char)((rhs_ok ? 1 : 0) | (lhs_ok ? 2 : 0) | min(R.minf, 3) << 2 |
-                                        min(R.maxf, 3) << 4 | (go ? 64 : 0));
+                                        min(R.maxf, 3) << 4 | (go ? 64 : 0) |
+                                        (dbits(R.lhs) == (long long)(1ULL << 63) ? 128 : 0));
     }
     __syncwarp();
     if (cand <= kCandCap) {
