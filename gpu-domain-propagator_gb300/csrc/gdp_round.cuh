@@ -1019,12 +1019,13 @@ __device__ __forceinline__ void split_exact(const DevProblem &P, int t, int lane
     if (pb < pe) split_row_candidates<kRec>(P, row, pb, pe, s, lane, change, tight_ctr, ws);
 }
 
-// Adds a thread's committed-change count to the round flags, one atomic per warp.
+// Adds the warp's committed-change counts to the round flags, one atomic per warp.
+// Every lane of the warp calls it, from wherever its loop left it.
 __device__ __forceinline__ void flush_changed(const DevProblem &P, unsigned long long changed) {
-    const unsigned active = __activemask();
+    __syncwarp();
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) changed += __shfl_down_sync(active, changed, off);
-    if ((threadIdx.x & 31) == __ffs(active) - 1 && changed) atomicAdd(&P.flags[0].changed_vars, changed);
+    for (int off = 16; off > 0; off >>= 1) changed += __shfl_down_sync(kFull, changed, off);
+    if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&P.flags[0].changed_vars, changed);
 }
 
 // Commit changed variables nxt -> cur, apply the infeasibility rules (a row
