@@ -18,8 +18,8 @@
 //     certified fixpoint of the same problem (every other row is at its
 //     fixpoint already and would find nothing).
 // The round loop runs in one cooperative kernel (grid barriers between the
-// phases, bounded waits) and the whole device part of a call is captured once
-// into a CUDA graph and replayed.
+// phases, bounded waits) and the whole device part of a call is built once as a
+// CUDA graph and replayed.
 //
 // Reference: the reference propagates one problem per call
 // (include/interface.h:10-251); its GPU round loop is
@@ -31,6 +31,7 @@
 #include <cstring>
 
 #include "gdp_learned.cuh"
+#include "gdp_sequence.h"
 #include "gdp_sweep.h"
 
 namespace gdp {
@@ -560,23 +561,17 @@ int batch_occupancy(int *blocks_per_sm, bool learned, bool little) {
 
 int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub, double *lb_out,
                  double *ub_out, const long long *var_base, int max_unit_n, const double2 *ref,
-                 const int *seed_mode, bool learned, bool little, cudaStream_t s) {
+                 const int *seed_mode, bool learned, bool little, Sequence &seq) {
     const dim3 vgrid((unsigned)std::max(1, std::min((max_unit_n + 255) / 256, 64)), (unsigned)B.n_units);
-    k_batch_init<<<vgrid, 256, 0, s>>>(B, lb, ub, var_base);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    if (ref) {
-        k_batch_seed_marks<<<vgrid, 256, 0, s>>>(B, ref, seed_mode);
-        if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-    }
-    k_batch_plan<<<1, kCtaThreads, 0, s>>>(B, seed_mode);
-    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
     BatchDev Bc = B;
-    void *args[] = {&Bc};
-    e = cudaLaunchCooperativeKernel(batch_loop(learned, little), dim3(grid), dim3(kCtaThreads), args, kCtaSmem, s);
-    if (e != cudaSuccess) return (int)e;
-    k_batch_fini<<<vgrid, 256, 0, s>>>(B, lb_out, ub_out, var_base);
-    return (int)cudaGetLastError();
+    void *init[] = {&Bc, &lb, &ub, &var_base}, *seed[] = {&Bc, &ref, &seed_mode}, *plan[] = {&Bc, &seed_mode},
+         *loop[] = {&Bc}, *fini[] = {&Bc, &lb_out, &ub_out, &var_base};
+    cudaError_t e = seq.kernel((const void *)k_batch_init, vgrid, 256, init, 0);
+    if (e == cudaSuccess && ref) e = seq.kernel((const void *)k_batch_seed_marks, vgrid, 256, seed, 0);
+    if (e == cudaSuccess) e = seq.kernel((const void *)k_batch_plan, 1, kCtaThreads, plan, 0);
+    if (e == cudaSuccess) e = seq.kernel(batch_loop(learned, little), grid, kCtaThreads, loop, kCtaSmem, true);
+    if (e == cudaSuccess) e = seq.kernel((const void *)k_batch_fini, vgrid, 256, fini, 0);
+    return (int)e;
 }
 
 }  // namespace gdp

@@ -34,7 +34,7 @@ struct BatchDev {
 
 int launch_batch(const BatchDev &B, int grid, const double *lb, const double *ub, double *lb_out,
                  double *ub_out, const long long *var_base, int max_unit_n, const double2 *ref,
-                 const int *seed_mode, bool learned, bool little, cudaStream_t s);
+                 const int *seed_mode, bool learned, bool little, Sequence &seq);
 int batch_occupancy(int *blocks_per_sm, bool learned, bool little);
 
 class Batch {
@@ -57,8 +57,8 @@ public:
 
     int n_units = 0;
     bool nodes = false;
-    bool use_graph = true;   // capture the device part once and replay it
-    bool graph_ok = false;   // the graph was captured and is used
+    bool use_graph = true;   // build the device part as a graph once and replay it
+    bool graph_ok = false;   // the graph was built and is used
     int grid = 1;
     bool little_ = false;  // little work in a round
     int max_rounds = GDP_MAX_NUM_ROUNDS;
@@ -66,7 +66,8 @@ public:
 private:
     GDP_RETCODE finish_init(int device, int ctas_per_sm);
     GDP_RETCODE size_grid();
-    GDP_RETCODE enqueue(cudaStream_t s);
+    GDP_RETCODE enqueue(Sequence &seq);
+    GDP_RETCODE build_graph();
     void copy_in(const double *const *lbs, const double *const *ubs);
     void copy_out(double *const *lbs, double *const *ubs);
 

@@ -1,6 +1,6 @@
 // gdp_batch_host.cu -- host side of the batched engine: builds the units
 // (per-instance layouts, or per-node state over one shared layout), the batch
-// queues, and runs a batch as one captured CUDA graph.
+// queues, and runs a batch as one CUDA graph.
 #include <algorithm>
 #include <chrono>
 #include <climits>
@@ -9,6 +9,7 @@
 #include <string>
 
 #include "gdp_batch.h"
+#include "gdp_sequence.h"
 
 namespace gdp {
 
@@ -251,7 +252,7 @@ GDP_RETCODE Batch::set_model(const Mlp *m, float threshold, int min_len) {
                               cudaMemcpyHostToDevice, stream_));
     GDP_BCUDA(cudaStreamSynchronize(stream_));
     if (size_grid() != GDP_OKAY) return GDP_ERROR;
-    // the captured graph holds the other loop instantiation and grid: capture again
+    // the graph holds the other loop instantiation and grid: it is built again
     if (graph_exec_) { cudaGraphExecDestroy(graph_exec_); graph_exec_ = nullptr; }
     if (graph_) { cudaGraphDestroy(graph_); graph_ = nullptr; }
     graph_failed_ = false;
@@ -295,32 +296,34 @@ void Batch::copy_out(double *const *lbs, double *const *ubs) {
     });
 }
 
-// The device part of one batch call, in stream order.
-GDP_RETCODE Batch::enqueue(cudaStream_t s) {
-    const size_t vbytes = sizeof(double) * (size_t)total_vars_;
-    if (vbytes) {
-        GDP_BCUDA(cudaMemcpyAsync(d_lb_, h_lb_, vbytes, cudaMemcpyHostToDevice, s));
-        GDP_BCUDA(cudaMemcpyAsync(d_ub_, h_ub_, vbytes, cudaMemcpyHostToDevice, s));
-    }
-    GDP_BCUDA(cudaMemcpyAsync(d_seed_mode_, h_seed_, sizeof(int) * (size_t)n_units, cudaMemcpyHostToDevice, s));
-    GDP_BCUDA(cudaMemcpyAsync(d_flags_, h_flags_init_, sizeof(RoundFlags) * 3 * (size_t)n_units,
-                              cudaMemcpyHostToDevice, s));
-    GDP_BCUDA(cudaMemsetAsync(B_.ctr, 0, sizeof(unsigned) * 8, s));
-    GDP_BCUDA(cudaMemsetAsync(B_.tail, 0, sizeof(unsigned) * 4, s));
-    GDP_BCUDA(cudaMemsetAsync(B_.barrier, 0, sizeof(unsigned) * 2, s));
-    GDP_BCUDA(cudaMemsetAsync(B_.error, 0, sizeof(int) * 3, s));
-    // external records: inside a stream capture they become graph event nodes
-    GDP_BCUDA(cudaEventRecordWithFlags(ev0_, s, cudaEventRecordExternal));
+// The device part of one batch call, in order.
+GDP_RETCODE Batch::enqueue(Sequence &seq) {
+    const size_t vbytes = sizeof(double) * (size_t)total_vars_, units = (size_t)n_units;
+    const auto up = cudaMemcpyHostToDevice, down = cudaMemcpyDeviceToHost;
+    GDP_BCUDA(seq.copy(d_lb_, h_lb_, vbytes, up));
+    GDP_BCUDA(seq.copy(d_ub_, h_ub_, vbytes, up));
+    GDP_BCUDA(seq.copy(d_seed_mode_, h_seed_, sizeof(int) * units, up));
+    GDP_BCUDA(seq.copy(d_flags_, h_flags_init_, sizeof(RoundFlags) * 3 * units, up));
+    GDP_BCUDA(seq.clear(B_.ctr, sizeof(unsigned) * 8));
+    GDP_BCUDA(seq.clear(B_.tail, sizeof(unsigned) * 4));
+    GDP_BCUDA(seq.clear(B_.barrier, sizeof(unsigned) * 2));
+    GDP_BCUDA(seq.clear(B_.error, sizeof(int) * 3));
+    GDP_BCUDA(seq.record(ev0_));
     GDP_BCUDA((cudaError_t)launch_batch(B_, grid, d_lb_, d_ub_, d_lb_, d_ub_, d_var_base_, max_unit_n_, ref_,
-                                        d_seed_mode_, learned_, little_, s));
-    GDP_BCUDA(cudaEventRecordWithFlags(ev1_, s, cudaEventRecordExternal));
-    if (vbytes) {
-        GDP_BCUDA(cudaMemcpyAsync(h_lb_, d_lb_, vbytes, cudaMemcpyDeviceToHost, s));
-        GDP_BCUDA(cudaMemcpyAsync(h_ub_, d_ub_, vbytes, cudaMemcpyDeviceToHost, s));
-    }
-    GDP_BCUDA(cudaMemcpyAsync(h_flags_, d_flags_, sizeof(RoundFlags) * 3 * (size_t)n_units,
-                              cudaMemcpyDeviceToHost, s));
-    GDP_BCUDA(cudaMemcpyAsync(h_rounds_, B_.error, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));
+                                        d_seed_mode_, learned_, little_, seq));
+    GDP_BCUDA(seq.record(ev1_));
+    GDP_BCUDA(seq.copy(h_lb_, d_lb_, vbytes, down));
+    GDP_BCUDA(seq.copy(h_ub_, d_ub_, vbytes, down));
+    GDP_BCUDA(seq.copy(h_flags_, d_flags_, sizeof(RoundFlags) * 3 * units, down));
+    GDP_BCUDA(seq.copy(h_rounds_, B_.error, sizeof(int) * 2, down));
+    return GDP_OKAY;
+}
+
+GDP_RETCODE Batch::build_graph() {
+    GDP_BCUDA(cudaGraphCreate(&graph_, 0));
+    Sequence nodes(graph_);
+    if (enqueue(nodes) != GDP_OKAY) return GDP_ERROR;
+    GDP_BCUDA(cudaGraphInstantiate(&graph_exec_, graph_, 0));
     return GDP_OKAY;
 }
 
@@ -343,28 +346,19 @@ GDP_RETCODE Batch::propagate(const double *const *lbs_in, const double *const *u
     // fixpoint when its last propagation certified one; otherwise they sweep
     const int seed = nodes && base_ && base_->certified ? 1 : 0;
     for (int u = 0; u < n_units; u++) h_seed_[u] = nodes ? seed : seed_mode_[u];
-    if (use_graph && !graph_exec_ && !graph_failed_) {
-        cudaGraph_t g = nullptr;
-        bool ok = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        const bool enq = ok && enqueue(stream_) == GDP_OKAY;
-        const cudaError_t ec = cudaStreamEndCapture(stream_, &g);
-        ok = ok && enq && ec == cudaSuccess && g;
-        cudaGraphExec_t ge = nullptr;
-        if (ok) ok = cudaGraphInstantiate(&ge, g, 0) == cudaSuccess;
-        if (ok) {
-            graph_ = g;
-            graph_exec_ = ge;
-        } else {
-            if (g) cudaGraphDestroy(g);
-            graph_failed_ = true;  // launch the same sequence directly from now on
-        }
+    if (use_graph && !graph_exec_ && !graph_failed_ && build_graph() != GDP_OKAY) {
+        if (graph_) cudaGraphDestroy(graph_);
+        graph_ = nullptr;
+        graph_exec_ = nullptr;
+        graph_failed_ = true;  // the same sequence goes to the stream from now on
         cudaGetLastError();
     }
     graph_ok = graph_exec_ != nullptr;
     if (graph_ok) {
         GDP_BCUDA(cudaGraphLaunch(graph_exec_, stream_));
-    } else if (enqueue(stream_) != GDP_OKAY) {
-        return GDP_ERROR;
+    } else {
+        Sequence direct(stream_);
+        if (enqueue(direct) != GDP_OKAY) return GDP_ERROR;
     }
     GDP_BCUDA(cudaStreamSynchronize(stream_));
     if (h_rounds_[0] != kErrNone) {

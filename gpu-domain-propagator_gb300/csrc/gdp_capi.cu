@@ -295,7 +295,7 @@ GDP_RETCODE gdp_context_set_options(gdp_context *ctx, int max_rounds, int sync_t
     ctx->impl.opts.max_rounds = max_rounds > 0 ? max_rounds : GDP_MAX_NUM_ROUNDS;
     ctx->impl.opts.sync_type = sync_type;
     ctx->impl.P.max_rounds = ctx->impl.opts.max_rounds;
-    // the GPU_LOOP graph holds the round cap in its captured kernel arguments
+    // the GPU_LOOP graph holds the round cap in its kernel arguments
     if (ctx->impl.graph_exec) { cudaGraphExecDestroy(ctx->impl.graph_exec); ctx->impl.graph_exec = nullptr; }
     if (ctx->impl.graph) { cudaGraphDestroy(ctx->impl.graph); ctx->impl.graph = nullptr; }
     return GDP_OKAY;

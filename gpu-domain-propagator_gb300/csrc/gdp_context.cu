@@ -33,6 +33,7 @@
 #include "gdp_context.h"
 #include "gdp_device.cuh"
 #include "gdp_learned.h"
+#include "gdp_sequence.h"
 
 namespace gdp {
 
@@ -1047,13 +1048,18 @@ GDP_RETCODE Context::rounds_cpu_loop(cudaStream_t s, int *launches, const std::f
 }
 
 // GPU_LOOP: one CUDA graph whose conditional WHILE node repeats the round's
-// phase kernels until the condition kernel clears it -- the device-driven loop
-// the reference built with dynamic parallelism (src/kernels/atomic_kernel.cuh:452-503).
-GDP_RETCODE Context::build_graph(cudaStream_t s) {
-    cudaGraph_t g = nullptr;
-    GDP_CUDA(cudaGraphCreate(&g, 0));
+// phase kernels until the finalize kernel clears its condition -- the device-driven
+// loop the reference built with dynamic parallelism (src/kernels/atomic_kernel.cuh:452-503).
+GDP_RETCODE Context::build_graph() {
+    struct Graph {  // destroyed unless it is complete
+        cudaGraph_t g = nullptr;
+        ~Graph() {
+            if (g) cudaGraphDestroy(g);
+        }
+    } made;
+    GDP_CUDA(cudaGraphCreate(&made.g, 0));
     cudaGraphConditionalHandle h;
-    GDP_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1u, cudaGraphCondAssignDefault));
+    GDP_CUDA(cudaGraphConditionalHandleCreate(&h, made.g, 1u, cudaGraphCondAssignDefault));
     // cudaGraphNodeParams has no usable default constructor in C++: zero a raw buffer
     alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
     std::memset(cp_buf, 0, sizeof(cp_buf));
@@ -1063,39 +1069,17 @@ GDP_RETCODE Context::build_graph(cudaStream_t s) {
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
     cudaGraphNode_t node;
-    GDP_CUDA(cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    cudaStream_t cs;
-    GDP_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    GDP_CUDA(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    int rc = launch_activity_phase(P, act_blocks, cs);
-    if (!rc) rc = launch_candidate_phase(P, cand_blocks, cs);
-    if (!rc) rc = launch_exact_phase(P, cand_blocks, cs);
-    if (!rc) rc = launch_finalize(P, (unsigned long long)h, vec_blocks, cs);
-    cudaGraph_t captured = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(cs, &captured);
-    cudaStreamDestroy(cs);
-    (void)s;
-    if (rc || ec != cudaSuccess) {
-        cudaGraphDestroy(g);
-        set_error(std::string("GPU_LOOP graph capture failed: ") +
-                  cudaGetErrorString(rc ? (cudaError_t)rc : ec));
-        return GDP_ERROR;
-    }
-    cudaGraphExec_t ge = nullptr;
-    const cudaError_t ei = cudaGraphInstantiate(&ge, g, 0);
-    if (ei != cudaSuccess) {
-        cudaGraphDestroy(g);
-        set_error(std::string("GPU_LOOP graph instantiation failed: ") + cudaGetErrorString(ei));
-        return GDP_ERROR;
-    }
-    graph = g;
-    graph_exec = ge;
+    GDP_CUDA(cudaGraphAddNode(&node, made.g, nullptr, nullptr, 0, &cp));
+    Sequence body(cp.conditional.phGraph_out[0]);
+    GDP_CUDA(add_round(P, (unsigned long long)h, act_blocks, cand_blocks, vec_blocks, body));
+    GDP_CUDA(cudaGraphInstantiate(&graph_exec, made.g, 0));
+    graph = made.g;
+    made.g = nullptr;
     return GDP_OKAY;
 }
 
 GDP_RETCODE Context::rounds_gpu_loop(cudaStream_t s) {
-    if (!graph_exec && build_graph(s) != GDP_OKAY) return GDP_ERROR;
+    if (!graph_exec && build_graph() != GDP_OKAY) return GDP_ERROR;
     GDP_CUDA(launch_round_begin(P, s));
     GDP_CUDA(cudaGraphLaunch(graph_exec, s));
     return GDP_OKAY;

@@ -113,7 +113,7 @@ public:
 private:
     GDP_RETCODE run(const double *lb_in, const double *ub_in, double *lb_out, double *ub_out,
                     cudaStream_t s, gdp_stats *st);
-    GDP_RETCODE build_graph(cudaStream_t s);
+    GDP_RETCODE build_graph();
     // meanwhile: host work to do once the first rounds are queued
     GDP_RETCODE rounds_cpu_loop(cudaStream_t s, int *launches, const std::function<void()> &meanwhile);
     GDP_RETCODE rounds_gpu_loop(cudaStream_t s);

@@ -222,6 +222,8 @@ constexpr long long kLongSpinLimit = 1LL << 40;
 constexpr int kWarpsPerCta = 8;
 constexpr int kCtaThreads = 32 * kWarpsPerCta;
 
+class Sequence;
+
 // Launch helpers (gdp_round.cu). All return the cudaError_t of the launch.
 // Round state and bounds at the start of a propagation from lb / ub (two
 // kernels, one for small problems), and the result (unless the rounds ended
@@ -229,10 +231,9 @@ constexpr int kCtaThreads = 32 * kWarpsPerCta;
 int launch_start(const DevProblem &P, const double *lb, const double *ub, int blocks, cudaStream_t s);
 int launch_finish(const DevProblem &P, double *lb, double *ub, int blocks, cudaStream_t s);
 int launch_round_begin(const DevProblem &P, cudaStream_t s);
-int launch_activity_phase(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_candidate_phase(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_exact_phase(const DevProblem &P, int blocks, cudaStream_t s);
-int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, cudaStream_t s);
+// The phase kernels of one round; the last one sets the condition `handle`.
+int add_round(const DevProblem &P, unsigned long long handle, int act_blocks, int cand_blocks, int vec_blocks,
+              Sequence &seq);
 // Rounds first .. last; mail (may be null) is host memory that receives {round,
 // whether another one follows} at the end of the launch. cta_warps: 4, 8 or 16
 // warps per CTA.

@@ -6,6 +6,7 @@
 #include <cstddef>
 
 #include "gdp_round.cuh"
+#include "gdp_sequence.h"
 
 namespace gdp {
 
@@ -333,26 +334,17 @@ int launch_round_begin(const DevProblem &P, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int launch_activity_phase(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (P.n_items == 0) return 0;
-    k_activity<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
-    return (int)cudaGetLastError();
-}
-
-int launch_candidate_phase(const DevProblem &P, int blocks, cudaStream_t s) {
-    k_candidates<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
-    return (int)cudaGetLastError();
-}
-
-int launch_exact_phase(const DevProblem &P, int blocks, cudaStream_t s) {
-    if (P.n_mtiles == 0) return 0;
-    k_exact<<<blocks, kCtaThreads, kCtaSmem, s>>>(P);
-    return (int)cudaGetLastError();
-}
-
-int launch_finalize(const DevProblem &P, unsigned long long handle, int blocks, cudaStream_t s) {
-    k_finalize<<<blocks, 256, 0, s>>>(P, (cudaGraphConditionalHandle)handle);
-    return (int)cudaGetLastError();
+int add_round(const DevProblem &P, unsigned long long handle, int act_blocks, int cand_blocks, int vec_blocks,
+              Sequence &seq) {
+    DevProblem Pc = P;
+    cudaGraphConditionalHandle h = (cudaGraphConditionalHandle)handle;
+    void *args[] = {&Pc, &h};
+    cudaError_t e = cudaSuccess;
+    if (P.n_items) e = seq.kernel((const void *)k_activity, act_blocks, kCtaThreads, args, kCtaSmem);
+    if (e == cudaSuccess) e = seq.kernel((const void *)k_candidates, cand_blocks, kCtaThreads, args, kCtaSmem);
+    if (e == cudaSuccess && P.n_mtiles) e = seq.kernel((const void *)k_exact, cand_blocks, kCtaThreads, args, kCtaSmem);
+    if (e == cudaSuccess) e = seq.kernel((const void *)k_finalize, vec_blocks, 256, args, 0);
+    return (int)e;
 }
 
 namespace {

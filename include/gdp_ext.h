@@ -147,7 +147,7 @@ GDP_RETCODE gdp_propagate_once(int n_cons, int n_vars, int nnz, const int *csr_c
  * propagates one problem per call) ----------------------------------------
  * A batch propagates many problems ("instances"), or many bound vectors of one
  * context's problem ("nodes", e.g. branch-and-bound children), together in
- * one persistent cooperative launch that is captured once into a CUDA graph
+ * one persistent cooperative launch that is built once into a CUDA graph
  * and replayed. Every member gets the bounds, round count and infeasibility
  * verdict that a single-problem propagation of it returns; members that
  * converge early stop costing work. */
@@ -180,7 +180,7 @@ GDP_RETCODE gdp_batch_propagate_into(gdp_batch *b, const double *const *lbs_in, 
                                      double *const *lbs_out, double *const *ubs_out, gdp_stats *member_stats,
                                      gdp_stats *total);
 
-/* 1 if the batch runs as a captured CUDA graph (known after the first
+/* 1 if the batch runs as a CUDA graph (known after the first
  * propagation), 0 if it launches the same sequence directly. */
 int gdp_batch_uses_graph(const gdp_batch *b);
 
