@@ -22,25 +22,9 @@ struct gdp_batch {
     gdp::Batch impl;
 };
 
-namespace {
+using gdp::guarded;
 
-// The reference's CALL_AND_HANDLE (src/interface.cu:7-16): exceptions become
-// GDP_ERROR; here with the message kept for gdp_last_error().
-template <class F>
-GDP_RETCODE guarded(F &&f) {
-    try {
-        return f();
-    } catch (const std::bad_alloc &) {
-        gdp::set_error("host allocation failed");
-        return GDP_ERROR;
-    } catch (const std::exception &e) {
-        gdp::set_error(e.what());
-        return GDP_ERROR;
-    } catch (...) {
-        gdp::set_error("unknown exception");
-        return GDP_ERROR;
-    }
-}
+namespace {
 
 GDP_RETCODE propagate_once_impl(int n_cons, int n_vars, int nnz, const int *col, const int *row_ptr,
                                 const double *val, const double *lhs, const double *rhs,

@@ -3,8 +3,10 @@
 
 #include <cuda_runtime.h>
 
+#include <exception>
 #include <functional>
 #include <initializer_list>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -66,6 +68,24 @@ GDP_RETCODE autotune_clear_cache();
 
 GDP_RETCODE validate_csr(int m, int n, int nnz, const int *col, const int *row_ptr,
                          const double *val, const int *vartype);
+
+// The reference's CALL_AND_HANDLE (src/interface.cu:7-16): exceptions become
+// GDP_ERROR; here with the message kept for gdp_last_error().
+template <class F>
+GDP_RETCODE guarded(F &&f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc &) {
+        set_error("host allocation failed");
+        return GDP_ERROR;
+    } catch (const std::exception &e) {
+        set_error(e.what());
+        return GDP_ERROR;
+    } catch (...) {
+        set_error("unknown exception");
+        return GDP_ERROR;
+    }
+}
 
 class Context {
 public:

@@ -746,7 +746,10 @@ GDP_RETCODE gdp_mlp_create(unsigned long long seed, int device, gdp_mlp **out) {
     *out = nullptr;
     gdp_mlp *m = new (std::nothrow) gdp_mlp();
     if (!m) { gdp::set_error("host allocation failed"); return GDP_ERROR; }
-    if (m->impl.init(seed, device) != GDP_OKAY) { delete m; return GDP_ERROR; }
+    if (gdp::guarded([&]() -> GDP_RETCODE { return m->impl.init(seed, device); }) != GDP_OKAY) {
+        delete m;
+        return GDP_ERROR;
+    }
     *out = m;
     return GDP_OKAY;
 }
@@ -758,29 +761,29 @@ GDP_RETCODE gdp_mlp_destroy(gdp_mlp *m) {
 
 GDP_RETCODE gdp_mlp_get_params(const gdp_mlp *m, float *params) {
     if (!m) { gdp::set_error("null model"); return GDP_ERROR; }
-    return m->impl.get(params);
+    return gdp::guarded([&]() -> GDP_RETCODE { return m->impl.get(params); });
 }
 
 GDP_RETCODE gdp_mlp_set_params(gdp_mlp *m, const float *params) {
     if (!m) { gdp::set_error("null model"); return GDP_ERROR; }
-    return m->impl.set(params);
+    return gdp::guarded([&]() -> GDP_RETCODE { return m->impl.set(params); });
 }
 
 GDP_RETCODE gdp_mlp_forward(gdp_mlp *m, int n, const float *x, float *logits) {
     if (!m) { gdp::set_error("null model"); return GDP_ERROR; }
-    return m->impl.forward(n, x, logits);
+    return gdp::guarded([&]() -> GDP_RETCODE { return m->impl.forward(n, x, logits); });
 }
 
 GDP_RETCODE gdp_mlp_gradient(gdp_mlp *m, int n, const float *x, const float *y, const float *w, float *grad,
                              float *loss) {
     if (!m) { gdp::set_error("null model"); return GDP_ERROR; }
-    return m->impl.gradient(n, x, y, w, grad, loss);
+    return gdp::guarded([&]() -> GDP_RETCODE { return m->impl.gradient(n, x, y, w, grad, loss); });
 }
 
 GDP_RETCODE gdp_mlp_train(gdp_mlp *m, int n, const float *x, const float *y, const float *w, int epochs, int batch,
                           float lr, unsigned long long seed, float *final_loss) {
     if (!m) { gdp::set_error("null model"); return GDP_ERROR; }
-    return m->impl.train(n, x, y, w, epochs, batch, lr, seed, final_loss);
+    return gdp::guarded([&]() -> GDP_RETCODE { return m->impl.train(n, x, y, w, epochs, batch, lr, seed, final_loss); });
 }
 
 }  // extern "C"

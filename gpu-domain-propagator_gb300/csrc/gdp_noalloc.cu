@@ -880,13 +880,10 @@ extern "C" GDP_RETCODE gdp_propagate_noalloc(int n_cons, int n_vars, int nnz, co
                                              const double *d_lhss, const double *d_rhss, double *d_lbs,
                                              double *d_ubs, const int *d_vartypes, int max_rounds,
                                              void *stream, gdp_stats *stats) {
-    try {
+    return gdp::guarded([&]() -> GDP_RETCODE {
         return gdp::propagate_noalloc(n_cons, n_vars, nnz, d_csr_col_indices, d_csr_row_ptrs, d_csr_vals,
                                       d_lhss, d_rhss, d_lbs, d_ubs, d_vartypes, max_rounds,
                                       static_cast<cudaStream_t>(stream), stats);
-    } catch (const std::exception &e) {
-        gdp::set_error(e.what());
-        return GDP_ERROR;
-    }
+    });
 }
 #pragma GCC visibility pop
