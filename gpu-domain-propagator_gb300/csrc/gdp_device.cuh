@@ -85,6 +85,19 @@ __device__ __forceinline__ bool gt0_bits(long long b) { return b > 0; }
 __device__ __forceinline__ bool neginf_bits(long long b) { return (unsigned long long)b >= kBitsNegInf; }
 // x >= 1e20 (ISPOSINF)
 __device__ __forceinline__ bool posinf_bits(long long b) { return b >= kBitsPosInf; }
+// The same with kNan, false for a NaN as the compares are; without, a NaN bound
+// counts as infinite (two integer instructions less per element: 26.65 against 26.91 ms on 2M rows).
+template <bool kNan>
+__device__ __forceinline__ bool neg_inf(double x) {
+    const long long b = dbits(x);
+    return kNan ? (unsigned long long)b - kBitsNegInf <= 0xFFF0000000000000ULL - kBitsNegInf : neginf_bits(b);
+}
+template <bool kNan>
+__device__ __forceinline__ bool pos_inf(double x) {
+    const long long b = dbits(x);
+    return kNan ? (unsigned long long)(b - kBitsPosInf) <= (unsigned long long)(kBitsIeeeInf - kBitsPosInf)
+                : posinf_bits(b);
+}
 // EPSGT(x, y) with the FP64 subtraction only when x > y.
 __device__ __forceinline__ bool eps_gt_fast(double x, double y) {
     return order_key(dbits(x)) > order_key(dbits(y)) && eps_gt(x, y);

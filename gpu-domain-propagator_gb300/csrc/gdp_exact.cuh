@@ -99,9 +99,11 @@ __device__ __forceinline__ int flat_slot(const FlatRows &F, int f0, int lane) {
 // The terms of one element as computeActivities forms them
 // (src/propagation_methods.cuh:188-214); an infinite contribution is left out
 // of its sum (adding +0.0 changes no sum that starts at +0.0).
+// kNan: a NaN bound is no infinity (T::kNan).
+template <bool kNan>
 __device__ __forceinline__ void exact_terms(double a, double2 b, double &tmin, double &tmax, double &d) {
     const long long ab = dbits(a);
-    const bool pos = gt_eps_bits(ab), lneg = neginf_bits(dbits(b.x)), upos = posinf_bits(dbits(b.y));
+    const bool pos = gt_eps_bits(ab), lneg = neg_inf<kNan>(b.x), upos = pos_inf<kNan>(b.y);
     const bool gt0 = gt0_bits(ab);
     tmin = (pos ? lneg : upos) ? 0.0 : dmul(a, gt0 ? b.x : b.y);
     tmax = (pos ? upos : lneg) ? 0.0 : dmul(a, gt0 ? b.y : b.x);
@@ -162,8 +164,8 @@ __device__ __forceinline__ void exact_push(const T &t, ExactSmem &xs, ExactQueue
         const int minf = (info >> 2) & 3, maxf = (info >> 4) & 3;
         const int nu = pos ? minf : maxf, nl = pos ? maxf : minf;
         // a side with one infinite contribution is usable if it is this variable's
-        uo = (pos ? rs : ls) && (nu == 0 || (nu == 1 && neginf_bits(dbits(b.x))));
-        lo = (pos ? ls : rs) && (nl == 0 || (nl == 1 && posinf_bits(dbits(b.y))));
+        uo = (pos ? rs : ls) && (nu == 0 || (nu == 1 && neg_inf<T::kNan>(b.x)));
+        lo = (pos ? ls : rs) && (nl == 0 || (nl == 1 && pos_inf<T::kNan>(b.y)));
     }
     const unsigned bu = __ballot_sync(kFull, uo), bl = __ballot_sync(kFull, lo);
     const unsigned lt = (1u << lane) - 1u;
@@ -270,7 +272,7 @@ __device__ __forceinline__ ExactSums exact_sums(const T &t, ExactSmem &xs, const
         for (int i = 0; i < kU; i++)
             if (s0 + i < steps) {
                 double tmin, tmax, d;
-                exact_terms(a[i], b[i], tmin, tmax, d);
+                exact_terms<T::kNan>(a[i], b[i], tmin, tmax, d);
                 acc = dadd(acc, tmin);
                 acc2 = dadd(acc2, tmax);
                 const long long db = dbits(d), kd = order_key(db);
@@ -344,7 +346,7 @@ __device__ __forceinline__ ExactSums exact_sums_spread(const T &t, ExactSmem &xs
             bool keep = false;
             if (j[i] >= 0) {
                 double d;
-                exact_terms(a[i], b[i], tmin, tmax, d);
+                exact_terms<T::kNan>(a[i], b[i], tmin, tmax, d);
                 const long long db = dbits(d), kd = order_key(db);
                 if (kd > km && kd <= kKeyPosInf) {
                     km = kd;
@@ -400,8 +402,8 @@ __device__ __forceinline__ void exact_candidates(const T &t, ExactSmem &xs, Exac
                                                  int *row_tight = nullptr) {
     if (!__any_sync(kFull, go)) return;
     if (R.in) {
-        const bool rhs_ok = !posinf_bits(dbits(R.rhs)) && !neginf_bits(dbits(S.minact));
-        const bool lhs_ok = !neginf_bits(dbits(R.lhs)) && !posinf_bits(dbits(S.maxact));
+        const bool rhs_ok = !pos_inf<T::kNan>(R.rhs) && !neg_inf<T::kNan>(S.minact);
+        const bool lhs_ok = !neg_inf<T::kNan>(R.lhs) && !pos_inf<T::kNan>(S.maxact);
         xs.slack[lane] = s;
         xs.nsur[lane] = u;
         xs.info[lane] = (unsigned char)((rhs_ok ? 1 : 0) | (lhs_ok ? 2 : 0) | min(R.minf, 3) << 2 |

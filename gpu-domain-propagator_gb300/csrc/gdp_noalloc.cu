@@ -203,8 +203,8 @@ __device__ __forceinline__ float bound_screen_bits(long long b, bool infinite, f
 }
 __device__ __forceinline__ float2 bnd_screen_bits(double2 v) {
     const long long l = dbits(v.x), u = dbits(v.y);
-    return make_float2(bound_screen_bits(l, neginf_bits(l), -kF32Inf),
-                       bound_screen_bits(u, posinf_bits(u), kF32Inf));
+    return make_float2(bound_screen_bits(l, neg_inf<true>(v.x), -kF32Inf),
+                       bound_screen_bits(u, pos_inf<true>(v.y), kF32Inf));
 }
 
 __device__ __forceinline__ bool bit_of(const unsigned *map, int j) { return (map[j >> 5] >> (j & 31)) & 1u; }
@@ -271,6 +271,7 @@ constexpr size_t kNaSmem = sizeof(NaWarp) * kNaWarps;
 // Elements, bounds and targets of the exact pass: candidates go to the
 // caller's arrays.
 struct NaTarget {
+    static constexpr bool kNan = true;
     const int *col;
     const double *val;
     const double2 *bnd;
@@ -325,7 +326,7 @@ __device__ __forceinline__ ExactSums flat_sums(const NaTarget &t, NaWarp &ws, co
         for (int i = 0; i < kSteps; i++) {
             if (w0 + 32 * i >= F.total) break;  // warp-uniform
             double d;
-            exact_terms(a[i], b[i], ws.t[0][32 * i + lane], ws.t[1][32 * i + lane], d);
+            exact_terms<NaTarget::kNan>(a[i], b[i], ws.t[0][32 * i + lane], ws.t[1][32 * i + lane], d);
             ws.d[32 * i + lane] = d;
             const long long db = dbits(d);
             const long long cut = __shfl_sync(kFull, my_cut, max(slots[i], 0));
@@ -608,7 +609,7 @@ __device__ __forceinline__ void na_long_row(const Csr &A, const NoallocView &S, 
         for (int i = 0; i < kStage / 32; i++)
             if (j[i] >= 0) {
                 double d;
-                exact_terms(a[i], bb[i], wss[wid].t[0][32 * i + lane], wss[wid].t[1][32 * i + lane], d);
+                exact_terms<NaTarget::kNan>(a[i], bb[i], wss[wid].t[0][32 * i + lane], wss[wid].t[1][32 * i + lane], d);
                 const long long kd = order_key(dbits(d));
                 if (kd > km && kd <= kKeyPosInf) {
                     km = kd;

@@ -162,6 +162,7 @@ __device__ __forceinline__ bool row_due(const DevProblem &P, int round, int chg)
 // row-contiguous copy of the SELL rows, or the split rows.
 struct CtxTarget {
     static constexpr bool kAligned = true;  // one-lane rows (gdp_internal.h)
+    static constexpr bool kNan = false;
     const DevProblem &P;
     const int *col;
     const double *val;
